@@ -57,7 +57,8 @@ typedef struct {
     double viscosity;
     double gravity[3];
     double dt;
-    int    solver_type;               /* 0: CG, 1: ICCG */
+    int    solver_type;               /* 0: CG, 1: preconditioned CG (the reference's ICCG; here a
+                                         multilevel preconditioner, IC(0) with MPS_SWEEP=0..2) */
     int    cg_max_iter;
     double cg_tolerance;
     double relaxation_coeff;
@@ -229,7 +230,8 @@ int  mps_get_ppe(mps_session *s, int *eq_idx, int *row_ptr, int *col_idx, double
 /* The last step's PPE and IC(0) preconditioner in the solver's own unknown
  * numbering (block colour order: colour by colour, cell by cell), for
  * checking the factorisation (pressure_solver.c:156-232 restated on this
- * ordering) and the sweeps.  ICCG sessions only.
+ * ordering) and the sweeps.  Sessions of solver_type 1 only; the factor is
+ * formed by the first of these calls where the solve did not need it.
  *
  * mps_get_ic0: row_ptr[n_eq+1], col[nnz] (sorted), A[nnz] and b[n_eq] (FP64)
  * and F[nnz], the factor in A's pattern: L_ij below the diagonal, 1/L_ii on
@@ -242,7 +244,7 @@ int  mps_get_ppe(mps_session *s, int *eq_idx, int *row_ptr, int *col_idx, double
  * (0 entries for cells above 64 unknowns, which the sweeps solve by
  * substitution); colour_rows[2^dim + 1] the first row of each colour.
  * mps_apply_preconditioner: z = (L L^T)^-1 r by the device sweeps of the
- * last solve's form (the FP32 factor copies after a mixed-form solve); r, z
+ * last solve's precision form (FP32 factor copies after a mixed-form solve); r, z
  * are host arrays of n_eq doubles in the solver's numbering. */
 int  mps_get_ic0(mps_session *s, int *row_ptr, int *col, double *A, double *F, double *b, int *n_eq,
                  long long *nnz);
@@ -314,7 +316,7 @@ int  mps_run_stage(mps_session *s, int stage, const int *neighbors, const int *c
  * Every discrete decision of the step is held fixed (neighbour sets,
  * collision partners, order and branches, free-surface flags, the PPE
  * unknown set, the P_min argument, ghosting); the PPE adjoint is a second
- * ICCG solve with the step's matrix and IC(0) factor to relative residual
+ * PCG solve with the step's matrix and preconditioner to relative residual
  * 1e-12 (in the session's precision form: with MPS_PREC_MIXED, the mixed
  * solve with reliable updates, to 1e-12 or the FP64 rounding floor if
  * that is higher).  Walls, dummies and ghosts get zero adjoints.  Supported: hs_mode

@@ -30,6 +30,7 @@
 #include "k_ops.cuh"
 #include "k_ppe.cuh"
 #include "k_pcg.cuh"
+#include "k_ml.cuh"
 #include "k_sort.cuh"
 #include "k_adj.cuh"
 
@@ -285,11 +286,15 @@ private:
     // cell (jlen_, its scan jdc_*), diagonal slots (jdp_*), row of each rank
     DevArray<int> jlen_, jdc_lo_, jdc_up_, jdp_lo_, jdp_up_;
     DevArray<unsigned char> jperm_lo_, jperm_up_;
-    // ICCG loop (MPS_SWEEP): 2 the persistent k_pcg (one cooperative launch
-    // per batch of iterations), 0 the launch-per-colour k_sweep_colour with
-    // separate SpMV and vector kernels, 1 the same with the CTA-per-cell
-    // k_sweep_cell over jagged-diagonal cross blocks
-    int sweep_mode_ = 0;
+    // preconditioner and loop of the ICCG solver type (MPS_SWEEP): 3 the
+    // multilevel preconditioner (default); the IC(0) of the block-colour order
+    // with 2 the persistent k_pcg (one cooperative launch per batch of
+    // iterations), 0 the launch-per-colour k_sweep_colour with separate SpMV
+    // and vector kernels, 1 the same with the CTA-per-cell k_sweep_cell over
+    // jagged-diagonal cross blocks.  Mode 3 forms the IC(0) factor only when a
+    // caller asks for it (get_ic0 and its companions), for mode 0's sweeps.
+    int sweep_mode_ = 3;
+    int ic_mode() const { return sweep_mode_ == 3 ? 0 : sweep_mode_; }
     DevArray<unsigned> pcg_bar_;   // grid-barrier counter of k_pcg
     DevArray<unsigned long long> pcg_trace_;    // k_pcg phase timestamps while profiling
     std::vector<unsigned long long> trace_host_;
@@ -352,8 +357,34 @@ private:
     int win_ = CELL_WIN;
     bool win_valid_ = false;               // the window tables match the current factor and win_
     std::vector<int> inv_col_off_;         // block-inverse offsets at the colour boundaries
+    // ---- multilevel preconditioner
+    MlLevels ml_{};                        // grids of the cell grid; lo of the current structure
+    int ml_total_ = 0;                     // nodes of all grids, margins included (0: too many)
+    bool ml_on_ = false;                   // the current solve uses it
+    bool ml_add_ = false;                  // additive first grid
+    int ml_l0_ = 0;                        // first grid of the cluster kernel
+    // unknowns below which the first grid is additive (MPS_ML_ADD): two products
+    // with its operator fewer per iteration for about a third more iterations,
+    // which pays where an iteration is a chain of short launches; and nodes
+    // up to which a grid runs in the cluster kernel (MPS_ML_CLUSTER): beyond,
+    // a product streams more of the operator than one cluster's SMs can draw
+    int ml_add_rows_ = 60000, ml_cl_nodes_ = 4096;
+    DevArray<int> mlflag_, mlpos_, mlmap_, mlact_, mlcell_, mlncell_, mlcnode_, ufpar_, ufkeep_, mlscan_;
+    DevArray<unsigned char> bounded_;
+    DevArray<float> mlfrac_;
+    DevArray<double> mlcm_, mlA_, mldinv_, mlb_, mlx_, mly_, mlinv_, mlcsum_, jdinv_;
+    void ml_levels();
+    void ml_nodes(int nact);
+    void ml_build(int n_eq);
+    MlVecs ml_vecs() const;
+    const double *ml_result() const { return ml_.nl == 1 || ml_add_ ? mlx_.p : mly_.p; }
+    void ml_update(bool restrict_only, double *x, double *r, const double *p, const double *Ap);
+    void ml_cycle();
+    void ml_prolong(bool rz, const double *r, double *z);
+
     bool ppe_valid_ = false;
-    bool ic0_valid_ = false;     // the IC(0) factor and its sweep tables belong to the last PPE
+    bool ic0_valid_ = false;     // the last PPE was an ICCG one: its IC(0) factor can be had
+    bool ic0_built_ = false;     // the factor and its sweep tables have been formed
     bool last_fp32_ = false;     // the last solve ran the mixed form (FP32 factor copies exist)
 
     // ---- driven walls
@@ -430,8 +461,15 @@ private:
     // step's metrics as they are
     void mixed_solve(int n_eq, long long nnz, bool icc, bool adjoint = false);
     void build_windows(bool fp32);
+    void factor_ic0();      // IC(0) factor and sweep tables of the current matrix
+    void convert_ic0();     // their FP32 copies
+    void require_ic0();     // both, for callers that inspect them
     static constexpr int kMaxUpdates = 200;      // reliable updates of the mixed form, at most
-    static constexpr double kDelta = 0.01;       // residual reduction between reliable updates (mixed form)
+    // residual reduction between reliable updates (mixed form); measured at c2:
+    // 0.01 30.3 ms of solve, 0.001 28.9, 0.0001 26.9, 0.00001 27.6
+    static constexpr double kDelta = 0.0001;
+    static constexpr double kNear = 16.0;        // an inner solve that would end within this of the goal
+    static constexpr double kAim = 0.25;         // aims at this part of it instead
     static constexpr double kStall = 0.5;        // a reliable update that does not halve the best true
     static constexpr int kMaxStalls = 2;         // residual is a stall; this many in a row end the solve
     static constexpr double kUnitRoundoff = 1.1102230246251565e-16;   // 2^-53
@@ -473,8 +511,10 @@ Engine<D>::Engine(const mps_params_t &p, int capacity)
     if (const char *e = std::getenv("MPS_PACK")) pack_ = std::atoi(e) ? 1 : 0;
     if (const char *e = std::getenv("MPS_SWEEP")) {
         int v = std::atoi(e);
-        sweep_mode_ = (v == 0 || v == 1) ? v : 2;
+        sweep_mode_ = (v == 0 || v == 1 || v == 3) ? v : 2;
     }
+    if (const char *e = std::getenv("MPS_ML_ADD")) ml_add_rows_ = std::max(0, std::atoi(e));
+    if (const char *e = std::getenv("MPS_ML_CLUSTER")) ml_cl_nodes_ = std::max(0, std::atoi(e));
     if (const char *e = std::getenv("MPS_SWEEP_HB")) head_batch_ = std::atoi(e) == 8 ? 8 : 4;
     if (const char *e = std::getenv("MPS_SWEEP_OCC")) sweep_occ_ = std::atoi(e) == 8 ? 8 : 6;
     if (const char *e = std::getenv("MPS_SWEEP_HR")) head_rows_ = std::atoi(e) == 2 ? 2 : 1;
@@ -665,8 +705,37 @@ void Engine<D>::build_grid()
     aflag_.reserve(total + 1);
     apos_.reserve(total + 1);
     acells_.reserve(total + 1);
-    sizes_.reserve(16);
+    sizes_.reserve(64);
+    ml_levels();
+}
 
+// The nested grids over the cell grid: nodes on the cell corners, then every
+// other node until the box holds at most ML_COARSEST nodes.
+template <int D>
+void Engine<D>::ml_levels()
+{
+    ml_ = MlLevels{};
+    long long first = 0;
+    int n[3] = {g_.dims[0] + 1, g_.dims[1] + 1, D == 3 ? g_.dims[D - 1] + 1 : 1};
+    for (;;) {
+        MlGrid &m = ml_.g[ml_.nl++];
+        long long s1 = n[0] + 4, s2 = s1 * (n[1] + 4), size = D == 3 ? s2 * (n[2] + 4) : s2;
+        if (first + size > 0x7fffff00LL) {
+            ml_total_ = 0;   // the grids' node numbers would not fit: IC(0) instead
+            return;
+        }
+        for (int d = 0; d < 3; d++) m.n[d] = n[d];
+        m.s1 = (int)s1;
+        m.s2 = (int)s2;
+        m.first = (int)first;
+        m.size = (int)size;
+        m.base = (int)(first + 2 + 2 * s1 + (D == 3 ? 2 * s2 : 0));
+        first += size;
+        if ((long long)n[0] * n[1] * n[2] <= ML_COARSEST) break;
+        for (int d = 0; d < D; d++) n[d] = n[d] / 2 + 1;
+    }
+    ml_total_ = (int)first;
+    mlscan_.reserve(scan_workspace(ml_total_ + 1));
 }
 
 // Constants evaluated with the reference's expressions.
@@ -1142,6 +1211,334 @@ void Engine<D>::step_with_list(const int *nb, const int *cnt, int max_nb)
     tstep_++;
 }
 
+// ---- multilevel preconditioner ---------------------------------------------------
+
+// Nodes of every grid under the cells that hold unknowns, numbered grid by
+// grid; the counts go to sizes_.
+template <int D>
+void Engine<D>::ml_nodes(int nact)
+{
+    int total = ml_total_, nl = ml_.nl;
+    for (auto *v : {&mlflag_, &mlpos_, &mlmap_, &mlact_}) v->reserve((size_t)total + 1);
+    mlcnode_.reserve((size_t)nact + 1);
+    mlcell_.reserve((size_t)g_.total);
+    MPS_CUDA(cudaMemsetAsync(mlflag_.p, 0, sizeof(int) * (size_t)total, st_));
+    launch(k_ml_flag1<D>, nblk(nact, TPB), TPB, 0, st_, nact, (const int *)acells_.p, g_, ml_.g[0], mlflag_.p,
+           mlcnode_.p);
+    MlFirsts firsts{};
+    for (int l = 0; l + 1 < nl; l++) {
+        const MlGrid &f = ml_.g[l];
+        launch(k_ml_flag_up<D>, nblk((long long)f.n[0] * f.n[1] * f.n[2], TPB), TPB, 0, st_, f, ml_.g[l + 1],
+               mlflag_.p);
+    }
+    for (int l = 0; l < nl; l++) firsts.v[l] = ml_.g[l].first;
+    firsts.v[nl] = total;
+    scan_exclusive<int>(mlflag_.p, mlpos_.p, total, mlscan_.p, st_);
+    launch(k_ml_compact, nblk(total, TPB), TPB, 0, st_, total, (const int *)mlflag_.p, (const int *)mlpos_.p,
+           mlact_.p, mlmap_.p);
+    launch(k_ml_sizes, 1, 32, 0, st_, firsts, nl, (const int *)mlpos_.p, sizes_.p);
+    launch(k_ml_cellact, nblk(g_.total, TPB), TPB, 0, st_, g_.total, (const int *)ccells_.p, (const int *)ucol_.p,
+           (const int *)apos_.p, mlcell_.p);
+}
+
+template <int D>
+MlVecs Engine<D>::ml_vecs() const
+{
+    MlVecs v;
+    v.b = mlb_.p;
+    v.x = mlx_.p;
+    v.y = mly_.p;
+    v.act = mlact_.p;
+    v.A = mlA_.p;
+    v.dinv = mldinv_.p;
+    v.ncell = mlncell_.p;
+    v.csum = mlcsum_.p;
+    v.inv = mlinv_.p;
+    v.na1 = ml_.lo[1];
+    return v;
+}
+
+// P, the Galerkin operators and their smoother factors for the current
+// matrix and right-hand side.
+template <int D>
+void Engine<D>::ml_build(int n_eq)
+{
+    using L = MlDim<D>;
+    State<D> &s = S();
+    int nl = ml_.nl, na1 = ml_.lo[1], nall = ml_.lo[nl], nact = act_off_[1 << D];
+    ml_add_ = n_eq < ml_add_rows_;
+    ml_l0_ = 0;
+    while (ml_l0_ + 1 < nl && ml_.lo[ml_l0_ + 1] - ml_.lo[ml_l0_] > ml_cl_nodes_) ml_l0_++;
+    for (auto *v : {&mlb_, &mlx_, &mly_}) {
+        v->reserve((size_t)ml_total_);
+        MPS_CUDA(cudaMemsetAsync(v->p, 0, sizeof(double) * (size_t)ml_total_, st_));
+    }
+    mlncell_.reserve((size_t)L::NC * na1);
+    mlcm_.reserve((size_t)nact * L::NC * L::W4);
+    mlA_.reserve((size_t)nall * L::STP);
+    mldinv_.reserve((size_t)nall);
+    mlcsum_.reserve((size_t)nact * L::NC);
+    mlinv_.reserve((size_t)ML_COARSEST * ML_COARSEST);
+    mlfrac_.reserve((size_t)D * cap_);
+    jdinv_.reserve((size_t)cap_);
+    ufpar_.reserve((size_t)cap_);
+    ufkeep_.reserve((size_t)cap_);
+    const int *rp = row_ptr_.p, *dp = diagpos_.p, *ci = col_.p;
+    const double *A = A_.p;
+    adesc_.reserve((size_t)nact + 1);
+    launch(k_cell_desc, nblk(nact, TPB), TPB, 0, st_, nact, (const int *)acells_.p, (const int *)cell_row0_.p,
+           (const int *)ucount_.p, adesc_.p, err_.p);
+    launch(k_uf_init, nblk(n_eq, TPB), TPB, 0, st_, n_eq, rp, dp, ci, A, ufpar_.p, ufkeep_.p);
+    launch(k_uf_hook, nblk((long long)n_eq * 8, TPB), TPB, 0, st_, n_eq, rp, dp, ci, A, ufpar_.p);
+    launch(k_uf_keep, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const double *)b_.p, (const unsigned char *)bounded_.p,
+           ufpar_.p, ufkeep_.p);
+    launch(k_ml_rows<D>, nblk(n_eq, TPB), TPB, 0, st_, s, g_, n_eq, cap_, (const int *)part_of_row_.p, dp, A,
+           ufpar_.p, (const int *)ufkeep_.p, mlfrac_.p, jdinv_.p);
+    launch(k_ml_node_cells<D>, nblk(na1, TPB), TPB, 0, st_, na1, (const int *)mlact_.p, ml_.g[0], g_,
+           (const int *)mlcell_.p, mlncell_.p);
+    launch(k_ml_cellmat<D>, nact, D == 3 ? 256 : 64, 0, st_, nact, (const int *)acells_.p, (const int2 *)adesc_.p, g_,
+           (const int *)cell_row0_.p, (const int *)ucount_.p, rp, ci, A, (const float *)mlfrac_.p, cap_, mlcm_.p);
+    launch(k_ml_a1<D>, na1, L::STP, 0, st_, na1, (const int *)mlncell_.p, (const double *)mlcm_.p,
+           ml_add_ && nl > 1, mlA_.p, mldinv_.p);
+    for (int l = 0; l + 1 < nl; l++) {
+        int lof = ml_.lo[l], loc = ml_.lo[l + 1], nc = ml_.lo[l + 2] - loc;
+        launch(k_ml_galerkin<D>, nc, L::STP, 0, st_, ml_.g[l], ml_.g[l + 1], lof, loc, (const int *)mlact_.p,
+               (const int *)mlmap_.p, (const double *)mlA_.p + (size_t)lof * L::STP,
+               mlA_.p + (size_t)loc * L::STP, mldinv_.p + loc);
+    }
+    int lo = ml_.lo[nl - 1], n = nall - lo;
+    launch(k_ml_inverse<D>, 1, 1024, sizeof(double) * (size_t)(n * n + n), st_, ml_.g[nl - 1], lo, n,
+           (const int *)mlact_.p, (const int *)mlmap_.p, (const double *)mlA_.p + (size_t)lo * L::STP, mlinv_.p);
+    MPS_CUDA(cudaGetLastError());
+}
+
+// x += alpha p, r -= alpha Ap, r.r and the cells' parts of P^T r (the last
+// alone when restrict_only).
+template <int D>
+void Engine<D>::ml_update(bool restrict_only, double *x, double *r, const double *p, const double *Ap)
+{
+    int nact = act_off_[1 << D];
+    launch_pdl(restrict_only ? k_ml_update<D, true> : k_ml_update<D, false>, RED_BLOCKS, CG_BLOCK, 0, st_, nact,
+               (const int2 *)adesc_.p, (const float *)mlfrac_.p, cap_, x, r, p, Ap, mlcsum_.p, partials_.p, ticket_.p,
+               sc_.p);
+}
+
+// The V-cycle: grids with many nodes a launch per step, the others in the
+// cluster kernel.
+template <int D>
+void Engine<D>::ml_cycle()
+{
+    MlVecs v = ml_vecs();
+    int nl = ml_.nl;
+    const CGScalars *sc = sc_.p;
+    auto blocks = [&](long long threads) { return std::min(nblk(threads, CG_BLOCK), 148 * 16); };
+    for (int l = 0; l < ml_l0_; l++) {
+        int lo = ml_.lo[l], hi = ml_.lo[l + 1], na = hi - lo;
+        bool above_add = ml_add_ && l == 1;
+        if (l == 0) launch_pdl(k_ml_nodes1<D>, blocks(na), CG_BLOCK, 0, st_, v, sc);
+        else
+            launch_pdl(k_ml_restrict<D>, blocks(na), CG_BLOCK, 0, st_, v, (const double *)(above_add ? v.b : v.y),
+                       ml_.g[l - 1], ml_.g[l], lo, hi, sc);
+        if (!(ml_add_ && l == 0))
+            launch_pdl(k_ml_residual<D, false>, blocks(8LL * na), CG_BLOCK, 0, st_, v, ml_.g[l], lo, hi, sc);
+    }
+    const double *src = ml_l0_ == 0 ? nullptr : (ml_add_ && ml_l0_ == 1) ? v.b : v.y;
+    launch_pdl(k_ml_cycle<D>, ML_CL, ML_CL_THREADS, 0, st_, v, ml_, ml_l0_, src, ml_add_, sc);
+    for (int l = ml_l0_ - 1; l >= 0; l--) {
+        int lo = ml_.lo[l], hi = ml_.lo[l + 1], na = hi - lo;
+        const double *cx = l + 1 == nl - 1 ? v.x : v.y;
+        launch_pdl(k_ml_prolong_add<D>, blocks(na), CG_BLOCK, 0, st_, v, cx, ml_.g[l], ml_.g[l + 1], lo, hi, sc);
+        if (!(ml_add_ && l == 0))
+            launch_pdl(k_ml_residual<D, true>, blocks(8LL * na), CG_BLOCK, 0, st_, v, ml_.g[l], lo, hi, sc);
+    }
+}
+
+// z = D^-1 r + P x_1, with r.z and beta when rz.
+template <int D>
+void Engine<D>::ml_prolong(bool rz, const double *r, double *z)
+{
+    int nact = act_off_[1 << D];
+    launch_pdl(rz ? k_ml_prolong<D, true> : k_ml_prolong<D, false>, RED_BLOCKS, CG_BLOCK, 0, st_, nact,
+               (const int2 *)adesc_.p, (const int *)mlcnode_.p, ml_.g[0], (const float *)mlfrac_.p, cap_,
+               (const double *)jdinv_.p, r, z, ml_result(), partials_.p, ticket_.p, sc_.p);
+}
+
+// The IC(0) factor of the current matrix, colour by colour, and the tables
+// of the colour sweeps.
+template <int D>
+void Engine<D>::factor_ic0()
+{
+    int ncol = 1 << D, n_eq = n_eq_;
+    size_t nnz = (size_t)nnz_;
+    State<D> &s = S();
+    F_.reserve(nnz);
+    launch(k_row_splits, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)row_ptr_.p, (const int *)diagpos_.p,
+           (const int *)col_.p, (const int *)part_of_row_.p, (const int *)s.cell, (const int *)cell_row0_.p,
+           (const int *)ucount_.p, inpos_.p, outpos_.p);
+    MPS_CUDA(cudaMemcpyAsync(F_.p, A_.p, sizeof(double) * nnz, cudaMemcpyDeviceToDevice, st_));
+    for (int c = 0; c < ncol; c++) {
+        int rb = row_off_[c], re = row_off_[c + 1];
+        if (re > rb)
+            launch(k_ic0_cross_warp, nblk((long long)(re - rb) * 32, 256), 256, 0, st_, rb, re,
+                   (const int *)row_ptr_.p, (const int *)diagpos_.p, (const int *)inpos_.p, (const int *)col_.p,
+                   (const double *)A_.p, F_.p);
+        int kb = act_off_[c], ke = act_off_[c + 1];
+        if (ke > kb)
+            launch(k_ic0_incell, nblk(ke - kb, SWEEP_WARPS_IC), 32 * SWEEP_WARPS_IC, 0, st_, kb, ke,
+                   (const int *)acells_.p, (const int *)cell_row0_.p, (const int *)ucount_.p,
+                   (const int *)row_ptr_.p, (const int *)diagpos_.p, (const int *)inpos_.p,
+                   (const int *)col_.p, (const double *)A_.p, F_.p);
+    }
+    // packed in-cell factor and cell descriptors for the sweeps
+    launch(k_pack_lengths, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)row_ptr_.p,
+           (const int *)diagpos_.p, (const int *)inpos_.p, (const int *)outpos_.p, pk_len_lo_.p, pk_len_up_.p);
+    scan_exclusive<int>(pk_len_lo_.p, pk_off_lo_.p, n_eq, scanws_.p, st_);
+    scan_exclusive<int>(pk_len_up_.p, pk_off_up_.p, n_eq, scanws_.p, st_);
+    size_t in_cap = (size_t)nnz;   // in-cell entries are a subset of the nonzeros
+    pk_val_lo_.reserve(in_cap);
+    pk_val_up_.reserve(in_cap);
+    pk_k_lo_.reserve(in_cap);
+    pk_k_up_.reserve(in_cap);
+    launch(k_pack_fill, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)diagpos_.p, (const int *)inpos_.p,
+           (const int *)outpos_.p, (const int *)col_.p, (const double *)F_.p, (const int *)part_of_row_.p,
+           (const int *)s.cell, (const int *)cell_row0_.p, (const int *)pk_off_lo_.p,
+           (const int *)pk_off_up_.p, pk_val_lo_.p, pk_k_lo_.p, pk_val_up_.p, pk_k_up_.p, dinv_.p, err_.p);
+    // packed cross-cell runs of the factor for the sweeps
+    for (auto *v : {&xlen_lo_, &xlen_up_, &xp_lo_, &xp_up_, &xs_lo_, &xs_up_}) v->reserve((size_t)n_eq + 1);
+    launch(k_cross_lengths, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)row_ptr_.p, (const int *)inpos_.p,
+           (const int *)outpos_.p, xlen_lo_.p, xlen_up_.p);
+    scan_exclusive<int>(xlen_lo_.p, xp_lo_.p, n_eq, scanws_.p, st_);
+    scan_exclusive<int>(xlen_up_.p, xp_up_.p, n_eq, scanws_.p, st_);
+    nx_lo_ = read_int(xp_lo_.p + n_eq);
+    nx_up_ = read_int(xp_up_.p + n_eq);
+    xc_lo_.reserve((size_t)nx_lo_ + 1);
+    xf_lo_.reserve((size_t)nx_lo_ + 1);
+    xc_up_.reserve((size_t)nx_up_ + 1);
+    xf_up_.reserve((size_t)nx_up_ + 1);
+    SweepColours swc{};
+    swc.ncol = ncol;
+    for (int c = 0; c <= ncol; c++) swc.row_off[c] = row_off_[c];
+    for (int k = 0; k < ncol; k++) {
+        // the colour swept just before k, forward (largest non-empty below) and backward
+        int pf = -1, pb = -1;
+        for (int j = k - 1; j >= 0 && pf < 0; j--)
+            if (row_off_[j + 1] > row_off_[j]) pf = j;
+        for (int j = k + 1; j < ncol && pb < 0; j++)
+            if (row_off_[j + 1] > row_off_[j]) pb = j;
+        swc.thr_lo[k] = pf >= 0 ? row_off_[pf] : 0;
+        swc.thr_up[k] = pb >= 0 ? row_off_[pb + 1] : 0x7fffffff;
+    }
+    int nact = act_off_[ncol];
+    adesc_.reserve((size_t)nact + 1);
+    if (nact)
+        launch(k_cell_desc, nblk(nact, TPB), TPB, 0, st_, nact, (const int *)acells_.p,
+               (const int *)cell_row0_.p, (const int *)ucount_.p, adesc_.p, err_.p);
+    if (ic_mode() != 0) {
+        // the cross runs of each cell in jagged-diagonal order (k_sweep_cell, k_pcg)
+        for (auto *v : {&jlen_, &jdc_lo_, &jdc_up_}) v->reserve((size_t)nact + 1);
+        for (auto *v : {&jperm_lo_, &jperm_up_}) v->reserve((size_t)n_eq + 1);
+        for (int lo = 1; lo >= 0; lo--) {
+            DevArray<int> &jdc = lo ? jdc_lo_ : jdc_up_, &jdp = lo ? jdp_lo_ : jdp_up_;
+            const int *xp = lo ? xp_lo_.p : xp_up_.p;
+            if (nact)
+                launch(k_jds_sizes, nblk((long long)nact * 32, 256), 256, 0, st_, nact, (const int2 *)adesc_.p,
+                       xp, jlen_.p, err_.p);
+            scan_exclusive<int>(jlen_.p, jdc.p, nact, scanws_.p, st_);
+            jdp.reserve((size_t)read_int(jdc.p + nact) + 1);
+            if (!nact) continue;
+            if (lo)
+                launch(k_jds_fill<true>, nblk(nact, 4), 128, 0, st_, nact, (const int2 *)adesc_.p, xp,
+                       (const int *)jdc.p, (const int *)row_ptr_.p, (const int *)inpos_.p,
+                       (const int *)outpos_.p, (const int *)col_.p, (const double *)F_.p, jdp.p, jperm_lo_.p,
+                       xc_lo_.p, xf_lo_.p);
+            else
+                launch(k_jds_fill<false>, nblk(nact, 4), 128, 0, st_, nact, (const int2 *)adesc_.p, xp,
+                       (const int *)jdc.p, (const int *)row_ptr_.p, (const int *)inpos_.p,
+                       (const int *)outpos_.p, (const int *)col_.p, (const double *)F_.p, jdp.p, jperm_up_.p,
+                       xc_up_.p, xf_up_.p);
+        }
+    } else {
+        launch(k_cross_fill, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)row_ptr_.p,
+               (const int *)inpos_.p, (const int *)outpos_.p, (const int *)col_.p, (const double *)F_.p,
+               (const int *)xp_lo_.p, (const int *)xp_up_.p, xc_lo_.p, xf_lo_.p, xc_up_.p, xf_up_.p, swc,
+               xs_lo_.p, xs_up_.p);
+    }
+    // inverses of the in-cell diagonal blocks of the factor, and the
+    // windows of each colour's range for the staged in-cell sweeps
+    inv_len_.reserve((size_t)nact + 1);
+    inv_off_.reserve((size_t)nact + 1);
+    if (nact) launch(k_inv_sizes, nblk(nact, TPB), TPB, 0, st_, nact, (const int2 *)adesc_.p, inv_len_.p);
+    scan_exclusive<int>(inv_len_.p, inv_off_.p, nact, scanws_.p, st_);
+    ColourIdx at{};
+    for (int c = 0; c <= ncol; c++) at.k[c] = act_off_[c];
+    colinv_.reserve(16);
+    launch(k_gather_colour_offsets, 1, 32, 0, st_, at, ncol + 1, (const int *)inv_off_.p, colinv_.p);
+    MPS_CUDA(cudaMemcpyAsync(int_host_, colinv_.p, sizeof(int) * (ncol + 1), cudaMemcpyDeviceToHost, st_));
+    MPS_CUDA(cudaStreamSynchronize(st_));
+    int ninv = int_host_[ncol];
+    if (ninv < 0) throw CudaError("in-cell inverses too large for 32-bit offsets", MPS_ERR_UNSUPPORTED);
+    inv_col_off_.assign(int_host_, int_host_ + ncol + 1);
+    inv_cm_.reserve((size_t)ninv + 1);
+    inv_rm_.reserve((size_t)ninv + 1);
+    ninv_ = ninv;
+    if (nact)
+        launch(k_cell_inverse, nblk(nact, 4), 128, 0, st_, nact, (const int2 *)adesc_.p,
+               (const int *)inv_off_.p, (const int *)pk_off_lo_.p, (const int *)pk_len_lo_.p,
+               (const double *)pk_val_lo_.p, (const unsigned char *)pk_k_lo_.p, (const double *)dinv_.p,
+               inv_cm_.p, inv_rm_.p);
+    win_valid_ = false;
+    if (ic_mode() == 0) build_windows(prm_.precision == MPS_PREC_MIXED);
+    met.sweep_cross_lo = nx_lo_;
+    met.sweep_cross_up = nx_up_;
+    met.sweep_inverse_entries = ninv_;
+    ic0_built_ = true;
+}
+
+// FP32 copies of the IC(0) factor and its sweep data (mixed form): the cross
+// runs as packed words or as separate arrays (MPS_PACK), the in-cell block
+// inverses and the packed in-cell runs.
+template <int D>
+void Engine<D>::convert_ic0()
+{
+    const int RB = RED_BLOCKS;
+    size_t nz = (size_t)nnz_;
+    const bool pk = pack_ && ic_mode() == 0 && head_batch_ == 4;
+    for (auto *v : {&pkv32_lo_, &pkv32_up_}) v->reserve(nz);
+    for (auto *v : {&inv32_cm_, &inv32_rm_}) v->reserve((size_t)ninv_ + 1);
+    dinv32_.reserve((size_t)cap_);
+    packed_ = pk;
+    if (pk) {
+        xfc32_lo_.reserve((size_t)nx_lo_ + 1);
+        xfc32_up_.reserve((size_t)nx_up_ + 1);
+        launch(k_pack_fc, RB, CG_BLOCK, 0, st_, (size_t)nx_lo_, (const double *)xf_lo_.p, (const int *)xc_lo_.p,
+               xfc32_lo_.p);
+        launch(k_pack_fc, RB, CG_BLOCK, 0, st_, (size_t)nx_up_, (const double *)xf_up_.p, (const int *)xc_up_.p,
+               xfc32_up_.p);
+    } else {
+        xf32_lo_.reserve((size_t)nx_lo_ + 1);
+        xf32_up_.reserve((size_t)nx_up_ + 1);
+        launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, (size_t)nx_lo_, (const double *)xf_lo_.p, xf32_lo_.p);
+        launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, (size_t)nx_up_, (const double *)xf_up_.p, xf32_up_.p);
+    }
+    launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, nz, (const double *)pk_val_lo_.p, pkv32_lo_.p);
+    launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, nz, (const double *)pk_val_up_.p, pkv32_up_.p);
+    launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, (size_t)n_eq_, (const double *)dinv_.p, dinv32_.p);
+    launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, (size_t)ninv_, (const double *)inv_cm_.p, inv32_cm_.p);
+    launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, (size_t)ninv_, (const double *)inv_rm_.p, inv32_rm_.p);
+}
+
+// The IC(0) factor of the last PPE for callers that inspect it: the
+// multilevel form's solve does not need it, so it is formed here.
+template <int D>
+void Engine<D>::require_ic0()
+{
+    if (!ppe_valid_ || !ic0_valid_) throw CudaError("no IC(0) factor: run an ICCG step first", MPS_ERR_INVALID);
+    if (ic0_built_ || n_eq_ == 0) return;
+    factor_ic0();
+    if (last_fp32_) convert_ic0();
+    check_err();
+}
+
 // ---- PPE ------------------------------------------------------------------------
 
 template <int D>
@@ -1186,145 +1583,35 @@ void Engine<D>::ppe(bool clamp)
         ppe_valid_ = true;
         return;
     }
+    ml_on_ = prm_.solver_type == 1 && sweep_mode_ == 3 && ml_total_ > 0;
+    if (ml_on_) ml_nodes(act_off_[ncol]);
     CellSource<D> src = cells();
     launch(k_row_count<D, CellSource<D>>, nblk(n_eq, TPB), TPB, 0, st_, src, s, part_of_row_.p, row_of_.p, n_eq,
                                                                      rcount_.p);
     scan_exclusive<int>(rcount_.p, row_ptr_.p, n_eq, scanws_.p, st_);
-    int nnz = read_int(row_ptr_.p + n_eq);
+    MPS_CUDA(cudaMemcpyAsync(int_host_, row_ptr_.p + n_eq, sizeof(int), cudaMemcpyDeviceToHost, st_));
+    if (ml_on_)
+        MPS_CUDA(cudaMemcpyAsync(int_host_ + 1, sizes_.p, sizeof(int) * (ml_.nl + 1), cudaMemcpyDeviceToHost, st_));
+    MPS_CUDA(cudaStreamSynchronize(st_));
+    int nnz = int_host_[0];
+    if (ml_on_)
+        for (int l = 0; l <= ml_.nl; l++) ml_.lo[l] = int_host_[1 + l];
     if (nnz < 0) throw CudaError("PPE too large for 32-bit row pointers", MPS_ERR_UNSUPPORTED);
     nnz_ = nnz;
     met.nnz = nnz;
     col_.reserve(nnz);
     A_.reserve(nnz);
-    F_.reserve(nnz);
+    bounded_.reserve(cap_);
     launch(k_fill<D>, nblk(n_eq, 128), 128, 0, st_, src, s, k_, part_of_row_.p, row_of_.p, n_eq, row_ptr_.p, col_.p,
-                                                A_.p, diagpos_.p, b_.p, err_.p);
+                                                A_.p, diagpos_.p, b_.p, bounded_.p, err_.p);
     MPS_CUDA(cudaEventRecord(ev_[2], st_));
     bool icc = prm_.solver_type == 1;
-    if (icc) {
-        launch(k_row_splits, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)row_ptr_.p, (const int *)diagpos_.p,
-               (const int *)col_.p, (const int *)part_of_row_.p, (const int *)s.cell, (const int *)cell_row0_.p,
-               (const int *)ucount_.p, inpos_.p, outpos_.p);
-        MPS_CUDA(cudaMemcpyAsync(F_.p, A_.p, sizeof(double) * nnz, cudaMemcpyDeviceToDevice, st_));
-        for (int c = 0; c < ncol; c++) {
-            int rb = row_off_[c], re = row_off_[c + 1];
-            if (re > rb)
-                launch(k_ic0_cross_warp, nblk((long long)(re - rb) * 32, 256), 256, 0, st_, rb, re,
-                       (const int *)row_ptr_.p, (const int *)diagpos_.p, (const int *)inpos_.p, (const int *)col_.p,
-                       (const double *)A_.p, F_.p);
-            int kb = act_off_[c], ke = act_off_[c + 1];
-            if (ke > kb)
-                launch(k_ic0_incell, nblk(ke - kb, SWEEP_WARPS_IC), 32 * SWEEP_WARPS_IC, 0, st_, kb, ke,
-                       (const int *)acells_.p, (const int *)cell_row0_.p, (const int *)ucount_.p,
-                       (const int *)row_ptr_.p, (const int *)diagpos_.p, (const int *)inpos_.p,
-                       (const int *)col_.p, (const double *)A_.p, F_.p);
-        }
-        // packed in-cell factor and cell descriptors for the sweeps
-        launch(k_pack_lengths, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)row_ptr_.p,
-               (const int *)diagpos_.p, (const int *)inpos_.p, (const int *)outpos_.p, pk_len_lo_.p, pk_len_up_.p);
-        scan_exclusive<int>(pk_len_lo_.p, pk_off_lo_.p, n_eq, scanws_.p, st_);
-        scan_exclusive<int>(pk_len_up_.p, pk_off_up_.p, n_eq, scanws_.p, st_);
-        size_t in_cap = (size_t)nnz;   // in-cell entries are a subset of the nonzeros
-        pk_val_lo_.reserve(in_cap);
-        pk_val_up_.reserve(in_cap);
-        pk_k_lo_.reserve(in_cap);
-        pk_k_up_.reserve(in_cap);
-        launch(k_pack_fill, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)diagpos_.p, (const int *)inpos_.p,
-               (const int *)outpos_.p, (const int *)col_.p, (const double *)F_.p, (const int *)part_of_row_.p,
-               (const int *)s.cell, (const int *)cell_row0_.p, (const int *)pk_off_lo_.p,
-               (const int *)pk_off_up_.p, pk_val_lo_.p, pk_k_lo_.p, pk_val_up_.p, pk_k_up_.p, dinv_.p, err_.p);
-        // packed cross-cell runs of the factor for the sweeps
-        for (auto *v : {&xlen_lo_, &xlen_up_, &xp_lo_, &xp_up_, &xs_lo_, &xs_up_}) v->reserve((size_t)n_eq + 1);
-        launch(k_cross_lengths, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)row_ptr_.p, (const int *)inpos_.p,
-               (const int *)outpos_.p, xlen_lo_.p, xlen_up_.p);
-        scan_exclusive<int>(xlen_lo_.p, xp_lo_.p, n_eq, scanws_.p, st_);
-        scan_exclusive<int>(xlen_up_.p, xp_up_.p, n_eq, scanws_.p, st_);
-        nx_lo_ = read_int(xp_lo_.p + n_eq);
-        nx_up_ = read_int(xp_up_.p + n_eq);
-        xc_lo_.reserve((size_t)nx_lo_ + 1);
-        xf_lo_.reserve((size_t)nx_lo_ + 1);
-        xc_up_.reserve((size_t)nx_up_ + 1);
-        xf_up_.reserve((size_t)nx_up_ + 1);
-        SweepColours swc{};
-        swc.ncol = ncol;
-        for (int c = 0; c <= ncol; c++) swc.row_off[c] = row_off_[c];
-        for (int k = 0; k < ncol; k++) {
-            // the colour swept just before k, forward (largest non-empty below) and backward
-            int pf = -1, pb = -1;
-            for (int j = k - 1; j >= 0 && pf < 0; j--)
-                if (row_off_[j + 1] > row_off_[j]) pf = j;
-            for (int j = k + 1; j < ncol && pb < 0; j++)
-                if (row_off_[j + 1] > row_off_[j]) pb = j;
-            swc.thr_lo[k] = pf >= 0 ? row_off_[pf] : 0;
-            swc.thr_up[k] = pb >= 0 ? row_off_[pb + 1] : 0x7fffffff;
-        }
-        int nact = act_off_[ncol];
-        adesc_.reserve((size_t)nact + 1);
-        if (nact)
-            launch(k_cell_desc, nblk(nact, TPB), TPB, 0, st_, nact, (const int *)acells_.p,
-                   (const int *)cell_row0_.p, (const int *)ucount_.p, adesc_.p);
-        if (sweep_mode_ != 0) {
-            // the cross runs of each cell in jagged-diagonal order (k_sweep_cell, k_pcg)
-            for (auto *v : {&jlen_, &jdc_lo_, &jdc_up_}) v->reserve((size_t)nact + 1);
-            for (auto *v : {&jperm_lo_, &jperm_up_}) v->reserve((size_t)n_eq + 1);
-            for (int lo = 1; lo >= 0; lo--) {
-                DevArray<int> &jdc = lo ? jdc_lo_ : jdc_up_, &jdp = lo ? jdp_lo_ : jdp_up_;
-                const int *xp = lo ? xp_lo_.p : xp_up_.p;
-                if (nact)
-                    launch(k_jds_sizes, nblk((long long)nact * 32, 256), 256, 0, st_, nact, (const int2 *)adesc_.p,
-                           xp, jlen_.p, err_.p);
-                scan_exclusive<int>(jlen_.p, jdc.p, nact, scanws_.p, st_);
-                jdp.reserve((size_t)read_int(jdc.p + nact) + 1);
-                if (!nact) continue;
-                if (lo)
-                    launch(k_jds_fill<true>, nblk(nact, 4), 128, 0, st_, nact, (const int2 *)adesc_.p, xp,
-                           (const int *)jdc.p, (const int *)row_ptr_.p, (const int *)inpos_.p,
-                           (const int *)outpos_.p, (const int *)col_.p, (const double *)F_.p, jdp.p, jperm_lo_.p,
-                           xc_lo_.p, xf_lo_.p);
-                else
-                    launch(k_jds_fill<false>, nblk(nact, 4), 128, 0, st_, nact, (const int2 *)adesc_.p, xp,
-                           (const int *)jdc.p, (const int *)row_ptr_.p, (const int *)inpos_.p,
-                           (const int *)outpos_.p, (const int *)col_.p, (const double *)F_.p, jdp.p, jperm_up_.p,
-                           xc_up_.p, xf_up_.p);
-            }
-        } else {
-            launch(k_cross_fill, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)row_ptr_.p,
-                   (const int *)inpos_.p, (const int *)outpos_.p, (const int *)col_.p, (const double *)F_.p,
-                   (const int *)xp_lo_.p, (const int *)xp_up_.p, xc_lo_.p, xf_lo_.p, xc_up_.p, xf_up_.p, swc,
-                   xs_lo_.p, xs_up_.p);
-        }
-        // inverses of the in-cell diagonal blocks of the factor, and the
-        // windows of each colour's range for the staged in-cell sweeps
-        inv_len_.reserve((size_t)nact + 1);
-        inv_off_.reserve((size_t)nact + 1);
-        if (nact) launch(k_inv_sizes, nblk(nact, TPB), TPB, 0, st_, nact, (const int2 *)adesc_.p, inv_len_.p);
-        scan_exclusive<int>(inv_len_.p, inv_off_.p, nact, scanws_.p, st_);
-        ColourIdx at{};
-        for (int c = 0; c <= ncol; c++) at.k[c] = act_off_[c];
-        colinv_.reserve(16);
-        launch(k_gather_colour_offsets, 1, 32, 0, st_, at, ncol + 1, (const int *)inv_off_.p, colinv_.p);
-        MPS_CUDA(cudaMemcpyAsync(int_host_, colinv_.p, sizeof(int) * (ncol + 1), cudaMemcpyDeviceToHost, st_));
-        MPS_CUDA(cudaStreamSynchronize(st_));
-        int ninv = int_host_[ncol];
-        if (ninv < 0) throw CudaError("in-cell inverses too large for 32-bit offsets", MPS_ERR_UNSUPPORTED);
-        inv_col_off_.assign(int_host_, int_host_ + ncol + 1);
-        inv_cm_.reserve((size_t)ninv + 1);
-        inv_rm_.reserve((size_t)ninv + 1);
-        ninv_ = ninv;
-        if (nact)
-            launch(k_cell_inverse, nblk(nact, 4), 128, 0, st_, nact, (const int2 *)adesc_.p,
-                   (const int *)inv_off_.p, (const int *)pk_off_lo_.p, (const int *)pk_len_lo_.p,
-                   (const double *)pk_val_lo_.p, (const unsigned char *)pk_k_lo_.p, (const double *)dinv_.p,
-                   inv_cm_.p, inv_rm_.p);
-        win_valid_ = false;
-        if (sweep_mode_ == 0) build_windows(prm_.precision == MPS_PREC_MIXED);
-        met.sweep_cross_lo = nx_lo_;
-        met.sweep_cross_up = nx_up_;
-        met.sweep_inverse_entries = ninv_;
-    }
+    ic0_valid_ = icc;
+    ic0_built_ = false;
+    if (icc && ml_on_) ml_build(n_eq);
+    else if (icc) factor_ic0();
     MPS_CUDA(cudaEventRecord(ev_[3], st_));
 
-    ic0_valid_ = icc;
     last_fp32_ = prm_.precision == MPS_PREC_MIXED;
     if (prm_.precision == MPS_PREC_MIXED) {
         mixed_solve(n_eq, nnz, icc);
@@ -1376,7 +1663,7 @@ void Engine<D>::run_sweep(const PcgBufs<TM> &v, bool fwdir)
             int c = fwdir ? i : ncol - 1 - i;
             if (act_off_[c + 1] > act_off_[c]) order[nc++] = c;
         }
-        if (sweep_mode_ == 1) {
+        if (ic_mode() == 1) {
             auto cellk = fwdir ? k_sweep_cell<true, TM> : k_sweep_cell<false, TM>;
             int resident = 0;
             MPS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, cellk, 32 * JW, 0));
@@ -1451,7 +1738,6 @@ void Engine<D>::pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc,
                           const double *zprev)
 {
     using T = double;
-    int ncol = 1 << D;
     const int RB = RED_BLOCKS;
     int iter_before = 0;
     if (!zprev) {
@@ -1504,8 +1790,13 @@ void Engine<D>::pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc,
             lk(4, k_cg_spmv<8, TM>, RB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap, partials_.p,
                ticket_.p, sc_.p, (const double *)nullptr, (const uint2 *)nullptr);
     };
-    const bool persist = icc && sweep_mode_ == 2;
-    if (icc) {
+    const bool ml = icc && ml_on_;
+    const bool persist = icc && !ml && sweep_mode_ == 2;
+    if (ml) {
+        ml_update(true, v.x, v.r, v.p, v.Ap);
+        ml_cycle();
+        ml_prolong(false, v.r, v.z);
+    } else if (icc) {
         if (persist) launch_pcg<TM>(v, true, 0);
         else {
             sweep(true);
@@ -1555,6 +1846,14 @@ void Engine<D>::pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc,
             if (prof) MPS_CUDA(cudaEventRecord(e[0], st_));
             spmv();
             if (prof) MPS_CUDA(cudaEventRecord(e[1], st_));
+            if (ml) {
+                ml_update(false, v.x, v.r, v.p, v.Ap);
+                ml_cycle();
+                ml_prolong(true, v.r, v.z);
+                lk(4, k_cg_update_p<T>, RB, CG_BLOCK, 0, n_eq, v.p, (const T *)z, sc_.p);
+                if (prof) MPS_CUDA(cudaEventRecord(e[2], st_));
+                continue;
+            }
             lk(4, k_cg_axpy<T>, RB, CG_BLOCK, 0, n_eq, v.x, v.r, (const T *)v.p, (const T *)v.Ap, partials_.p,
                ticket_.p, sc_.p);
             if (prof) MPS_CUDA(cudaEventRecord(e[2], st_));
@@ -1575,12 +1874,14 @@ void Engine<D>::pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc,
                 float a = 0, b2 = 0, c2 = 0, d2 = 0;
                 cudaEventElapsedTime(&a, e[0], e[1]);
                 cudaEventElapsedTime(&b2, e[1], e[2]);
-                cudaEventElapsedTime(&c2, e[2], e[3]);
-                cudaEventElapsedTime(&d2, e[3], e[4]);
+                if (!ml) {
+                    cudaEventElapsedTime(&c2, e[2], e[3]);
+                    cudaEventElapsedTime(&d2, e[3], e[4]);
+                }
                 met.prof_spmv_ms += a;
                 met.prof_spmv_launches += 1;
                 met.prof_vec_ms += b2;
-                if (icc) {
+                if (icc && !ml) {
                     met.prof_fwd_ms += c2;
                     met.prof_fwd_sweeps += 1;
                     met.prof_bwd_ms += d2;
@@ -1763,43 +2064,17 @@ void Engine<D>::mixed_solve(int n_eq, long long nnz, bool icc, bool adjoint)
     size_t nz = (size_t)nnz;
     // packed words for the launch-per-colour loop; the persistent and the
     // CTA-per-cell loops read the separate arrays
-    const bool pk = pack_ && sweep_mode_ == 0 && head_batch_ == 4;
+    const bool pk = pack_ && (ml_on_ || (sweep_mode_ == 0 && head_batch_ == 4));
     const bool pk_spmv = pk && mixed_spmv_ == 2;
-    for (auto *v : {&A32_, &pkv32_lo_, &pkv32_up_}) v->reserve(nz);
-    xf32_lo_.reserve((size_t)nx_lo_ + 1);
-    xf32_up_.reserve((size_t)nx_up_ + 1);
-    for (auto *v : {&inv32_cm_, &inv32_rm_}) v->reserve((size_t)ninv_ + 1);
-    dinv32_.reserve((size_t)cap_);
     zprev_.reserve((size_t)cap_);
     if (pk_spmv) {
         ac32_.reserve(nz);
         launch(k_pack_fc, RB, CG_BLOCK, 0, st_, nz, (const double *)A_.p, (const int *)col_.p, ac32_.p);
-    } else
+    } else {
+        A32_.reserve(nz);
         launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, nz, (const double *)A_.p, A32_.p);
-    if (icc && pk) {
-        xfc32_lo_.reserve((size_t)nx_lo_ + 1);
-        xfc32_up_.reserve((size_t)nx_up_ + 1);
-        launch(k_pack_fc, RB, CG_BLOCK, 0, st_, (size_t)nx_lo_, (const double *)xf_lo_.p, (const int *)xc_lo_.p,
-               xfc32_lo_.p);
-        launch(k_pack_fc, RB, CG_BLOCK, 0, st_, (size_t)nx_up_, (const double *)xf_up_.p, (const int *)xc_up_.p,
-               xfc32_up_.p);
     }
-    packed_ = icc && pk;
-    if (icc) {
-        if (!pk) {
-            launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, (size_t)nx_lo_, (const double *)xf_lo_.p,
-                   xf32_lo_.p);
-            launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, (size_t)nx_up_, (const double *)xf_up_.p,
-                   xf32_up_.p);
-        }
-        launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, nz, (const double *)pk_val_lo_.p, pkv32_lo_.p);
-        launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, nz, (const double *)pk_val_up_.p, pkv32_up_.p);
-        launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, (size_t)n_eq, (const double *)dinv_.p, dinv32_.p);
-        launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, (size_t)ninv_, (const double *)inv_cm_.p,
-               inv32_cm_.p);
-        launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, (size_t)ninv_, (const double *)inv_rm_.p,
-               inv32_rm_.p);
-    }
+    if (icc && !ml_on_) convert_ic0();
     CGScalars init{};
     MPS_CUDA(cudaMemcpyAsync(sc_.p, &init, sizeof(CGScalars), cudaMemcpyHostToDevice, st_));
     launch(k_refine_init, RB, CG_BLOCK, 0, st_, n_eq, x_.p, r_.p, (const double *)b_.p, partials_.p, ticket_.p,
@@ -1816,7 +2091,7 @@ void Engine<D>::mixed_solve(int n_eq, long long nnz, bool icc, bool adjoint)
                      part_.p,     b_.p};
     if (mixed_spmv_ == 1 && sweep_mode_ != 2) v.A64 = A_.p;   // tuning alternatives of the inner SpMV
     if (pk_spmv) v.ac = ac32_.p;
-    if (packed_) {
+    if (packed_ && icc && !ml_on_) {
         v.xfc_lo = xfc32_lo_.p;
         v.xfc_up = xfc32_up_.p;
     }
@@ -1827,8 +2102,15 @@ void Engine<D>::mixed_solve(int n_eq, long long nnz, bool icc, bool adjoint)
         v.dsum = dsum_.p;
     }
     const double *zsrc = icc ? z_.p : r_.p;   // the preconditioned residual
+    // tolerance of the next inner solve from a true residual `rn`: a reduction
+    // by rel_delta_, or, where that comes near the goal, well below it, since
+    // the true residual ends above the recursive one by its rounding
+    auto aim = [&](double goal, double rn) {
+        double t = rel_delta_ * rn;
+        return t > kNear * goal ? t : kAim * goal;
+    };
     if (rnorm > target) {
-        pcg_solve<float>(v, std::max(target, rel_delta_ * rnorm), prm_.cg_max_iter, icc, n_eq, nnz);
+        pcg_solve<float>(v, aim(target, rnorm), prm_.cg_max_iter, icc, n_eq, nnz);
         double goal = target;
         for (;;) {
             MPS_CUDA(cudaMemcpyAsync(zprev_.p, zsrc, sizeof(double) * n_eq, cudaMemcpyDeviceToDevice, st_));
@@ -1848,9 +2130,7 @@ void Engine<D>::mixed_solve(int n_eq, long long nnz, bool icc, bool adjoint)
             if (rnorm <= goal || sc_host_->iter >= prm_.cg_max_iter || sc_host_->breakdown ||
                 updates >= kMaxUpdates || stalls >= kMaxStalls)
                 break;
-            // the next inner solve aims at most at the goal: its recursive
-            // residual tracks the true one closely (FP64 vectors)
-            pcg_solve<float>(v, std::max(goal, rel_delta_ * rnorm), prm_.cg_max_iter, icc, n_eq, nnz, zprev_.p);
+            pcg_solve<float>(v, aim(goal, rnorm), prm_.cg_max_iter, icc, n_eq, nnz, zprev_.p);
         }
     }
     int inner = sc_host_->iter;
@@ -2102,13 +2382,13 @@ void Engine<D>::step_adjoint()
                 // the mixed form's solve (FP32 matrix and factor, FP64
                 // vectors, reliable updates) down to the same relative
                 // residual, or to the FP64 rounding floor if that is higher
-                if (icc && sweep_mode_ == 0) build_windows(true);
+                if (icc && !ml_on_ && sweep_mode_ == 0) build_windows(true);
                 mixed_solve(n_eq, nnz_, icc, true);
             } else {
                 PcgBufs<double> v{A_.p,      xf_lo_.p, xf_up_.p, pk_val_lo_.p, pk_val_up_.p, dinv_.p, inv_cm_.p,
                                   inv_rm_.p, x_.p,     r_.p,     z_.p,         p_.p,         Ap_.p,   y_.p,
                                   part_.p,   b_.p};
-                if (icc && sweep_mode_ == 0) build_windows(false);   // FP64 sweeps: FP64 windows
+                if (icc && !ml_on_ && sweep_mode_ == 0) build_windows(false);   // FP64 sweeps: FP64 windows
                 pcg_solve<double>(v, kAdjRtol, prm_.cg_max_iter, icc, n_eq, nnz_);
             }
             launch(k_adj_mu, RB, CG_BLOCK, 0, st_, n_eq, (const int *)part_of_row_.p, (const int *)S().id,
@@ -2287,7 +2567,7 @@ void Engine<D>::get_ppe(int *eq_idx, int *row_ptr, int *col, double *val, double
 template <int D>
 void Engine<D>::get_ic0(int *row_ptr, int *col, double *A, double *F, double *b, int *n_eq, long long *nnz)
 {
-    if (!ppe_valid_ || !ic0_valid_) throw CudaError("no IC(0) factor: run an ICCG step first", MPS_ERR_INVALID);
+    require_ic0();
     if (n_eq) *n_eq = n_eq_;
     if (nnz) *nnz = nnz_;
     if (!row_ptr) return;
@@ -2304,7 +2584,7 @@ template <int D>
 void Engine<D>::get_cell_blocks(int *cells, int *inv_off, double *inv, int *colour_rows, int *ncells,
                                 long long *ninv)
 {
-    if (!ppe_valid_ || !ic0_valid_) throw CudaError("no IC(0) factor: run an ICCG step first", MPS_ERR_INVALID);
+    require_ic0();
     int ncol = 1 << D;
     int nact = act_off_[ncol];
     if (ncells) *ncells = nact;
@@ -2320,13 +2600,13 @@ void Engine<D>::get_cell_blocks(int *cells, int *inv_off, double *inv, int *colo
 template <int D>
 void Engine<D>::apply_preconditioner(const double *r, double *z)
 {
-    if (!ppe_valid_ || !ic0_valid_) throw CudaError("no IC(0) factor: run an ICCG step first", MPS_ERR_INVALID);
+    require_ic0();
     if (!r || !z) throw CudaError("null vector", MPS_ERR_INVALID);
     int ne = n_eq_;
     MPS_CUDA(cudaMemcpyAsync(r_.p, r, sizeof(double) * ne, cudaMemcpyHostToDevice, st_));
     MPS_CUDA(cudaMemsetAsync(&sc_.p->done, 0, sizeof(int), st_));
     if (last_fp32_) {
-        if (sweep_mode_ == 0) build_windows(true);
+        if (ic_mode() == 0) build_windows(true);
         PcgBufs<float> v{A32_.p,      xf32_lo_.p, xf32_up_.p, pkv32_lo_.p, pkv32_up_.p, dinv32_.p, inv32_cm_.p,
                          inv32_rm_.p, x_.p,       r_.p,       z_.p,        p_.p,        Ap_.p,     y_.p,
                          part_.p,     b_.p};
@@ -2334,17 +2614,17 @@ void Engine<D>::apply_preconditioner(const double *r, double *z)
             v.xfc_lo = xfc32_lo_.p;
             v.xfc_up = xfc32_up_.p;
         }
-        if (sweep_mode_ == 2) launch_pcg<float>(v, true, 0);
+        if (ic_mode() == 2) launch_pcg<float>(v, true, 0);
         else {
             run_sweep<float>(v, true);
             run_sweep<float>(v, false);
         }
     } else {
-        if (sweep_mode_ == 0) build_windows(false);
+        if (ic_mode() == 0) build_windows(false);
         PcgBufs<double> v{A_.p,      xf_lo_.p, xf_up_.p, pk_val_lo_.p, pk_val_up_.p, dinv_.p, inv_cm_.p,
                           inv_rm_.p, x_.p,     r_.p,     z_.p,         p_.p,         Ap_.p,   y_.p,
                           part_.p,   b_.p};
-        if (sweep_mode_ == 2) launch_pcg<double>(v, true, 0);
+        if (ic_mode() == 2) launch_pcg<double>(v, true, 0);
         else {
             run_sweep<double>(v, true);
             run_sweep<double>(v, false);

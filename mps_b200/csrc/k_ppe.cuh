@@ -189,14 +189,15 @@ __device__ double ppe_rhs(const Src &src, const State<D> &s, const Consts &k, in
 }
 
 // One row of A and b.  Pass 1 walks the list in the reference's order for
-// the diagonal sum and the source term; pass 2 walks the neighbour cells in
+// the diagonal sum and the source term (bounded[row]: the row couples to a
+// known pressure); pass 2 walks the neighbour cells in
 // (colour, index) order so the off-diagonals come out with ascending
 // columns, the diagonal in its place.
 template <int D>
 __global__ void k_fill(CellSource<D> src, State<D> s, Consts k, const int *__restrict__ part_of_row,
                        const int *__restrict__ row_of, int n_eq, const int *__restrict__ row_ptr,
                        int *__restrict__ col, double *__restrict__ val, int *__restrict__ diagpos,
-                       double *__restrict__ b, unsigned *err)
+                       double *__restrict__ b, unsigned char *__restrict__ bounded, unsigned *err)
 {
     int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n_eq) return;
@@ -205,12 +206,16 @@ __global__ void k_fill(CellSource<D> src, State<D> s, Consts k, const int *__res
     load_vec<D>(pi, s.pos, i);
 
     double sum_w = 0.0;
+    bool known = k.diag_scale != k.coeff;   // the row sum is not zero
     src.for_each(i, [&](int j) {
         if (s.type[j] == DUMMY) return;
         double pj[D];
         load_vec<D>(pj, s.pos, j);
-        sum_w += kweight(sqrt(dist2<D>(pi, pj)), k.re_lap, k.rmin);
+        double w = kweight(sqrt(dist2<D>(pi, pj)), k.re_lap, k.rmin);
+        sum_w += w;
+        known = known || (row_of[j] < 0 && w > 0.0);
     });
+    bounded[r] = known;
     double diag = k.diag_scale * sum_w;
     b[r] = ppe_rhs<D>(src, s, k, i, pi);
 
@@ -550,13 +555,15 @@ __global__ void k_pack_fill(int n_eq, const int *__restrict__ diagpos, const int
     }
 }
 
-// (first row, unknowns) of every active cell
+// (first row, unknowns) of every active cell; the preconditioners number a
+// cell's unknowns in a byte
 __global__ void k_cell_desc(int nact, const int *__restrict__ acells, const int *__restrict__ cell_row0,
-                            const int *__restrict__ ucount, int2 *__restrict__ desc)
+                            const int *__restrict__ ucount, int2 *__restrict__ desc, unsigned *err)
 {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nact) return;
     int c = acells[k];
+    if (ucount[c] > 256) atomicOr(err, ERR_CELL_OVERFULL);
     desc[k] = make_int2(cell_row0[c], ucount[c]);
 }
 
