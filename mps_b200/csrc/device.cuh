@@ -262,6 +262,37 @@ struct CellSource {
     }
 };
 
+// Neighbours from the compact lists k_nbr_list wrote for the current cell
+// structure: the members CellSource finds, in its order.  Particles are taken
+// 32 at a time and entry k of the slice's particles is one 128-byte row, so a
+// warp with a thread per particle reads its lists coalesced.  A particle with
+// more than `pitch` neighbours walks the cells.
+template <int D>
+struct NbrSource {
+    CellSource<D> cells;
+    const int *idx;
+    const int *cnt;
+    int pitch;
+
+    template <class F>
+    __device__ __forceinline__ void for_each(int i, F &&f) const
+    {
+        int c = __ldg(&cnt[i]);
+        if (c > pitch) {
+            cells.for_each(i, f);
+            return;
+        }
+        const int *p = idx + (size_t)(i >> 5) * 32 * pitch + (i & 31);
+        int next = c > 0 ? __ldg(p) : 0;
+        for (int k = 1; k <= c; k++) {
+            int j = next;
+            p += 32;
+            if (k < c) next = __ldg(p);
+            f(j);
+        }
+    }
+};
+
 // Neighbours from a caller-supplied list (CSR of the reference's
 // NeighborList, entries in engine indices).
 struct ListSource {

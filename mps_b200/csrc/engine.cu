@@ -325,6 +325,7 @@ private:
 
     // ---- PPE
     DevArray<int> ucount_, ucol_, rs_, cell_row0_, row_of_, part_of_row_, rcount_, row_ptr_, diagpos_, col_;
+    DevArray<unsigned short> runs_, diagoff_;   // neighbour-cell runs of every row, [visit order][row]; diagonal
     DevArray<double> A_, F_, b_, x_, r_, z_, p_, Ap_, y_, part_, partials_, p2_;
     DevArray<float> A32_, xf32_lo_, xf32_up_, pkv32_lo_, pkv32_up_, inv32_cm_, inv32_rm_, dinv32_;
     DevArray<double> zprev_, dsum_;
@@ -426,6 +427,16 @@ private:
         c.re2 = k_.re_list2;
         return c;
     }
+
+    // the compact lists of the current structure, built on first use after a
+    // sort or a checkpoint load
+    NbrSource<D> near();
+    DevArray<int> nbr_idx_, nbr_cnt_;
+    DevArray<float4> keyf_;
+    bool nbr_valid_ = false;
+    int nbr_pitch_ = 0;
+    // bytes the lists may take; beyond, operators walk the cells
+    static constexpr double kNbrBytes = 24.0e9;
 
     void alloc_state();
     void build_grid();
@@ -571,30 +582,30 @@ Engine<D>::Engine(const mps_params_t &p, int capacity)
     MPS_CUDA(cudaMemsetAsync(err_.p, 0, sizeof(unsigned), st_));
 
     // Neighbour-cell visit orders for PPE rows: sorted by (colour, z, y, x).
-    signed char t3[8][27][3], t2[4][9][2];
+    constexpr int NCELL = D == 3 ? 27 : 9;
+    unsigned char visit[1 << D][NCELL], rank[1 << D][NCELL];
     for (int par = 0; par < (1 << D); par++) {
-        std::vector<std::array<int, 3>> offs;
-        for (int dz = (D == 3 ? -1 : 0); dz <= (D == 3 ? 1 : 0); dz++)
-            for (int dy = -1; dy <= 1; dy++)
-                for (int dx = -1; dx <= 1; dx++) offs.push_back({dx, dy, dz});
-        auto color = [&](const std::array<int, 3> &o) {
+        std::vector<int> cells(NCELL);
+        std::iota(cells.begin(), cells.end(), 0);
+        auto color = [&](int q) {
+            int o[3] = {q % 3 - 1, (q / 3) % 3 - 1, q / 9 - 1};
             int c = 0;
             for (int d = 0; d < D; d++) c |= (((par >> d) & 1) ^ (o[d] & 1)) << d;
             return c;
         };
-        std::stable_sort(offs.begin(), offs.end(),
-                         [&](const std::array<int, 3> &a, const std::array<int, 3> &b) {
-                             return color(a) < color(b);
-                         });
-        for (size_t q = 0; q < offs.size(); q++)
-            for (int d = 0; d < D; d++) {
-                if (D == 3) t3[par][q][d] = (signed char)offs[q][d];
-                else t2[par][q][d] = (signed char)offs[q][d];
-            }
+        std::stable_sort(cells.begin(), cells.end(), [&](int a, int b) { return color(a) < color(b); });
+        for (int q = 0; q < NCELL; q++) {
+            visit[par][q] = (unsigned char)cells[q];
+            rank[par][cells[q]] = (unsigned char)q;
+        }
     }
-    if (D == 3) MPS_CUDA(cudaMemcpyToSymbol(c_order3, t3, sizeof(t3)));
-    else MPS_CUDA(cudaMemcpyToSymbol(c_order2, t2, sizeof(t2)));
-
+    if (D == 3) {
+        MPS_CUDA(cudaMemcpyToSymbol(c_visit3, visit, sizeof(visit)));
+        MPS_CUDA(cudaMemcpyToSymbol(c_rank3, rank, sizeof(rank)));
+    } else {
+        MPS_CUDA(cudaMemcpyToSymbol(c_visit2, visit, sizeof(visit)));
+        MPS_CUDA(cudaMemcpyToSymbol(c_rank2, rank, sizeof(rank)));
+    }
 }
 
 template <int D>
@@ -646,6 +657,8 @@ void Engine<D>::alloc_state()
     rcount_.reserve(cap_ + 1);
     row_ptr_.reserve(cap_ + 1);
     diagpos_.reserve(cap_);
+    diagoff_.reserve(cap_);
+    runs_.reserve((size_t)(D == 3 ? 27 : 9) * cap_);
     inpos_.reserve(cap_);
     outpos_.reserve(cap_);
     for (auto *v : {&pk_len_lo_, &pk_len_up_, &pk_off_lo_, &pk_off_up_}) v->reserve((size_t)cap_ + 1);
@@ -819,6 +832,7 @@ void Engine<D>::update_params(const mps_params_t &p)
     if (regrid) {
         build_grid();
         structure_ = false;
+        nbr_valid_ = false;
     }
     compute_consts();
 }
@@ -868,6 +882,7 @@ void Engine<D>::upload_aos(const void *aos, int num)
     MPS_CUDA(cudaStreamSynchronize(st_));
     tstep_ = 0;
     structure_ = false;
+    nbr_valid_ = false;
     ppe_valid_ = false;
 }
 
@@ -902,6 +917,7 @@ void Engine<D>::upload_soa(const double *pos, const double *vel, const int *type
     MPS_CUDA(cudaStreamSynchronize(st_));
     tstep_ = 0;
     structure_ = false;
+    nbr_valid_ = false;
     ppe_valid_ = false;
 }
 
@@ -939,7 +955,51 @@ void Engine<D>::sort()
     cur_ ^= 1;
     g_.start = start_.p;
     structure_ = true;
+    nbr_valid_ = false;
     ppe_valid_ = false;
+}
+
+template <int D>
+NbrSource<D> Engine<D>::near()
+{
+    NbrSource<D> src{cells(), nullptr, nullptr, 0};
+    int n = n_;
+    nbr_cnt_.reserve((size_t)cap_);
+    if (!nbr_valid_ && n) {
+        // room for 1.4 times the neighbours of the rest lattice; a particle
+        // with more (a blow-up) walks the cells in every operator
+        double q = re_list_ / prm_.particle_distance;
+        int m = (int)std::min(q, 64.0), count = 0;
+        for (int z = (D == 3 ? -m : 0); z <= (D == 3 ? m : 0); z++)
+            for (int y = -m; y <= m; y++)
+                for (int x = -m; x <= m; x++) count += x * x + y * y + z * z < q * q;
+        nbr_pitch_ = ((int)(1.4 * count) + 15) & ~7;
+        double bytes = 4.0 * nbr_pitch_ * ((double)cap_ + 32.0);
+        if (bytes > kNbrBytes) nbr_pitch_ = 0;
+        if (nbr_pitch_) {
+            try {
+                nbr_idx_.reserve((size_t)nbr_pitch_ * (((size_t)cap_ + 31) & ~(size_t)31));
+            } catch (const CudaError &) {
+                (void)cudaGetLastError();
+                nbr_pitch_ = 0;
+            }
+        }
+        keyf_.reserve((size_t)cap_);
+        // FP32 coordinates are off by at most 2^-24 of the grid's extent (in
+        // cells); a squared distance near 1 by less than 8 times that (on
+        // wider grids FP32 decides nothing)
+        int ext = 1;
+        for (int d = 0; d < D; d++) ext = std::max(ext, g_.dims[d]);
+        float band = ext > 1000000 ? 1.0e30f : 8.0f * 1.1920929e-7f * (float)ext + 4.0e-6f;
+        launch(k_key_cells<D>, nblk(n, TPB), TPB, 0, st_, S(), g_, n, keyf_.p);
+        launch(k_nbr_list<D>, nblk(n, 128), 128, 0, st_, cells(), n, (const float4 *)keyf_.p, band, nbr_pitch_,
+               nbr_idx_.p, nbr_cnt_.p);
+        nbr_valid_ = true;
+    }
+    src.idx = nbr_idx_.p;
+    src.cnt = nbr_cnt_.p;
+    src.pitch = nbr_pitch_;
+    return src;
 }
 
 template <int D>
@@ -950,6 +1010,7 @@ void Engine<D>::unsort()
     MPS_CUDA(cudaGetLastError());
     cur_ ^= 1;
     structure_ = false;
+    nbr_valid_ = false;
     ppe_valid_ = false;
 }
 
@@ -960,7 +1021,7 @@ void Engine<D>::neighbor_search()
     if (n_) {
         // list lengths only: the reference aborts on overflow during the search
         lcnt_.reserve((size_t)n_ + 1);
-        launch(k_build_list<D>, nblk(n_, TPB), TPB, 0, st_, cells(), (const int *)S().id, n_, k_.max_nb, 0,
+        launch(k_build_list<D>, nblk(n_, TPB), TPB, 0, st_, near(), (const int *)S().id, n_, k_.max_nb, 0,
                (int *)nullptr, lcnt_.p, err_.p);
     }
     check_err();
@@ -1120,15 +1181,15 @@ void Engine<D>::explicit_stage(bool from_list)
     if (!n) return;
     int nb = nblk(n, TPB);
     if (from_list) launch(k_viscosity<D, ListSource>, nb, TPB, 0, st_, list(), S(), k_, n, 0);
-    else launch(k_viscosity<D, CellSource<D>>, nb, TPB, 0, st_, cells(), S(), k_, n, 0);
+    else launch(k_viscosity<D, NbrSource<D>>, nb, TPB, 0, st_, near(), S(), k_, n, 0);
     if (k_.st_on) {
         if (from_list) launch(k_surface_tension<D, ListSource>, nb, TPB, 0, st_, list(), S(), k_, n, 3);
-        else launch(k_surface_tension<D, CellSource<D>>, nb, TPB, 0, st_, cells(), S(), k_, n, 3);
+        else launch(k_surface_tension<D, NbrSource<D>>, nb, TPB, 0, st_, near(), S(), k_, n, 3);
     }
     if (k_.fr_on) {
         launch(k_explicit_part<D>, nb, TPB, 0, st_, S(), k_, n, 1);
         if (from_list) launch(k_friction<D, ListSource>, nb, TPB, 0, st_, list(), S(), k_, n);
-        else launch(k_friction<D, CellSource<D>>, nb, TPB, 0, st_, cells(), S(), k_, n);
+        else launch(k_friction<D, NbrSource<D>>, nb, TPB, 0, st_, near(), S(), k_, n);
         launch(k_explicit_part<D>, nb, TPB, 0, st_, S(), k_, n, 2);
     } else {
         launch(k_explicit_update<D>, nb, TPB, 0, st_, S(), k_, n);
@@ -1143,10 +1204,10 @@ void Engine<D>::explicit_stage(bool from_list)
     if (k_.collision_on) {
         if (D == 3) {
             if (from_list) launch(k_collision_list<D, ListSource>, nb, TPB, 0, st_, list(), S(), k_, n, vafter_.p);
-            else launch(k_collision_list<D, CellSource<D>>, nb, TPB, 0, st_, cells(), S(), k_, n, vafter_.p);
+            else launch(k_collision_list<D, NbrSource<D>>, nb, TPB, 0, st_, near(), S(), k_, n, vafter_.p);
         } else {
             sort();
-            launch(k_collision_allpairs<D>, nb, TPB, 0, st_, cells(), S(), k_, n, vafter_.p);
+            launch(k_collision_allpairs<D>, nb, TPB, 0, st_, near(), S(), k_, n, vafter_.p);
         }
         launch(k_collision_apply<D>, nb, TPB, 0, st_, S(), k_, n, vafter_.p);
     }
@@ -1160,12 +1221,12 @@ void Engine<D>::implicit_stage()
     sort();
     if (!n) return;
     int nb = nblk(n, TPB);
-    launch(k_density<D, CellSource<D>>, nb, TPB, 0, st_, cells(), S(), k_, n, err_.p, 1, 1);
+    launch(k_density<D, NbrSource<D>>, nb, TPB, 0, st_, near(), S(), k_, n, err_.p, 1, 1);
     MPS_CUDA(cudaEventRecord(ev_[1], st_));
     ppe(k_.clamp != 0);
     MPS_CUDA(cudaEventRecord(ev_[4], st_));
-    if (k_.cmps != 2) launch(k_pmin<D, CellSource<D>>, nb, TPB, 0, st_, cells(), S(), n, pmin_.p);
-    launch(k_gradient<D, CellSource<D>>, nb, TPB, 0, st_, cells(), S(), k_, n, k_.cmps != 2 ? pmin_.p : nullptr);
+    if (k_.cmps != 2) launch(k_pmin<D, NbrSource<D>>, nb, TPB, 0, st_, near(), S(), n, pmin_.p);
+    launch(k_gradient<D, NbrSource<D>>, nb, TPB, 0, st_, near(), S(), k_, n, k_.cmps != 2 ? pmin_.p : nullptr);
     launch(k_correct<D>, nb, TPB, 0, st_, S(), k_, n, 1, 1, 1);
     MPS_CUDA(cudaGetLastError());
 }
@@ -1296,8 +1357,8 @@ void Engine<D>::ml_build(int n_eq)
            ufpar_.p, (const int *)ufkeep_.p, mlfrac_.p, jdinv_.p);
     launch(k_ml_node_cells<D>, nblk(na1, TPB), TPB, 0, st_, na1, (const int *)mlact_.p, ml_.g[0], g_,
            (const int *)mlcell_.p, mlncell_.p);
-    launch(k_ml_cellmat<D>, nact, D == 3 ? 256 : 64, 0, st_, nact, (const int *)acells_.p, (const int2 *)adesc_.p, g_,
-           (const int *)cell_row0_.p, (const int *)ucount_.p, rp, ci, A, (const float *)mlfrac_.p, cap_, mlcm_.p);
+    launch(k_ml_cellmat<D>, nact, D == 3 ? 256 : 128, 0, st_, (const int *)acells_.p, (const int2 *)adesc_.p, g_, rp,
+           (const unsigned short *)runs_.p, ci, A, (const float *)mlfrac_.p, cap_, mlcm_.p);
     launch(k_ml_a1<D>, na1, L::STP, 0, st_, na1, (const int *)mlncell_.p, (const double *)mlcm_.p,
            ml_add_ && nl > 1, mlA_.p, mldinv_.p);
     for (int l = 0; l + 1 < nl; l++) {
@@ -1585,9 +1646,9 @@ void Engine<D>::ppe(bool clamp)
     }
     ml_on_ = prm_.solver_type == 1 && sweep_mode_ == 3 && ml_total_ > 0;
     if (ml_on_) ml_nodes(act_off_[ncol]);
-    CellSource<D> src = cells();
-    launch(k_row_count<D, CellSource<D>>, nblk(n_eq, TPB), TPB, 0, st_, src, s, part_of_row_.p, row_of_.p, n_eq,
-                                                                     rcount_.p);
+    NbrSource<D> src = near();
+    launch(k_row_count<D>, nblk(n_eq, ROW_BLOCK), ROW_BLOCK, 0, st_, src, s, (const int *)part_of_row_.p,
+           (const int *)row_of_.p, n_eq, cap_, rcount_.p, runs_.p, diagoff_.p);
     scan_exclusive<int>(rcount_.p, row_ptr_.p, n_eq, scanws_.p, st_);
     MPS_CUDA(cudaMemcpyAsync(int_host_, row_ptr_.p + n_eq, sizeof(int), cudaMemcpyDeviceToHost, st_));
     if (ml_on_)
@@ -1602,8 +1663,9 @@ void Engine<D>::ppe(bool clamp)
     col_.reserve(nnz);
     A_.reserve(nnz);
     bounded_.reserve(cap_);
-    launch(k_fill<D>, nblk(n_eq, 128), 128, 0, st_, src, s, k_, part_of_row_.p, row_of_.p, n_eq, row_ptr_.p, col_.p,
-                                                A_.p, diagpos_.p, b_.p, bounded_.p, err_.p);
+    launch(k_fill<D>, nblk(n_eq, ROW_BLOCK), ROW_BLOCK, 0, st_, src, s, k_, (const int *)part_of_row_.p,
+           (const int *)row_of_.p, n_eq, cap_, (const int *)row_ptr_.p, (const unsigned short *)runs_.p,
+           (const unsigned short *)diagoff_.p, col_.p, A_.p, diagpos_.p, b_.p, bounded_.p, err_.p);
     MPS_CUDA(cudaEventRecord(ev_[2], st_));
     bool icc = prm_.solver_type == 1;
     ic0_valid_ = icc;
@@ -2218,6 +2280,7 @@ void Engine<D>::state_load(const void *src)
     tstep_ = h.tstep;
     g_.start = start_.p;
     structure_ = true;
+    nbr_valid_ = false;
     ppe_valid_ = false;
 }
 
@@ -2357,15 +2420,15 @@ void Engine<D>::step_adjoint()
     }
     adj_rec_ = false;
     sort();
-    launch(k_density<D, CellSource<D>>, nb, TPB, 0, st_, cells(), S(), k_, n, err_.p, 1, 1);
+    launch(k_density<D, NbrSource<D>>, nb, TPB, 0, st_, near(), S(), k_, n, err_.p, 1, 1);
     ppe(false);
-    launch(k_pmin<D, CellSource<D>>, nb, TPB, 0, st_, cells(), S(), n, pmin_.p);
-    launch(k_gradient<D, CellSource<D>>, nb, TPB, 0, st_, cells(), S(), k_, n, (const double *)pmin_.p);
+    launch(k_pmin<D, NbrSource<D>>, nb, TPB, 0, st_, near(), S(), n, pmin_.p);
+    launch(k_gradient<D, NbrSource<D>>, nb, TPB, 0, st_, near(), S(), k_, n, (const double *)pmin_.p);
     check_err();
     // implicit part in reverse, on the fresh structure (state before the correction)
     launch(k_adj_seed<D>, nb, TPB, 0, st_, S(), k_, n, adj_);
-    launch(k_adj_pmin<D>, nb, TPB, 0, st_, cells(), S(), k_, n, adj_);
-    launch(k_adj_gradient<D>, nb, TPB, 0, st_, cells(), S(), k_, n, adj_);
+    launch(k_adj_pmin<D>, nb, TPB, 0, st_, near(), S(), k_, n, adj_);
+    launch(k_adj_gradient<D>, nb, TPB, 0, st_, near(), S(), k_, n, adj_);
     if (pseed) launch(k_adj_add, nb, TPB, 0, st_, n, (const double *)pseed_.p, adj_.lp);
     MPS_CUDA(cudaMemsetAsync(adj_.mu, 0, sizeof(double) * cap_, st_));
     int n_eq = n_eq_;
@@ -2395,27 +2458,27 @@ void Engine<D>::step_adjoint()
                    (const double *)x_.p, bnorm, adj_.mu);
         }
     }
-    launch(k_adj_ppe_pairs<D>, nb, TPB, 0, st_, cells(), S(), k_, n, adj_, (const int *)row_of_.p);
+    launch(k_adj_ppe_pairs<D>, nb, TPB, 0, st_, near(), S(), k_, n, adj_, (const int *)row_of_.p);
     // explicit part in reverse, on the previous step's structure
     state_load(snap_.p);
     if (k_.collision_on) {
         if (D == 3) {
-            launch(k_adj_collision<D, true>, nb, TPB, 0, st_, cells(), S(), k_, n, adj_, err_.p);
-            launch(k_adj_collision_gather<D>, nb, TPB, 0, st_, cells(), S(), n, adj_);
+            launch(k_adj_collision<D, true>, nb, TPB, 0, st_, near(), S(), k_, n, adj_, err_.p);
+            launch(k_adj_collision_gather<D>, nb, TPB, 0, st_, near(), S(), n, adj_);
         } else {
             // the 2-D collision runs on a structure sorted after the explicit update
-            launch(k_viscosity<D, CellSource<D>>, nb, TPB, 0, st_, cells(), S(), k_, n, 0);
+            launch(k_viscosity<D, NbrSource<D>>, nb, TPB, 0, st_, near(), S(), k_, n, 0);
             launch(k_explicit_update<D>, nb, TPB, 0, st_, S(), k_, n);
             sort();
-            launch(k_adj_collision<D, false>, nb, TPB, 0, st_, cells(), S(), k_, n, adj_, err_.p);
-            launch(k_adj_collision_gather<D>, nb, TPB, 0, st_, cells(), S(), n, adj_);
+            launch(k_adj_collision<D, false>, nb, TPB, 0, st_, near(), S(), k_, n, adj_, err_.p);
+            launch(k_adj_collision_gather<D>, nb, TPB, 0, st_, near(), S(), n, adj_);
             state_load(snap_.p);
         }
     } else {
         launch(k_adj_no_collision<D>, nb, TPB, 0, st_, S(), n, adj_);
     }
     launch(k_adj_accel<D>, nb, TPB, 0, st_, S(), k_, n, adj_);
-    launch(k_adj_viscosity<D>, nb, TPB, 0, st_, cells(), S(), k_, n, adj_);
+    launch(k_adj_viscosity<D>, nb, TPB, 0, st_, near(), S(), k_, n, adj_);
     {
         DriveT dv{};
         dv.A = prm_.wall_drive_amp;
@@ -2462,7 +2525,7 @@ void Engine<D>::get_neighbor_list(int *nb, int *cnt, int max_nb)
         hcnt = hc.data();
     }
     if (n)
-        launch(k_build_list<D>, nblk(n, TPB), TPB, 0, st_, cells(), (const int *)S().id, n, max_nb, 0,
+        launch(k_build_list<D>, nblk(n, TPB), TPB, 0, st_, near(), (const int *)S().id, n, max_nb, 0,
                (int *)nullptr, lcnt_.p, err_.p);
     MPS_CUDA(cudaMemcpyAsync(hcnt, lcnt_.p, sizeof(int) * n, cudaMemcpyDeviceToHost, st_));
     check_err();
@@ -2471,7 +2534,7 @@ void Engine<D>::get_neighbor_list(int *nb, int *cnt, int max_nb)
     for (int i = 0; i < n; i++) mc = std::max(mc, hcnt[i]);
     if (mc == 0) return;
     lout_.reserve((size_t)n * mc);
-    launch(k_build_list<D>, nblk(n, TPB), TPB, 0, st_, cells(), (const int *)S().id, n, max_nb, mc, lout_.p,
+    launch(k_build_list<D>, nblk(n, TPB), TPB, 0, st_, near(), (const int *)S().id, n, max_nb, mc, lout_.p,
            lcnt_.p, err_.p);
     MPS_CUDA(cudaMemcpy2DAsync(nb, sizeof(int) * (size_t)max_nb, lout_.p, sizeof(int) * mc, sizeof(int) * mc, n,
                                cudaMemcpyDeviceToHost, st_));
@@ -2676,7 +2739,7 @@ void Engine<D>::run_stage(int stage, const int *nb, const int *cnt, int max_nb, 
             launch(k_collision_list<D, ListSource>, bl, TPB, 0, st_, list(), S(), k_, n, vafter_.p);
         } else {
             sort();
-            launch(k_collision_allpairs<D>, bl, TPB, 0, st_, cells(), S(), k_, n, vafter_.p);
+            launch(k_collision_allpairs<D>, bl, TPB, 0, st_, near(), S(), k_, n, vafter_.p);
         }
         launch(k_collision_apply<D>, bl, TPB, 0, st_, S(), k_, n, vafter_.p);
         break;
@@ -2684,7 +2747,7 @@ void Engine<D>::run_stage(int stage, const int *nb, const int *cnt, int max_nb, 
         // the block-colour solver needs the cell structure; the caller's
         // list must be the one that structure produces
         sort();
-        launch(k_compare_list<D>, bl, TPB, 0, st_, cells(), S().id, n, lptr_.p, lidx_.p, err_.p);
+        launch(k_compare_list<D>, bl, TPB, 0, st_, near(), S().id, n, lptr_.p, lidx_.p, err_.p);
         check_err();
         ppe(false);
         break;

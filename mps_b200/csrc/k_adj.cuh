@@ -126,7 +126,7 @@ __global__ void k_adj_add(int n, const double *__restrict__ src, double *dst)
 // and, for fluid i, the adjoint that reaches P at that argument:
 //   psc_i = -Kc sum_j phi_ij (e_ij . lap_i),  phi = w / r^2, e_ij = x_j - x_i.
 template <int D>
-__global__ void k_adj_pmin(CellSource<D> src, State<D> s, Consts k, int n, Adj<D> a)
+__global__ void k_adj_pmin(NbrSource<D> src, State<D> s, Consts k, int n, Adj<D> a)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -169,7 +169,7 @@ __global__ void k_adj_pmin(CellSource<D> src, State<D> s, Consts k, int n, Adj<D
 //   dT_ij/dx_j = (P_j - Pmin_i) M(e),  M(e) = phi I + (phi'/r) e e^T,
 //   dT_ij/dx_i = -dT_ij/dx_j,  dT_ij/dP_j = phi e.
 template <int D>
-__global__ void k_adj_gradient(CellSource<D> src, State<D> s, Consts k, int n, Adj<D> a)
+__global__ void k_adj_gradient(NbrSource<D> src, State<D> s, Consts k, int n, Adj<D> a)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -265,7 +265,7 @@ __global__ void k_adj_mu(int n_eq, const int *__restrict__ part_of_row, const in
 //   dL/dn_i       = mu_i rhs_k / n0           (i a fluid unknown)
 // and the weights move x^c through r_ij.
 template <int D>
-__global__ void k_adj_ppe_pairs(CellSource<D> src, State<D> s, Consts k, int n, Adj<D> a,
+__global__ void k_adj_ppe_pairs(NbrSource<D> src, State<D> s, Consts k, int n, Adj<D> a,
                                 const int *__restrict__ row_of)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -341,7 +341,7 @@ __device__ __forceinline__ void collide_reverse(const double *vin, const double 
 // and u^c = v.  The partner terms go to the impulse records, gathered by
 // the partners in k_adj_collision_gather.
 template <int D, bool LIST>
-__global__ void k_adj_collision(CellSource<D> src, State<D> s, Consts k, int n, Adj<D> a, unsigned *err)
+__global__ void k_adj_collision(NbrSource<D> src, State<D> s, Consts k, int n, Adj<D> a, unsigned *err)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -448,7 +448,7 @@ __global__ void k_adj_collision(CellSource<D> src, State<D> s, Consts k, int n, 
 // adjoint feeds the wall drive's gradient) adds what every fluid i that hit
 // it recorded (i is in p's candidate set, which is symmetric).
 template <int D>
-__global__ void k_adj_collision_gather(CellSource<D> src, State<D> s, int n, Adj<D> a)
+__global__ void k_adj_collision_gather(NbrSource<D> src, State<D> s, int n, Adj<D> a)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -514,7 +514,7 @@ __global__ void k_adj_accel(State<D> s, Consts k, int n, Adj<D> a)
 // start, for the wall drive's gradient), and the per-particle gravity and
 // viscosity gradient terms.
 template <int D>
-__global__ void k_adj_viscosity(CellSource<D> src, State<D> s, Consts k, int n, Adj<D> a)
+__global__ void k_adj_viscosity(NbrSource<D> src, State<D> s, Consts k, int n, Adj<D> a)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;

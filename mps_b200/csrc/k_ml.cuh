@@ -314,125 +314,92 @@ __device__ __forceinline__ void ml_weights(const float *__restrict__ frac, int s
 
 // ---- Galerkin operators -------------------------------------------------------------------
 
-// Part of one cell's rows in A_1 = P^T A P, a CTA per active cell: thread
-// (q, k) sums, over the cell's rows i, the row's entries in neighbour cell q
-// weighted by their cells' corner k, then spreads the sum over the row's own
-// corners.  out[cell][own corner][node of the cell and its neighbours].
+// Part of one cell's rows in A_1 = P^T A P, a CTA per active cell, ML_RB rows
+// at a time: a thread per (row, neighbour cell) sums the row's entries there
+// weighted onto that cell's corners, the corner sums are added up on the 4^D
+// nodes of the cell and its neighbours, and the rows of that product are
+// spread over the cell's own corners: out[cell][own corner][node].
+// (A thread per neighbour cell and corner, every entry read by 2^D threads,
+// took 14.7 ms at 2.2 M rows.)
+constexpr int ML_RB = 8;
+
 template <int D>
-__global__ void __launch_bounds__(D == 3 ? 256 : 64)
-k_ml_cellmat(int nact, const int *__restrict__ acells, const int2 *__restrict__ desc, Grid<D> cg,
-             const int *__restrict__ cell_row0, const int *__restrict__ ucount, const int *__restrict__ row_ptr,
-             const int *__restrict__ col, const double *__restrict__ A, const float *__restrict__ frac, int stride,
-             double *__restrict__ out)
+__global__ void __launch_bounds__(D == 3 ? 256 : 128)
+k_ml_cellmat(const int *__restrict__ acells, const int2 *__restrict__ desc, Grid<D> cg,
+             const int *__restrict__ row_ptr, const unsigned short *__restrict__ runs, const int *__restrict__ col,
+             const double *__restrict__ A, const float *__restrict__ frac, int stride, double *__restrict__ out)
 {
     using L = MlDim<D>;
-    constexpr int NT = L::CELLS * L::NC;
-    constexpr int RB = 8;   // rows per pass
-    __shared__ double sm[L::NC][NT];
-    __shared__ double sw[RB][L::NC];
-    __shared__ int sb[RB][L::CELLS], se[RB][L::CELLS];
-    __shared__ int c0[L::CELLS], c1[L::CELLS];
-    int kk = blockIdx.x;
+    constexpr int BLOCK = D == 3 ? 256 : 128;
+    constexpr int ITEMS = (L::NC * L::W4 + BLOCK - 1) / BLOCK;
+    __shared__ double sp[ML_RB][L::CELLS][L::NC];
+    __shared__ double sn[ML_RB][L::W4];
+    __shared__ double sw[ML_RB][L::NC];
+    int kk = blockIdx.x, t = threadIdx.x;
     int2 dd = desc[kk];
-    int r0 = dd.x, m = dd.y;
-    if (threadIdx.x < L::CELLS) {
-        int q = threadIdx.x, rem = acells[kk];
-        int o[3] = {q % 3 - 1, (q / 3) % 3 - 1, q / 9 - 1};
-        int lin = 0;
-        bool in = true;
-        int cc[3];
+    int par = cell_parity<D>(cg, acells[kk]);
+    double acc[ITEMS];
 #pragma unroll
-        for (int d = 0; d < D; d++) { cc[d] = rem % cg.dims[d]; rem /= cg.dims[d]; }
+    for (int j = 0; j < ITEMS; j++) acc[j] = 0.0;
+    for (int i0 = 0; i0 < dd.y; i0 += ML_RB) {
+        int nr = min(ML_RB, dd.y - i0);
+        for (int w = t; w < nr * L::CELLS; w += BLOCK) {
+            int i = w / L::CELLS, q = w % L::CELLS;
+            int r = dd.x + i0 + i;
+            int base = row_ptr[r];
+            int e = base + runs[(size_t)q * stride + r];
+            int end = q + 1 < L::CELLS ? base + runs[(size_t)(q + 1) * stride + r] : row_ptr[r + 1];
+            double s[L::NC];
 #pragma unroll
-        for (int d = D - 1; d >= 0; d--) {
-            int x = cc[d] + o[d];
-            in = in && x >= 0 && x < cg.dims[d];
-            lin = lin * cg.dims[d] + x;
-        }
-        int u = in ? ucount[lin] : 0;
-        c0[q] = u ? cell_row0[lin] : 0;
-        c1[q] = u ? c0[q] + u : 0;
-    }
-    int t = threadIdx.x;
-    int q = t / L::NC, k = t % L::NC;
-    double acc[L::NC];
+            for (int k = 0; k < L::NC; k++) s[k] = 0.0;
+            for (; e < end; e++) {
+                double a = __ldg(&A[e]);
+                double wt[L::NC];
+                ml_weights<D>(frac, stride, __ldg(&col[e]), wt);
 #pragma unroll
-    for (int j = 0; j < L::NC; j++) acc[j] = 0.0;
-    __syncthreads();
-    for (int i0 = 0; i0 < m; i0 += RB) {
-        int nr = min(RB, m - i0);
-        for (int w = t; w < nr * L::CELLS; w += blockDim.x) {
-            int i = w / L::CELLS, cq = w % L::CELLS;
-            int a = row_ptr[r0 + i0 + i], e = row_ptr[r0 + i0 + i + 1];
-            int lo = a, hi = a;
-            if (c1[cq] > c0[cq]) {
-                // the sorted row's run of columns in [c0, c1)
-                int x = a, y = e;
-                while (x < y) {
-                    int mid = (x + y) >> 1;
-                    if (col[mid] < c0[cq]) x = mid + 1;
-                    else y = mid;
-                }
-                lo = x;
-                y = e;
-                while (x < y) {
-                    int mid = (x + y) >> 1;
-                    if (col[mid] < c1[cq]) x = mid + 1;
-                    else y = mid;
-                }
-                hi = x;
+                for (int k = 0; k < L::NC; k++) s[k] = fma(a, wt[k], s[k]);
             }
-            sb[i][cq] = lo;
-            se[i][cq] = hi;
+            int nb = visit_cell<D>(par, q);
+#pragma unroll
+            for (int k = 0; k < L::NC; k++) sp[i][nb][k] = s[k];
         }
         if (t < nr) {
             double w[L::NC];
-            ml_weights<D>(frac, stride, r0 + i0 + t, w);
+            ml_weights<D>(frac, stride, dd.x + i0 + t, w);
 #pragma unroll
             for (int j = 0; j < L::NC; j++) sw[t][j] = w[j];
         }
         __syncthreads();
-        if (t < NT) {
-            for (int i = 0; i < nr; i++) {
-                double s = 0.0;
-                for (int e = sb[i][q]; e < se[i][q]; e++) {
-                    int c = __ldg(&col[e]);
-                    double f = (double)__ldg(&frac[c]);
-                    double w = f < 0.0 ? 0.0 : ((k & 1) ? f : 1.0 - f);
+        // the (cell, corner) pairs that name one node, in a fixed order
+        for (int w = t; w < nr * L::W4; w += BLOCK) {
+            int i = w / L::W4, nd = w % L::W4;
+            int nx = nd % 4, ny = (nd / 4) % 4, nz = nd / 16;
+            double s = 0.0;
 #pragma unroll
-                    for (int d = 1; d < D; d++) {
-                        double fd = (double)__ldg(&frac[(size_t)d * stride + c]);
-                        w *= ((k >> d) & 1) ? fd : 1.0 - fd;
+            for (int kz = 0; kz < (D == 3 ? 2 : 1); kz++)
+#pragma unroll
+                for (int ky = 0; ky < 2; ky++)
+#pragma unroll
+                    for (int kx = 0; kx < 2; kx++) {
+                        int qx = nx - kx, qy = ny - ky, qz = D == 3 ? nz - kz : 0;
+                        if (qx < 0 || qx > 2 || qy < 0 || qy > 2 || qz < 0 || qz > 2) continue;
+                        s += sp[i][qx + 3 * qy + 9 * qz][kx + 2 * ky + 4 * kz];
                     }
-                    s = fma(__ldg(&A[e]), w, s);
-                }
+            sn[i][nd] = s;
+        }
+        __syncthreads();
 #pragma unroll
-                for (int j = 0; j < L::NC; j++) acc[j] = fma(sw[i][j], s, acc[j]);
-            }
+        for (int j = 0; j < ITEMS; j++) {
+            int w = t + j * BLOCK;
+            if (w < L::NC * L::W4)
+                for (int i = 0; i < nr; i++) acc[j] = fma(sw[i][w / L::W4], sn[i][w % L::W4], acc[j]);
         }
         __syncthreads();
     }
-    if (t < NT) {
 #pragma unroll
-        for (int j = 0; j < L::NC; j++) sm[j][t] = acc[j];
-    }
-    __syncthreads();
-    // nodes: the (q, k) that name the same node, in a fixed order
-    for (int w = t; w < L::NC * L::W4; w += blockDim.x) {
-        int j = w / L::W4, nd = w % L::W4;
-        int nx = nd % 4, ny = (nd / 4) % 4, nz = nd / 16;
-        double s = 0.0;
-#pragma unroll
-        for (int kz = 0; kz < (D == 3 ? 2 : 1); kz++)
-#pragma unroll
-            for (int ky = 0; ky < 2; ky++)
-#pragma unroll
-                for (int kx = 0; kx < 2; kx++) {
-                    int qx = nx - kx, qy = ny - ky, qz = D == 3 ? nz - kz : 0;
-                    if (qx < 0 || qx > 2 || qy < 0 || qy > 2 || qz < 0 || qz > 2) continue;
-                    s += sm[j][(qx + 3 * qy + 9 * qz) * L::NC + kx + 2 * ky + 4 * kz];
-                }
-        out[(size_t)kk * (L::NC * L::W4) + w] = s;
+    for (int j = 0; j < ITEMS; j++) {
+        int w = t + j * BLOCK;
+        if (w < L::NC * L::W4) out[(size_t)kk * (L::NC * L::W4) + w] = acc[j];
     }
 }
 

@@ -1,8 +1,8 @@
 // k_ops.cuh -- particle operators of the time step, FP64, thread per particle.
 //
-// Each kernel is templated on its neighbour source: CellSource (the sorted
-// cell structure, membership decided on the positions of the last sort) or
-// ListSource (a caller-supplied NeighborList).  The loop bodies restate the
+// Each kernel is templated on its neighbour source: NbrSource (the lists of
+// the sorted cell structure, membership decided on the positions of the last
+// sort) or ListSource (a caller-supplied NeighborList).  The loop bodies restate the
 // reference operators in their exact floating-point order:
 //   viscosity            operators.c:50-85 + simulation.c:31-40
 //   explicit update      simulation.c:52-67
@@ -319,7 +319,7 @@ __global__ void k_collision_list(Src src, State<D> s, Consts k, int n, double *_
 // structure sorted at the current positions; the ascending order is
 // produced by repeatedly taking the smallest index above the last one.
 template <int D>
-__global__ void k_collision_allpairs(CellSource<D> src, State<D> s, Consts k, int n,
+__global__ void k_collision_allpairs(NbrSource<D> src, State<D> s, Consts k, int n,
                                      double *__restrict__ vafter)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;

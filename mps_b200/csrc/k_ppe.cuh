@@ -34,15 +34,44 @@ struct CGScalars {
 
 // Visit order of the 3^D neighbour cells for PPE rows: by (colour, linear
 // index), so that the columns they contribute come out ascending.  One table
-// per parity of the centre cell; entries are offsets in {-1,0,1}^D.
-__constant__ signed char c_order3[8][27][3];
-__constant__ signed char c_order2[4][9][2];
+// per parity of the centre cell; entries number the neighbours
+// (x + 3 y + 9 z, the centre 13; 2-D x + 3 y, the centre 4), and its inverse.
+__constant__ unsigned char c_visit3[8][27], c_rank3[8][27];
+__constant__ unsigned char c_visit2[4][9], c_rank2[4][9];
 
 template <int D>
-__device__ __forceinline__ const signed char *order_entry(int par, int k)
+__device__ __forceinline__ int visit_cell(int par, int q) { return D == 3 ? c_visit3[par][q] : c_visit2[par][q]; }
+
+template <int D>
+__device__ __forceinline__ int visit_rank(int par, int nb) { return D == 3 ? c_rank3[par][nb] : c_rank2[par][nb]; }
+
+// Parity of a cell's coordinates (its colour).
+template <int D>
+__device__ __forceinline__ int cell_parity(const Grid<D> &g, int c)
 {
-    if (D == 3) return c_order3[par][k];
-    return c_order2[par][k];
+    int par = 0;
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+        par |= ((c % g.dims[d]) & 1) << d;
+        c /= g.dims[d];
+    }
+    return par;
+}
+
+// Number of a neighbouring cell from the difference of the linear indices.
+template <int D>
+__device__ __forceinline__ int neighbour_cell(const Grid<D> &g, int diff)
+{
+    int nx = g.dims[0];
+    if (D == 2) {
+        int v = diff + nx + 1, y = v / nx;
+        return v - y * nx + 3 * y;
+    }
+    int nxy = nx * g.dims[1];
+    int v = diff + nxy + nx + 1, z = v / nxy;
+    v -= z * nxy;
+    int y = v / nx;
+    return v - y * nx + 3 * y + 9 * z;
 }
 
 __device__ __forceinline__ bool is_unknown(int type, int surf)
@@ -127,16 +156,47 @@ __global__ void k_offgrid_rows(State<D> s, int first, int n, int *__restrict__ r
 
 // ---- assembly --------------------------------------------------------------
 
-template <int D, class Src>
-__global__ void k_row_count(Src src, State<D> s, const int *__restrict__ part_of_row,
-                            const int *__restrict__ row_of, int n_eq, int *__restrict__ rcount)
+constexpr int ROW_BLOCK = 128;
+
+// Entries of every row, the start of each neighbour cell's run in it
+// (runs[q][row], q in visit order, so columns ascend along the row) and the
+// diagonal's place.
+template <int D>
+__global__ void __launch_bounds__(ROW_BLOCK)
+k_row_count(NbrSource<D> src, State<D> s, const int *__restrict__ part_of_row, const int *__restrict__ row_of,
+            int n_eq, int stride, int *__restrict__ rcount, unsigned short *__restrict__ runs,
+            unsigned short *__restrict__ diagoff)
 {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int CELLS = D == 3 ? 27 : 9;
+    __shared__ unsigned short cnt[CELLS][ROW_BLOCK];
+    int r = blockIdx.x * ROW_BLOCK + threadIdx.x;
     if (r >= n_eq) return;
+#pragma unroll
+    for (int q = 0; q < CELLS; q++) cnt[q][threadIdx.x] = 0;
     int i = part_of_row[r];
-    int cnt = 1;
-    src.for_each(i, [&](int j) { cnt += (s.type[j] != DUMMY && row_of[j] >= 0); });
-    rcount[r] = cnt;
+    int ci = s.cell[i];
+    const Grid<D> &g = src.cells.g;
+    int prev = ci, nb = CELLS / 2, below = 0;
+    src.for_each(i, [&](int j) {
+        if (row_of[j] < 0) return;
+        int c = s.cell[j];
+        if (c != prev) {
+            prev = c;
+            nb = neighbour_cell<D>(g, c - ci);
+        }
+        cnt[nb][threadIdx.x]++;
+        below += c == ci && j < i;
+    });
+    cnt[CELLS / 2][threadIdx.x]++;
+    int par = cell_parity<D>(g, ci);
+    int off = 0;
+    for (int q = 0; q < CELLS; q++) {
+        int nq = visit_cell<D>(par, q);
+        runs[(size_t)q * stride + r] = (unsigned short)off;
+        if (nq == CELLS / 2) diagoff[r] = (unsigned short)(off + below);
+        off += cnt[nq][threadIdx.x];
+    }
+    rcount[r] = off;
 }
 
 // Right-hand side of one unknown row (pressure_solver.c:328-362, 524-529).
@@ -188,23 +248,29 @@ __device__ double ppe_rhs(const Src &src, const State<D> &s, const Consts &k, in
     return k.rhs_k * (s.n[i] - n0) / n0;
 }
 
-// One row of A and b.  Pass 1 walks the list in the reference's order for
-// the diagonal sum and the source term (bounded[row]: the row couples to a
-// known pressure); pass 2 walks the neighbour cells in
-// (colour, index) order so the off-diagonals come out with ascending
-// columns, the diagonal in its place.
+// One row of A and b: the row's neighbours in the reference's order for the
+// diagonal sum and the source term (bounded[row]: the row couples to a known
+// pressure), each off-diagonal at its place in its cell's run.  A neighbour's
+// weight is computed once, for the sum and the entry.
 template <int D>
-__global__ void k_fill(CellSource<D> src, State<D> s, Consts k, const int *__restrict__ part_of_row,
-                       const int *__restrict__ row_of, int n_eq, const int *__restrict__ row_ptr,
-                       int *__restrict__ col, double *__restrict__ val, int *__restrict__ diagpos,
-                       double *__restrict__ b, unsigned char *__restrict__ bounded, unsigned *err)
+__global__ void __launch_bounds__(ROW_BLOCK)
+k_fill(NbrSource<D> src, State<D> s, Consts k, const int *__restrict__ part_of_row,
+       const int *__restrict__ row_of, int n_eq, int stride, const int *__restrict__ row_ptr,
+       const unsigned short *__restrict__ runs, const unsigned short *__restrict__ diagoff, int *__restrict__ col,
+       double *__restrict__ val, int *__restrict__ diagpos, double *__restrict__ b,
+       unsigned char *__restrict__ bounded, unsigned *err)
 {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
+    int r = blockIdx.x * ROW_BLOCK + threadIdx.x;
     if (r >= n_eq) return;
     int i = part_of_row[r];
     double pi[D];
     load_vec<D>(pi, s.pos, i);
-
+    const Grid<D> &g = src.cells.g;
+    int ci = s.cell[i];
+    int par = cell_parity<D>(g, ci);
+    int base = row_ptr[r], end = row_ptr[r + 1];
+    int dpos = base + diagoff[r];
+    int prev = -1, pos = base, placed = 1;
     double sum_w = 0.0;
     bool known = k.diag_scale != k.coeff;   // the row sum is not zero
     src.for_each(i, [&](int j) {
@@ -213,60 +279,30 @@ __global__ void k_fill(CellSource<D> src, State<D> s, Consts k, const int *__res
         load_vec<D>(pj, s.pos, j);
         double w = kweight(sqrt(dist2<D>(pi, pj)), k.re_lap, k.rmin);
         sum_w += w;
-        known = known || (row_of[j] < 0 && w > 0.0);
+        int rj = row_of[j];
+        if (rj < 0) {
+            known = known || w > 0.0;
+            return;
+        }
+        int c = s.cell[j];
+        if (c != prev) {
+            prev = c;
+            pos = base + runs[(size_t)visit_rank<D>(par, neighbour_cell<D>(g, c - ci)) * stride + r];
+        }
+        if (pos == dpos) pos++;
+        if (pos < end) {
+            col[pos] = rj;
+            val[pos] = k.neg_coeff * w;
+        }
+        pos++;
+        placed++;
     });
     bounded[r] = known;
-    double diag = k.diag_scale * sum_w;
+    diagpos[r] = dpos;
+    col[dpos] = r;
+    val[dpos] = k.diag_scale * sum_w;
     b[r] = ppe_rhs<D>(src, s, k, i, pi);
-
-    int c = s.cell[i];
-    int cc[D];
-    int rem = c;
-#pragma unroll
-    for (int d = 0; d < D; d++) { cc[d] = rem % src.g.dims[d]; rem /= src.g.dims[d]; }
-    int par = 0;
-#pragma unroll
-    for (int d = 0; d < D; d++) par |= (cc[d] & 1) << d;
-    double ki[D];
-    load_vec<D>(ki, s.key, i);
-    int pos = row_ptr[r];
-    int end = row_ptr[r + 1];
-    const int NC = (D == 3) ? 27 : 9;
-    for (int q = 0; q < NC; q++) {
-        const signed char *off = order_entry<D>(par, q);
-        int lin = 0;
-        bool inside = true;
-#pragma unroll
-        for (int d = D - 1; d >= 0; d--) {
-            int x = cc[d] + off[d];
-            if (x < 0 || x >= src.g.dims[d]) inside = false;
-            lin = lin * src.g.dims[d] + x;
-        }
-        if (!inside) continue;
-        for (int t = src.g.start[lin]; t < src.g.start[lin + 1]; t++) {
-            if (t == i) {
-                diagpos[r] = pos;
-                col[pos] = r;
-                val[pos] = diag;
-                pos++;
-                continue;
-            }
-            int rj = row_of[t];
-            if (rj < 0 || s.type[t] == DUMMY) continue;
-            double kt[D];
-            load_vec<D>(kt, s.key, t);
-            if (!(dist2<D>(ki, kt) < src.re2)) continue;
-            double pt[D];
-            load_vec<D>(pt, s.pos, t);
-            double w = kweight(sqrt(dist2<D>(pi, pt)), k.re_lap, k.rmin);
-            if (pos < end) {
-                col[pos] = rj;
-                val[pos] = k.neg_coeff * w;
-            }
-            pos++;
-        }
-    }
-    if (pos != end) atomicOr(err, ERR_COLORING);
+    if (placed != end - base) atomicOr(err, ERR_COLORING);
 }
 
 // ---- IC(0) factorisation ---------------------------------------------------

@@ -114,11 +114,100 @@ __global__ void k_unsort(State<D> dst, State<D> src, const int *__restrict__ whe
     dst.cell[r] = -1;
 }
 
+// ---- compact lists of the cell structure ---------------------------------------
+//
+// Every operator of a step visits the same neighbours: a seventh of the
+// candidates in the 3^D cells.  Testing them in each operator costs a pass
+// over all candidates in FP64 and, worse, runs the operator's body (square
+// root and division) for every candidate that any lane of the warp accepts.
+// The lists are built once per sort and the operators run over accepted
+// neighbours only.
+//
+// The test is bit for bit that of CellSource.  Positions in cell units are
+// first compared in FP32 (one 16-byte load per candidate and half the issue
+// cost); only a candidate within `band` of the radius, where FP32 cannot
+// decide, is tested in FP64.
+
+// Sort keys in cell units, FP32.
+template <int D>
+__global__ void k_key_cells(State<D> s, Grid<D> g, int n, float4 *__restrict__ kf)
+{
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float f[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int d = 0; d < D; d++) f[d] = (float)((s.key[d][i] - g.origin[d]) * g.cs_inv);
+    kf[i] = make_float4(f[0], f[1], f[2], f[3]);
+}
+
+// Lists of the current structure: idx[(slice * pitch + k) * 32 + lane], cnt
+// the number of neighbours (those past `pitch` are counted, not stored).
+template <int D>
+__global__ void k_nbr_list(CellSource<D> src, int n, const float4 *__restrict__ kf, float band, int pitch,
+                           int *__restrict__ idx, int *__restrict__ cnt)
+{
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int c = src.cell[i];
+    int k = 0;
+    if (c >= 0) {
+        const Grid<D> &g = src.g;
+        float4 me = kf[i];
+        double ki[D];
+#pragma unroll
+        for (int d = 0; d < D; d++) ki[d] = src.key[d][i];
+        int cc[D];
+        int rem = c;
+#pragma unroll
+        for (int d = 0; d < D; d++) { cc[d] = rem % g.dims[d]; rem /= g.dims[d]; }
+        int x0 = cc[0] > 0 ? cc[0] - 1 : 0;
+        int x1 = cc[0] < g.dims[0] - 1 ? cc[0] + 1 : g.dims[0] - 1;
+        int y0 = cc[1] > 0 ? cc[1] - 1 : 0;
+        int y1 = cc[1] < g.dims[1] - 1 ? cc[1] + 1 : g.dims[1] - 1;
+        int z0 = 0, z1 = 0;
+        if (D == 3) {
+            z0 = cc[D - 1] > 0 ? cc[D - 1] - 1 : 0;
+            z1 = cc[D - 1] < g.dims[D - 1] - 1 ? cc[D - 1] + 1 : g.dims[D - 1] - 1;
+        }
+        int *out = idx + (size_t)(i >> 5) * 32 * pitch + (i & 31);
+        for (int z = z0; z <= z1; z++) {
+            for (int y = y0; y <= y1; y++) {
+                int base = (D == 3) ? (z * g.dims[1] + y) * g.dims[0] : y * g.dims[0];
+                int t0 = g.start[base + x0], t1 = g.start[base + x1 + 1];
+#pragma unroll 4
+                for (int t = t0; t < t1; t++) {
+                    float4 o = __ldg(&kf[t]);
+                    float dx = o.x - me.x, dy = o.y - me.y;
+                    float d2 = fmaf(dx, dx, dy * dy);
+                    if (D == 3) {
+                        float dz = o.z - me.z;
+                        d2 = fmaf(dz, dz, d2);
+                    }
+                    if (d2 < 1.0f + band) {
+                        bool hit = t != i;
+                        if (d2 >= 1.0f - band) {
+                            double kt[D];
+#pragma unroll
+                            for (int d = 0; d < D; d++) kt[d] = src.key[d][t];
+                            hit = hit && dist2<D>(ki, kt) < src.re2;
+                        }
+                        if (hit) {
+                            if (k < pitch) out[(size_t)k * 32] = t;
+                            k++;
+                        }
+                    }
+                }
+            }
+        }
+    }
+    cnt[i] = k;
+}
+
 // Neighbour list in the reference's layout (rows by reference index,
 // entries as reference indices, reference order).  Row r starts at
 // out_nb[r * pitch]; rows longer than max_nb raise the overflow flag.
 template <int D>
-__global__ void k_build_list(CellSource<D> src, const int *__restrict__ id, int n, int max_nb, int pitch,
+__global__ void k_build_list(NbrSource<D> src, const int *__restrict__ id, int n, int max_nb, int pitch,
                              int *__restrict__ out_nb, int *__restrict__ out_cnt, unsigned *err)
 {
     int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -181,7 +270,7 @@ __global__ void k_cell_ref_order(const int *__restrict__ cell, const int *__rest
 // Compare a caller's list (CSR by reference index, reference indices) with
 // the cell structure's list, entry by entry.
 template <int D>
-__global__ void k_compare_list(CellSource<D> src, const int *__restrict__ id, int n,
+__global__ void k_compare_list(NbrSource<D> src, const int *__restrict__ id, int n,
                                const int *__restrict__ lptr, const int *__restrict__ lidx, unsigned *err)
 {
     int q = blockIdx.x * blockDim.x + threadIdx.x;
