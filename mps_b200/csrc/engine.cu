@@ -85,6 +85,13 @@ constexpr int TPB = 256;             // threads per block, particle kernels
 constexpr int RED_BLOCKS = 148 * 8;  // fixed grid of the reduction kernels: full occupancy at 256 threads
 constexpr int CG_BATCH = 8;          // CG iterations between convergence reads
 
+// Grid of a reduction kernel over `items`, `per_block` in a block at a time:
+// no more blocks than there is work for (each one takes a ticket).
+static inline int red_grid(long long items, int per_block)
+{
+    return (int)std::max(1LL, std::min((long long)RED_BLOCKS, (items + per_block - 1) / per_block));
+}
+
 template <int D>
 struct AosLayout {
     static constexpr int size = (24 * D + 28 + 7) / 8 * 8;   // 104 (3-D), 80 (2-D)
@@ -360,25 +367,26 @@ private:
     std::vector<int> inv_col_off_;         // block-inverse offsets at the colour boundaries
     // ---- multilevel preconditioner
     MlLevels ml_{};                        // grids of the cell grid; lo of the current structure
+    MlLevels mlc_{};                       // those the current solve uses
     int ml_total_ = 0;                     // nodes of all grids, margins included (0: too many)
     bool ml_on_ = false;                   // the current solve uses it
     bool ml_add_ = false;                  // additive first grid
-    int ml_l0_ = 0;                        // first grid of the cluster kernel
-    // unknowns below which the first grid is additive (MPS_ML_ADD): two products
-    // with its operator fewer per iteration for about a third more iterations,
-    // which pays where an iteration is a chain of short launches; and nodes
-    // up to which a grid runs in the cluster kernel (MPS_ML_CLUSTER): beyond,
-    // a product streams more of the operator than one cluster's SMs can draw
-    int ml_add_rows_ = 60000, ml_cl_nodes_ = 4096;
-    DevArray<int> mlflag_, mlpos_, mlmap_, mlact_, mlcell_, mlncell_, mlcnode_, ufpar_, ufkeep_, mlscan_;
-    DevArray<unsigned char> bounded_;
+    int ml_ld_ = 0;                        // the dense grid
+    // unknowns below which the first grid is additive (MPS_ML_ADD): a product
+    // with its operator and with C fewer per iteration for about a third more
+    // iterations, which pays where an iteration is a chain of short launches;
+    // and nodes up to which a grid's V-cycle is dense (MPS_ML_DENSE)
+    int ml_add_rows_ = 60000, ml_dense_ = ML_DENSE;
+    DevArray<int> mlflag_, mlpos_, mlmap_, mlact_, mlcell_, mlncell_, mlcnode_, mlunder_, mlabove_, ufpar_, ufkeep_, mlscan_;
+    DevArray<unsigned char> bounded_, mlpar_;
     DevArray<float> mlfrac_;
-    DevArray<double> mlcm_, mlA_, mldinv_, mlb_, mlx_, mly_, mlinv_, mlcsum_, jdinv_;
+    DevArray<double> mlcm_, mlA_, mlC_, mldinv_, mlb_, mlx_, mly_, mlbd_, mlM_[2], mlMC_, mlcsum_, jdinv_;
+    const double *mlM_last_ = nullptr;     // the dense V-cycle of the current solve
     void ml_levels();
     void ml_nodes(int nact);
     void ml_build(int n_eq);
     MlVecs ml_vecs() const;
-    const double *ml_result() const { return ml_.nl == 1 || ml_add_ ? mlx_.p : mly_.p; }
+    const double *ml_result() const { return ml_ld_ == 0 ? mlx_.p : mly_.p; }
     void ml_update(bool restrict_only, double *x, double *r, const double *p, const double *Ap);
     void ml_cycle();
     void ml_prolong(bool rz, const double *r, double *z);
@@ -525,7 +533,7 @@ Engine<D>::Engine(const mps_params_t &p, int capacity)
         sweep_mode_ = (v == 0 || v == 1 || v == 3) ? v : 2;
     }
     if (const char *e = std::getenv("MPS_ML_ADD")) ml_add_rows_ = std::max(0, std::atoi(e));
-    if (const char *e = std::getenv("MPS_ML_CLUSTER")) ml_cl_nodes_ = std::max(0, std::atoi(e));
+    if (const char *e = std::getenv("MPS_ML_DENSE")) ml_dense_ = std::min(ML_DENSE, std::max(0, std::atoi(e)));
     if (const char *e = std::getenv("MPS_SWEEP_HB")) head_batch_ = std::atoi(e) == 8 ? 8 : 4;
     if (const char *e = std::getenv("MPS_SWEEP_OCC")) sweep_occ_ = std::atoi(e) == 8 ? 8 : 6;
     if (const char *e = std::getenv("MPS_SWEEP_HR")) head_rows_ = std::atoi(e) == 2 ? 2 : 1;
@@ -557,6 +565,8 @@ Engine<D>::Engine(const mps_params_t &p, int capacity)
     for (auto &e : pev_) MPS_CUDA(cudaEventCreate(&e));
     MPS_CUDA(cudaMallocHost((void **)&sc_host_, sizeof(CGScalars)));
     MPS_CUDA(cudaMallocHost((void **)&int_host_, 64 * sizeof(int)));
+    MPS_CUDA(cudaFuncSetAttribute(k_ml_inverse<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(sizeof(double) * ML_COARSEST * ML_COARSEST)));
     // the staged in-cell sweeps take more than the default 48 KB of dynamic shared memory
     MPS_CUDA(cudaFuncSetAttribute(k_sweep_colour<true, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(sizeof(double) * CELL_STAGE_MAX)));
@@ -723,7 +733,7 @@ void Engine<D>::build_grid()
 }
 
 // The nested grids over the cell grid: nodes on the cell corners, then every
-// other node until the box holds at most ML_COARSEST nodes.
+// other node until the box holds at most ML_BOX nodes.
 template <int D>
 void Engine<D>::ml_levels()
 {
@@ -732,7 +742,8 @@ void Engine<D>::ml_levels()
     int n[3] = {g_.dims[0] + 1, g_.dims[1] + 1, D == 3 ? g_.dims[D - 1] + 1 : 1};
     for (;;) {
         MlGrid &m = ml_.g[ml_.nl++];
-        long long s1 = n[0] + 4, s2 = s1 * (n[1] + 4), size = D == 3 ? s2 * (n[2] + 4) : s2;
+        constexpr int P = ML_PAD;
+        long long s1 = n[0] + 2 * P, s2 = s1 * (n[1] + 2 * P), size = D == 3 ? s2 * (n[2] + 2 * P) : s2;
         if (first + size > 0x7fffff00LL) {
             ml_total_ = 0;   // the grids' node numbers would not fit: IC(0) instead
             return;
@@ -742,9 +753,9 @@ void Engine<D>::ml_levels()
         m.s2 = (int)s2;
         m.first = (int)first;
         m.size = (int)size;
-        m.base = (int)(first + 2 + 2 * s1 + (D == 3 ? 2 * s2 : 0));
+        m.base = (int)(first + P + P * s1 + (D == 3 ? P * s2 : 0));
         first += size;
-        if ((long long)n[0] * n[1] * n[2] <= ML_COARSEST) break;
+        if ((long long)n[0] * n[1] * n[2] <= ML_BOX) break;
         for (int d = 0; d < D; d++) n[d] = n[d] / 2 + 1;
     }
     ml_total_ = (int)first;
@@ -1310,12 +1321,19 @@ MlVecs Engine<D>::ml_vecs() const
     v.x = mlx_.p;
     v.y = mly_.p;
     v.act = mlact_.p;
+    v.amap = mlmap_.p;
     v.A = mlA_.p;
+    v.under = mlunder_.p;
+    v.above = mlabove_.p;
+    v.parity = mlpar_.p;
+    v.C = mlC_.p;
     v.dinv = mldinv_.p;
     v.ncell = mlncell_.p;
     v.csum = mlcsum_.p;
-    v.inv = mlinv_.p;
-    v.na1 = ml_.lo[1];
+    v.bd = mlbd_.p;
+    v.M = mlM_last_;
+    v.ld = ml_ld_;
+    v.na1 = mlc_.lo[1];
     return v;
 }
 
@@ -1326,10 +1344,17 @@ void Engine<D>::ml_build(int n_eq)
 {
     using L = MlDim<D>;
     State<D> &s = S();
-    int nl = ml_.nl, na1 = ml_.lo[1], nall = ml_.lo[nl], nact = act_off_[1 << D];
+    mlc_ = ml_;
+    for (int l = 0; l < ml_.nl; l++)
+        if (ml_.lo[l + 1] - ml_.lo[l] <= ML_COARSEST) {
+            mlc_.nl = l + 1;
+            break;
+        }
+    int nl = mlc_.nl, na1 = mlc_.lo[1], nall = mlc_.lo[nl], nact = act_off_[1 << D];
     ml_add_ = n_eq < ml_add_rows_;
-    ml_l0_ = 0;
-    while (ml_l0_ + 1 < nl && ml_.lo[ml_l0_ + 1] - ml_.lo[ml_l0_] > ml_cl_nodes_) ml_l0_++;
+    ml_ld_ = 0;
+    while (ml_ld_ + 1 < nl && mlc_.lo[ml_ld_ + 1] - mlc_.lo[ml_ld_] > ml_dense_) ml_ld_++;
+    ml_add_ = ml_add_ && ml_ld_ > 0;
     for (auto *v : {&mlb_, &mlx_, &mly_}) {
         v->reserve((size_t)ml_total_);
         MPS_CUDA(cudaMemsetAsync(v->p, 0, sizeof(double) * (size_t)ml_total_, st_));
@@ -1337,9 +1362,13 @@ void Engine<D>::ml_build(int n_eq)
     mlncell_.reserve((size_t)L::NC * na1);
     mlcm_.reserve((size_t)nact * L::NC * L::W4);
     mlA_.reserve((size_t)nall * L::STP);
+    mlC_.reserve((size_t)(nall - na1) * L::W7P + 1);
     mldinv_.reserve((size_t)nall);
     mlcsum_.reserve((size_t)nact * L::NC);
-    mlinv_.reserve((size_t)ML_COARSEST * ML_COARSEST);
+    mlbd_.reserve((size_t)std::max(ML_DENSE, ML_COARSEST));
+    mlunder_.reserve((size_t)nall);
+    mlabove_.reserve((size_t)nall);
+    mlpar_.reserve((size_t)nall);
     mlfrac_.reserve((size_t)D * cap_);
     jdinv_.reserve((size_t)cap_);
     ufpar_.reserve((size_t)cap_);
@@ -1360,16 +1389,34 @@ void Engine<D>::ml_build(int n_eq)
     launch(k_ml_cellmat<D>, nact, D == 3 ? 256 : 128, 0, st_, (const int *)acells_.p, (const int2 *)adesc_.p, g_, rp,
            (const unsigned short *)runs_.p, ci, A, (const float *)mlfrac_.p, cap_, mlcm_.p);
     launch(k_ml_a1<D>, na1, L::STP, 0, st_, na1, (const int *)mlncell_.p, (const double *)mlcm_.p,
-           ml_add_ && nl > 1, mlA_.p, mldinv_.p);
+           ml_add_, mlA_.p, mldinv_.p);
     for (int l = 0; l + 1 < nl; l++) {
-        int lof = ml_.lo[l], loc = ml_.lo[l + 1], nc = ml_.lo[l + 2] - loc;
-        launch(k_ml_galerkin<D>, nc, L::STP, 0, st_, ml_.g[l], ml_.g[l + 1], lof, loc, (const int *)mlact_.p,
+        int lof = mlc_.lo[l], loc = mlc_.lo[l + 1], nc = mlc_.lo[l + 2] - loc;
+        launch(k_ml_galerkin<D>, nc, L::STP, 0, st_, mlc_.g[l], mlc_.g[l + 1], lof, loc, (const int *)mlact_.p,
                (const int *)mlmap_.p, (const double *)mlA_.p + (size_t)lof * L::STP,
-               mlA_.p + (size_t)loc * L::STP, mldinv_.p + loc);
+               (const double *)mldinv_.p + lof, mlA_.p + (size_t)loc * L::STP, mldinv_.p + loc,
+               mlC_.p + (size_t)(loc - na1) * L::W7P);
     }
-    int lo = ml_.lo[nl - 1], n = nall - lo;
-    launch(k_ml_inverse<D>, 1, 1024, sizeof(double) * (size_t)(n * n + n), st_, ml_.g[nl - 1], lo, n,
-           (const int *)mlact_.p, (const int *)mlmap_.p, (const double *)mlA_.p + (size_t)lo * L::STP, mlinv_.p);
+    launch(k_ml_tables<D>, nblk(nall, TPB), TPB, 0, st_, mlc_, (const int *)mlact_.p, mlunder_.p, mlabove_.p, mlpar_.p);
+    int lo = mlc_.lo[nl - 1], n = nall - lo;
+    mlM_[0].reserve((size_t)ML_COARSEST * ML_COARSEST);
+    launch(k_ml_inverse<D>, 1, 1024, sizeof(double) * ML_COARSEST * ML_COARSEST, st_, mlc_.g[nl - 1], lo, n,
+           (const int *)mlact_.p, (const int *)mlmap_.p, (const double *)mlA_.p + (size_t)lo * L::STP, mlM_[0].p);
+    int cur = 0;
+    for (int l = nl - 2; l >= ml_ld_; l--) {
+        int lof = mlc_.lo[l], loc = mlc_.lo[l + 1], nf = loc - lof, nc = mlc_.lo[l + 2] - loc;
+        mlMC_.reserve((size_t)nf * nc);
+        mlM_[cur ^ 1].reserve((size_t)nf * nf);
+        launch(k_ml_dense_mc<D>, nf, 128, 0, st_, mlc_.g[l + 1], lof, nf, loc, nc, na1, (const int *)mlmap_.p,
+               (const int *)mlabove_.p, (const unsigned char *)mlpar_.p, (const double *)mlC_.p,
+               (const double *)mlM_[cur].p, mlMC_.p);
+        launch(k_ml_dense<D>, nf, 256, 0, st_, mlc_.g[l], mlc_.g[l + 1], lof, nf, loc, na1, (const int *)mlact_.p,
+               (const int *)mlmap_.p, (const int *)mlabove_.p, (const unsigned char *)mlpar_.p,
+               (const double *)mlA_.p, (const double *)mldinv_.p, (const double *)mlC_.p, (const double *)mlMC_.p,
+               mlM_[cur ^ 1].p);
+        cur ^= 1;
+    }
+    mlM_last_ = mlM_[cur].p;
     MPS_CUDA(cudaGetLastError());
 }
 
@@ -1379,38 +1426,38 @@ template <int D>
 void Engine<D>::ml_update(bool restrict_only, double *x, double *r, const double *p, const double *Ap)
 {
     int nact = act_off_[1 << D];
-    launch_pdl(restrict_only ? k_ml_update<D, true> : k_ml_update<D, false>, RED_BLOCKS, CG_BLOCK, 0, st_, nact,
+    launch_pdl(restrict_only ? k_ml_update<D, true> : k_ml_update<D, false>, red_grid(nact, CG_BLOCK / 32), CG_BLOCK,
+               0, st_, nact,
                (const int2 *)adesc_.p, (const float *)mlfrac_.p, cap_, x, r, p, Ap, mlcsum_.p, partials_.p, ticket_.p,
                sc_.p);
 }
 
-// The V-cycle: grids with many nodes a launch per step, the others in the
-// cluster kernel.
+// The V-cycle: one launch down and one up per grid above the dense one.
 template <int D>
 void Engine<D>::ml_cycle()
 {
     MlVecs v = ml_vecs();
-    int nl = ml_.nl;
     const CGScalars *sc = sc_.p;
-    auto blocks = [&](long long threads) { return std::min(nblk(threads, CG_BLOCK), 148 * 16); };
-    for (int l = 0; l < ml_l0_; l++) {
-        int lo = ml_.lo[l], hi = ml_.lo[l + 1], na = hi - lo;
-        bool above_add = ml_add_ && l == 1;
-        if (l == 0) launch_pdl(k_ml_nodes1<D>, blocks(na), CG_BLOCK, 0, st_, v, sc);
+    const int *lo = mlc_.lo;
+    int ld = ml_ld_;
+    launch_pdl(k_ml_nodes1<D>, nblk(v.na1, CG_BLOCK), CG_BLOCK, 0, st_, v, sc);
+    for (int l = 0; l < ld; l++) {
+        int nc = lo[l + 2] - lo[l + 1], nf = lo[l + 1] - lo[l];
+        if (ml_add_ && l == 0)
+            launch_pdl(k_ml_add_down<D>, nblk(nc, CG_BLOCK), CG_BLOCK, 0, st_, v, mlc_.g[0], lo[1], lo[2], sc);
         else
-            launch_pdl(k_ml_restrict<D>, blocks(na), CG_BLOCK, 0, st_, v, (const double *)(above_add ? v.b : v.y),
-                       ml_.g[l - 1], ml_.g[l], lo, hi, sc);
-        if (!(ml_add_ && l == 0))
-            launch_pdl(k_ml_residual<D, false>, blocks(8LL * na), CG_BLOCK, 0, st_, v, ml_.g[l], lo, hi, sc);
+            launch_pdl(k_ml_down<D>, nblk(nc, CG_BLOCK / 32) + nblk(nf, CG_BLOCK / 8), CG_BLOCK, 0, st_, v, mlc_.g[l],
+                       l, lo[l], lo[l + 1], lo[l + 2], sc);
     }
-    const double *src = ml_l0_ == 0 ? nullptr : (ml_add_ && ml_l0_ == 1) ? v.b : v.y;
-    launch_pdl(k_ml_cycle<D>, ML_CL, ML_CL_THREADS, 0, st_, v, ml_, ml_l0_, src, ml_add_, sc);
-    for (int l = ml_l0_ - 1; l >= 0; l--) {
-        int lo = ml_.lo[l], hi = ml_.lo[l + 1], na = hi - lo;
-        const double *cx = l + 1 == nl - 1 ? v.x : v.y;
-        launch_pdl(k_ml_prolong_add<D>, blocks(na), CG_BLOCK, 0, st_, v, cx, ml_.g[l], ml_.g[l + 1], lo, hi, sc);
-        if (!(ml_add_ && l == 0))
-            launch_pdl(k_ml_residual<D, true>, blocks(8LL * na), CG_BLOCK, 0, st_, v, ml_.g[l], lo, hi, sc);
+    int nd = lo[ld + 1] - lo[ld];
+    launch_pdl(k_ml_matvec, nblk(nd, CG_BLOCK / 32), CG_BLOCK, 0, st_, v, lo[ld], nd, sc);
+    for (int l = ld - 1; l >= 0; l--) {
+        const double *cx = l + 1 == ld ? v.x : v.y;
+        int nf = lo[l + 1] - lo[l];
+        if (ml_add_ && l == 0)
+            launch_pdl(k_ml_add_up<D>, nblk(nf, CG_BLOCK), CG_BLOCK, 0, st_, v, mlc_.g[1], cx, sc);
+        else
+            launch_pdl(k_ml_up<D>, nblk(nf, CG_BLOCK / 8), CG_BLOCK, 0, st_, v, mlc_.g[l + 1], lo[l], nf, cx, sc);
     }
 }
 
@@ -1419,7 +1466,8 @@ template <int D>
 void Engine<D>::ml_prolong(bool rz, const double *r, double *z)
 {
     int nact = act_off_[1 << D];
-    launch_pdl(rz ? k_ml_prolong<D, true> : k_ml_prolong<D, false>, RED_BLOCKS, CG_BLOCK, 0, st_, nact,
+    launch_pdl(rz ? k_ml_prolong<D, true> : k_ml_prolong<D, false>, red_grid(nact, CG_BLOCK / 32), CG_BLOCK, 0, st_,
+               nact,
                (const int2 *)adesc_.p, (const int *)mlcnode_.p, ml_.g[0], (const float *)mlfrac_.p, cap_,
                (const double *)jdinv_.p, r, z, ml_result(), partials_.p, ticket_.p, sc_.p);
 }
@@ -1800,7 +1848,7 @@ void Engine<D>::pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc,
                           const double *zprev)
 {
     using T = double;
-    const int RB = RED_BLOCKS;
+    const int RB = red_grid(n_eq, CG_BLOCK);
     int iter_before = 0;
     if (!zprev) {
         CGScalars init{};
@@ -1821,35 +1869,36 @@ void Engine<D>::pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc,
     };
     auto sweep = [&](bool fwdir) { run_sweep<TM>(v, fwdir); };
     const int lpr = spmv_lpr_ ? spmv_lpr_ : (sizeof(TM) == 8 ? 8 : 16);
+    const int SB = red_grid(n_eq, CG_BLOCK / lpr);
     auto spmv = [&]() {
         const int *rp = row_ptr_.p, *ci = col_.p;
         if (v.A64)
-            lk(4, k_cg_spmv<8, double>, RB, CG_BLOCK, 0, n_eq, rp, ci, v.A64, (const T *)v.p, v.Ap, partials_.p,
+            lk(4, k_cg_spmv<8, double>, SB, CG_BLOCK, 0, n_eq, rp, ci, v.A64, (const T *)v.p, v.Ap, partials_.p,
                ticket_.p, sc_.p, (const double *)nullptr, (const uint2 *)nullptr);
         else if (v.dsum && v.ac) {
             if constexpr (sizeof(TM) == 4) {
                 if (lpr == 16)
-                    lk(4, k_cg_spmv<16, TM, true, true>, RB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap,
+                    lk(4, k_cg_spmv<16, TM, true, true>, SB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap,
                        partials_.p, ticket_.p, sc_.p, v.dsum, v.ac);
                 else
-                    lk(4, k_cg_spmv<8, TM, true, true>, RB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap,
+                    lk(4, k_cg_spmv<8, TM, true, true>, SB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap,
                        partials_.p, ticket_.p, sc_.p, v.dsum, v.ac);
             }
         }
         else if (v.dsum && lpr == 16)
-            lk(4, k_cg_spmv<16, TM, true>, RB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap, partials_.p,
+            lk(4, k_cg_spmv<16, TM, true>, SB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap, partials_.p,
                ticket_.p, sc_.p, v.dsum, (const uint2 *)nullptr);
         else if (v.dsum)
-            lk(4, k_cg_spmv<8, TM, true>, RB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap, partials_.p,
+            lk(4, k_cg_spmv<8, TM, true>, SB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap, partials_.p,
                ticket_.p, sc_.p, v.dsum, (const uint2 *)nullptr);
         else if (lpr == 16)
-            lk(4, k_cg_spmv<16, TM>, RB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap, partials_.p,
+            lk(4, k_cg_spmv<16, TM>, SB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap, partials_.p,
                ticket_.p, sc_.p, (const double *)nullptr, (const uint2 *)nullptr);
         else if (lpr == 32)
-            lk(4, k_cg_spmv<32, TM>, RB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap, partials_.p,
+            lk(4, k_cg_spmv<32, TM>, SB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap, partials_.p,
                ticket_.p, sc_.p, (const double *)nullptr, (const uint2 *)nullptr);
         else
-            lk(4, k_cg_spmv<8, TM>, RB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap, partials_.p,
+            lk(4, k_cg_spmv<8, TM>, SB, CG_BLOCK, 0, n_eq, rp, ci, v.A, (const T *)v.p, v.Ap, partials_.p,
                ticket_.p, sc_.p, (const double *)nullptr, (const uint2 *)nullptr);
     };
     const bool ml = icc && ml_on_;

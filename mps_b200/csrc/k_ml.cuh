@@ -14,7 +14,11 @@
 //     z = D^-1 r + P V(P^T r),
 // V a symmetric V-cycle over the grids (one l1-Jacobi step before and after
 // each coarse correction, an explicit inverse on the coarsest grid), or, with
-// `additive`, V(b) = s D_1^-1 b + I V_2(I^T b) (no matrix on the first grid).
+// `additive`, V(b) = s D_1^-1 b + I V_2(I^T b) (no product on the first grid).
+// From the first grid of at most ML_DENSE nodes on, the V-cycle is one dense
+// symmetric matrix, formed once per solve from the coarsest grid up: a chain
+// of dependent steps, each a fraction of a microsecond of work, becomes one
+// product.
 // Both are symmetric and positive definite: D_l1 = diag(sum_j |a_ij|) >= A_l,
 // so an l1-Jacobi step of relaxation below 2 always contracts (Baker, Falgout,
 // Kolev, Yang 2011, "Multigrid smoothers for ultra-parallel computing"), and
@@ -25,12 +29,17 @@
 // their cells, which are held in FP32: they define P, and the same numbers
 // are used in P, P^T and A_1.
 //
-// Measured against the block-colour IC(0) (a step, B200, one box): 3-D dam
-// break of 2.85 M particles, mixed form, 619 -> 34 iterations, 887 -> 103 ms;
-// 1.17 M particles in FP64, 507 -> 44, 387 -> 47 ms; 2,158 particles in 2-D,
-// 94 -> 44, 7.1 -> 2.6 ms.  What remains of an iteration is the product with
-// the matrix (HBM) at large sizes and the chain of dependent launches at
-// small ones.
+// Measured against the block-colour IC(0) (B200, the solve of a step): 3-D dam
+// break of 2.85 M particles, mixed form, 619 -> 30 iterations, 747 -> 23.5 ms;
+// 1.17 M particles in FP64, 507 -> 43, 336 -> 14.3 ms; 117 k particles, 160 ->
+// 40, 36.9 -> 2.7 ms; 2,158 particles in 2-D, 94 -> 37, 6.4 -> 1.0 ms.  What
+// remains of an iteration is the product with the matrix (HBM) at large sizes
+// and the chain of dependent launches at small ones.  With a V-cycle of
+// separate residual, restriction and interpolation steps the same solves took
+// 28.6, 18.8, 5.0 and 1.8 ms; that V-cycle in one cluster of 8 CTAs, with C and
+// C^T but the matrix on every grid, 26.3, 20.2, 5.5 and 1.2 ms (a step of a
+// few index operations and dependent loads takes 2-7 us however few nodes it
+// has), so the small grids became one dense product.
 //
 // No sum uses an atomic; every reduction runs in a fixed order, so results
 // are the same bits on every run.
@@ -42,12 +51,22 @@
 namespace mps {
 
 constexpr int ML_MAXL = 26;       // grids at most: 2^30 cells, even in one direction, reach the coarsest size
-constexpr int ML_COARSEST = 64;   // nodes (boundary box) of the coarsest grid at most
+constexpr int ML_BOX = 64;        // the grids end when their box holds at most this many nodes ...
+// ... and a solve's at the first with at most this many nodes in use: its
+// explicit inverse costs 128 pivots once and ends the chain of dependent
+// steps two or three grids earlier.
+constexpr int ML_COARSEST = 128;
+// Nodes up to which a grid's V-cycle is held as a dense matrix: 8 MB at most,
+// read from L2 in about 3 us, against three dependent launches per grid for
+// the steps it replaces.
+constexpr int ML_DENSE = 1024;
 // Relaxation of the l1-Jacobi steps (below 2 contracts); measured on the dam
 // break at l0 = 0.01: 42 iterations at 1.0, 40 at 1.4 to 1.9.
 constexpr double ML_OMEGA = 1.5;
 // Weight of the additive first grid's D_1^-1 (D_1 the true diagonal).
 constexpr double ML_ADD = 0.45;
+
+constexpr int ML_PAD = 4;   // a C row reaches 3 beyond the node under its own, which may be 1 outside
 
 template <int D>
 struct MlDim {
@@ -57,9 +76,10 @@ struct MlDim {
     static constexpr int ST = D == 3 ? 125 : 25;       // stencil (5 per axis)
     static constexpr int STP = D == 3 ? 128 : 32;      // its stride in memory
     static constexpr int W7 = D == 3 ? 343 : 49;       // nodes within 3 of a node (7 per axis)
+    static constexpr int W7P = D == 3 ? 352 : 64;      // their stride in memory
 };
 
-// One grid.  Vectors live on the whole box of nodes with a margin of two
+// One grid.  Vectors live on the whole box of nodes with a margin of ML_PAD
 // nodes per side that stays zero, so a stencil never leaves its grid; the
 // grids follow one another in one array.  at(x, y, z) = base + x + s1 y + s2 z.
 struct MlGrid {
@@ -81,13 +101,13 @@ __device__ __forceinline__ void ml_coords(const MlGrid &g, int idx, int *c)
 {
     int rel = idx - g.first;
     if (D == 3) {
-        c[2] = rel / g.s2 - 2;
+        c[2] = rel / g.s2 - ML_PAD;
         rel %= g.s2;
     } else {
         c[2] = 0;
     }
-    c[1] = rel / g.s1 - 2;
-    c[0] = rel % g.s1 - 2;
+    c[1] = rel / g.s1 - ML_PAD;
+    c[0] = rel % g.s1 - ML_PAD;
 }
 
 // Offset of stencil entry k (x fastest, -2..2 per axis).
@@ -458,12 +478,16 @@ k_ml_a1(int na, const int *__restrict__ ncell, const double *__restrict__ cellma
 }
 
 // A_{l+1} = I^T A_l I, a block per coarse node: the fine rows under the node
-// combined on the 7^D fine nodes around it, then gathered onto the coarse
-// stencil.
+// combined on the 7^D fine nodes around it, T = I^T A_l, then gathered onto
+// the coarse stencil.  With E = f D_l1^-1 the smoother, a pre-smoothed residual
+// restricts as I^T (b - A E b) = C b, C = I^T - T E, and C^T is the
+// post-smoothed interpolation (1 - E A) I: C is kept so that either direction
+// of the V-cycle is one dependent step per grid.
 template <int D>
 __global__ void __launch_bounds__(MlDim<D>::STP)
 k_ml_galerkin(MlGrid f, MlGrid c, int lof, int loc, const int *__restrict__ act, const int *__restrict__ amap,
-              const double *__restrict__ Af, double *__restrict__ Ac, double *__restrict__ dinv)
+              const double *__restrict__ Af, const double *__restrict__ dinvf, double *__restrict__ Ac,
+              double *__restrict__ dinv, double *__restrict__ C)
 {
     using L = MlDim<D>;
     __shared__ double T[L::W7];
@@ -472,32 +496,46 @@ k_ml_galerkin(MlGrid f, MlGrid c, int lof, int loc, const int *__restrict__ act,
     int t = blockIdx.x, k = threadIdx.x;
     int cc[3];
     ml_coords<D>(c, act[loc + t], cc);
+    int centre = ml_at(f, 2 * cc[0], 2 * cc[1], 2 * cc[2]);
     if (k < L::CELLS) {
-        int x = 2 * cc[0] + k % 3 - 1, y = 2 * cc[1] + (k / 3) % 3 - 1, z = D == 3 ? 2 * cc[2] + k / 9 - 1 : 0;
-        bool in = x >= 0 && x < f.n[0] && y >= 0 && y < f.n[1] && z >= 0 && z < f.n[2];
-        int a = in ? amap[ml_at(f, x, y, z)] : -1;
+        int x = k % 3 - 1, y = (k / 3) % 3 - 1, z = D == 3 ? k / 9 - 1 : 0;
+        int a = amap[centre + x + f.s1 * y + f.s2 * z];   // -1 in the margins
         frow[k] = a < 0 ? -1 : a - lof;
     }
     __syncthreads();
     for (int w = k; w < L::W7; w += L::STP) {
         int p[3] = {w % 7 - 3, (w / 7) % 7 - 3, D == 3 ? w / 49 - 3 : 0};
-        double s = 0.0;
+        double s = 0.0, own = 0.0;
         for (int j = 0; j < L::CELLS; j++) {
             if (frow[j] < 0) continue;
             int i[3] = {j % 3 - 1, (j / 3) % 3 - 1, D == 3 ? j / 9 - 1 : 0};
             int e = 0;
-            bool in = true;
+            bool in = true, same = true;
             double wt = 1.0;
 #pragma unroll
             for (int d = D - 1; d >= 0; d--) {
                 int x = p[d] - i[d] + 2;
                 in = in && x >= 0 && x < 5;
+                same = same && x == 2;
                 e = e * 5 + x;
                 if (i[d]) wt *= 0.5;
             }
+            if (same) own = wt;
             if (in) s = fma(wt, __ldg(&Af[(size_t)frow[j] * L::STP + e]), s);
         }
         T[w] = s;
+        double v = 0.0;
+        bool in = true;
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+            int x = 2 * cc[d] + p[d];
+            in = in && x >= 0 && x < f.n[d];
+        }
+        if (in) {
+            int a = amap[centre + p[0] + f.s1 * p[1] + f.s2 * p[2]];
+            if (a >= 0) v = own - s * __ldg(&dinvf[a - lof]);
+        }
+        C[(size_t)t * L::W7P + w] = v;
     }
     __syncthreads();
     double s = 0.0;
@@ -522,55 +560,189 @@ k_ml_galerkin(MlGrid f, MlGrid c, int lof, int loc, const int *__restrict__ act,
     ml_row_factor<D>(s, k, sh, false, &dinv[t]);
 }
 
-// Inverse of the coarsest operator (n <= ML_COARSEST nodes), one CTA:
-// Gauss-Jordan without pivoting on the symmetric matrix.  A pivot that
-// cancellation has emptied (below 1e-9 of its diagonal: a constant on a region
-// no known pressure bounds, or a node no row reaches) is dropped, which keeps
-// the inverse symmetric and semidefinite.
+// Inverse of the coarsest operator (n <= ML_COARSEST nodes), one CTA, the
+// matrix in registers (16 entries a thread): Gauss-Jordan without pivoting on
+// the symmetric matrix, one barrier per pivot.  A pivot that cancellation has
+// emptied (below 1e-9 of its diagonal: a constant on a region no known
+// pressure bounds, or a node no row reaches) is dropped, which keeps the
+// inverse symmetric and semidefinite.
 template <int D>
 __global__ void __launch_bounds__(1024)
 k_ml_inverse(MlGrid g, int lo, int n, const int *__restrict__ act, const int *__restrict__ amap,
              const double *__restrict__ A, double *__restrict__ inv)
 {
     using L = MlDim<D>;
-    extern __shared__ double a[];   // n x n, then the diagonal
-    double *dg = a + n * n;
-    __shared__ double piv;
-    for (int w = threadIdx.x; w < n * n; w += blockDim.x) a[w] = 0.0;
+    constexpr int N = ML_COARSEST, T = N / 32;
+    extern __shared__ double m[];   // N x N while loading and storing
+    __shared__ double row[2][N], cl[2][N], dg[N], piv[2];
+    int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int w = threadIdx.x; w < N * N; w += blockDim.x) m[w] = 0.0;
     __syncthreads();
     for (int w = threadIdx.x; w < n * L::ST; w += blockDim.x) {
         int i = w / L::ST, k = w % L::ST;
-        int j = amap[act[lo + i] + ml_offset<D>(g, k)];
         double v = A[(size_t)i * L::STP + k];
-        if (j >= lo && j < lo + n && v != 0.0) a[i * n + j - lo] = v;
+        if (v != 0.0) {
+            int j = amap[act[lo + i] + ml_offset<D>(g, k)];
+            if (j >= lo && j < lo + n) m[i * N + j - lo] = v;
+        }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) dg[i] = a[i * n + i];
+    double a[T][T];
+#pragma unroll
+    for (int p = 0; p < T; p++)
+#pragma unroll
+        for (int q = 0; q < T; q++) a[p][q] = m[(ty + 32 * p) * N + tx + 32 * q];
+    if (threadIdx.x < N) dg[threadIdx.x] = m[threadIdx.x * N + threadIdx.x];
+    __syncthreads();
     for (int k = 0; k < n; k++) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double d = a[k * n + k];
-            piv = d > 1.0e-9 * dg[k] ? 1.0 / d : 0.0;
+        double *rk = row[k & 1], *ck = cl[k & 1];
+        int kp = k >> 5, kt = k & 31;
+        if (ty == kt) {
+#pragma unroll
+            for (int p = 0; p < T; p++)
+                if (p == kp) {
+#pragma unroll
+                    for (int q = 0; q < T; q++) rk[tx + 32 * q] = a[p][q];
+                }
+        }
+        if (tx == kt) {
+#pragma unroll
+            for (int q = 0; q < T; q++)
+                if (q == kp) {
+#pragma unroll
+                    for (int p = 0; p < T; p++) ck[ty + 32 * p] = a[p][q];
+                    if (ty == kt) {
+                        double d = 0.0;
+#pragma unroll
+                        for (int p = 0; p < T; p++)
+                            if (p == kp) d = a[p][q];
+                        piv[k & 1] = d > 1.0e-9 * dg[k] ? 1.0 / d : 0.0;
+                    }
+                }
         }
         __syncthreads();
-        double p = piv;
-        // off the pivot's row and column
-        for (int w = threadIdx.x; w < n * n; w += blockDim.x) {
-            int i = w / n, j = w % n;
-            if (i != k && j != k && p != 0.0) a[w] -= a[i * n + k] * p * a[k * n + j];
+        double pv = piv[k & 1];
+        double r[T];
+#pragma unroll
+        for (int q = 0; q < T; q++) r[q] = rk[tx + 32 * q];
+#pragma unroll
+        for (int p = 0; p < T; p++) {
+            double f = ck[ty + 32 * p] * pv;
+            bool prow = p == kp && ty == kt;
+#pragma unroll
+            for (int q = 0; q < T; q++) {
+                bool pcol = q == kp && tx == kt;
+                double v = fma(-f, r[q], a[p][q]);
+                v = prow ? pv * r[q] : v;
+                v = pcol ? (prow ? pv : -f) : v;
+                a[p][q] = v;
+            }
         }
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            if (i == k) continue;
-            a[i * n + k] *= -p;
-            a[k * n + i] *= p;
-        }
-        if (threadIdx.x == 0) a[k * n + k] = p;
     }
+#pragma unroll
+    for (int p = 0; p < T; p++)
+#pragma unroll
+        for (int q = 0; q < T; q++) m[(ty + 32 * p) * N + tx + 32 * q] = a[p][q];
     __syncthreads();
     for (int w = threadIdx.x; w < n * n; w += blockDim.x) {
         int i = w / n, j = w % n;
-        inv[w] = 0.5 * (a[i * n + j] + a[j * n + i]);
+        inv[w] = 0.5 * (m[i * N + j] + m[j * N + i]);
+    }
+}
+
+// Per node: the index of the fine node under it (grids beyond the first), and
+// of the lowest coarse node whose C row reaches it (all but the last), with
+// the parities of its coordinates.
+template <int D>
+__global__ void k_ml_tables(const __grid_constant__ MlLevels lv, const int *__restrict__ act, int *__restrict__ under,
+                            int *__restrict__ above, unsigned char *__restrict__ parity)
+{
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= lv.lo[lv.nl]) return;
+    int l = 0;
+    while (t >= lv.lo[l + 1]) l++;
+    int c[3];
+    ml_coords<D>(lv.g[l], act[t], c);
+    if (l > 0) under[t] = ml_at(lv.g[l - 1], 2 * c[0], 2 * c[1], 2 * c[2]);
+    if (l + 1 < lv.nl) {
+        above[t] = ml_at(lv.g[l + 1], (c[0] >> 1) - 1, (c[1] >> 1) - 1, D == 3 ? (c[2] >> 1) - 1 : 0);
+        parity[t] = (unsigned char)((c[0] & 1) | (c[1] & 1) << 1 | (D == 3 ? (c[2] & 1) << 2 : 0));
+    }
+}
+
+// Candidate e (of 4^D) of a node's column of C: offset from above[node] and
+// the entry within that coarse node's row, -1 if out of its reach.
+template <int D>
+__device__ __forceinline__ int ml_cand(const MlGrid &c, int par, int e, int &off)
+{
+    int e0 = e & 3, e1 = (e >> 2) & 3, e2 = D == 3 ? e >> 4 : 0;
+    off = e0 + c.s1 * e1 + c.s2 * e2 * (D == 3);
+    int x = 5 + (par & 1) - 2 * e0, y = 5 + ((par >> 1) & 1) - 2 * e1, z = D == 3 ? 5 + (par >> 2) - 2 * e2 : 0;
+    if (x < 0 || y < 0 || z < 0) return -1;
+    return x + 7 * y + (D == 3 ? 49 * z : 0);
+}
+
+// Dense V-cycle of grid l from that of grid l + 1 (M_c, symmetric):
+// M = 2 E - E A E + C^T M_c C.  First MC = M_c C, a block per fine node.
+template <int D>
+__global__ void __launch_bounds__(128)
+k_ml_dense_mc(MlGrid c, int lo, int nf, int loc, int nc, int na1, const int *__restrict__ amap,
+              const int *__restrict__ above, const unsigned char *__restrict__ parity, const double *__restrict__ C,
+              const double *__restrict__ Mc, double *__restrict__ MC)
+{
+    constexpr int NE = D == 3 ? 64 : 16;
+    __shared__ int row[NE];
+    __shared__ double val[NE];
+    int i = blockIdx.x, t = threadIdx.x;
+    if (t < NE) {
+        int off, w = ml_cand<D>(c, parity[lo + i], t, off);
+        int a = w >= 0 ? amap[above[lo + i] + off] : -1;
+        row[t] = a >= 0 ? a - loc : 0;
+        val[t] = a >= 0 ? C[(size_t)(a - na1) * MlDim<D>::W7P + w] : 0.0;
+    }
+    __syncthreads();
+    for (int j = t; j < nc; j += 128) {
+        double s = 0.0;
+        for (int e = 0; e < NE; e++)
+            if (val[e] != 0.0) s = fma(val[e], __ldg(&Mc[(size_t)row[e] * nc + j]), s);
+        MC[(size_t)j * nf + i] = s;
+    }
+}
+
+template <int D>
+__global__ void __launch_bounds__(256)
+k_ml_dense(MlGrid f, MlGrid c, int lo, int nf, int loc, int na1, const int *__restrict__ act,
+           const int *__restrict__ amap, const int *__restrict__ above, const unsigned char *__restrict__ parity,
+           const double *__restrict__ A, const double *__restrict__ dinv, const double *__restrict__ C,
+           const double *__restrict__ MC, double *__restrict__ M)
+{
+    using L = MlDim<D>;
+    constexpr int NE = D == 3 ? 64 : 16;
+    __shared__ int row[NE];
+    __shared__ double val[NE];
+    int i = blockIdx.x, t = threadIdx.x;
+    if (t < NE) {
+        int off, w = ml_cand<D>(c, parity[lo + i], t, off);
+        int a = w >= 0 ? amap[above[lo + i] + off] : -1;
+        row[t] = a >= 0 ? a - loc : 0;
+        val[t] = a >= 0 ? C[(size_t)(a - na1) * L::W7P + w] : 0.0;
+    }
+    __syncthreads();
+    for (int j = t; j < nf; j += 256) {
+        double s = 0.0;
+        for (int e = 0; e < NE; e++)
+            if (val[e] != 0.0) s = fma(val[e], __ldg(&MC[(size_t)row[e] * nf + j]), s);
+        M[(size_t)i * nf + j] = s;
+    }
+    __syncthreads();
+    if (t < L::ST) {
+        int a = amap[act[lo + i] + ml_offset<D>(f, t)];
+        if (a >= 0) {
+            double ei = dinv[lo + i];
+            double s = -ei * A[(size_t)(lo + i) * L::STP + t] * dinv[a];
+            if (t == L::ST / 2) s += 2.0 * ei;
+            M[(size_t)i * nf + a - lo] += s;
+        }
     }
 }
 
@@ -700,201 +872,237 @@ k_ml_prolong(int nact, const int2 *__restrict__ desc, const int *__restrict__ cn
 // ---- grid operations; each on nodes t0, t0 + step, ... of one grid ----
 
 struct MlVecs {
-    double *b, *x, *y;       // right-hand side, iterate, residual (or the iterate's other buffer)
-    const int *act;
+    double *b, *x, *y;       // right-hand side, E b (or the dense grid's solution), result
+    double *bd;              // right-hand side of the dense grid, by node
+    const int *act, *amap, *under, *above;
+    const unsigned char *parity;
     const double *A, *dinv;  // operators and smoother factors by node number
+    const double *C;         // by node number beyond the first grid
     const int *ncell;
-    const double *csum, *inv;
+    const double *csum, *M;  // cells' parts of P^T r; the dense V-cycle
     int na1;                 // nodes of the first grid
+    int ld;                  // the dense grid
 };
 
-// b_1 = P^T r from the cells' parts, x_1 = f b_1.
-template <int D>
-__device__ __forceinline__ void ml_nodes1(const MlVecs &v, int t0, int step)
-{
-    for (int t = t0; t < v.na1; t += step) {
-        double s = 0.0;
-#pragma unroll
-        for (int k = 0; k < (1 << D); k++) {
-            int c = __ldg(&v.ncell[(size_t)k * v.na1 + t]);
-            if (c >= 0) s += __ldcg(&v.csum[(size_t)c * (1 << D) + k]);
-        }
-        int o = __ldg(&v.act[t]);
-        v.b[o] = s;
-        v.x[o] = __ldg(&v.dinv[t]) * s;
-    }
-}
-
-// POST: y = x + f (b - A x), else y = b - A x; eight lanes per node.
-template <int D, bool POST>
-__device__ __forceinline__ void ml_residual(const MlVecs &v, const MlGrid &g, int lo, int hi, int t0, int step)
-{
-    using L = MlDim<D>;
-    int lane = threadIdx.x & 7;
-    int nrow = (hi - lo + 3) & ~3;   // whole warps
-    for (int t = t0 >> 3; t < nrow; t += step >> 3) {
-        bool in = lo + t < hi;
-        int o = in ? __ldg(&v.act[lo + t]) : g.base;
-        const double *a = v.A + (size_t)(in ? lo + t : lo) * L::STP;
-        double s = 0.0;
-        if (in) {
-#pragma unroll
-            for (int j = 0; j < L::STP / 8; j++) {
-                int k = lane + 8 * j;
-                if (k < L::ST) s = fma(__ldg(&a[k]), __ldcg(&v.x[o + ml_offset<D>(g, k)]), s);
-            }
-        }
-        s += __shfl_xor_sync(0xffffffffu, s, 4);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        if (in && lane == 0) {
-            double res = __ldcg(&v.b[o]) - s;
-            v.y[o] = POST ? __ldcg(&v.x[o]) + __ldg(&v.dinv[lo + t]) * res : res;
-        }
-    }
-}
-
-// b_c = I^T src on the coarser grid c, x_c = f b_c.
-template <int D>
-__device__ __forceinline__ void ml_restrict(const MlVecs &v, const double *src, const MlGrid &f, const MlGrid &c,
-                                            int lo, int hi, int t0, int step)
-{
-    for (int t = lo + t0; t < hi; t += step) {
-        int o = __ldg(&v.act[t]);
-        int cc[3];
-        ml_coords<D>(c, o, cc);
-        int fo = ml_at(f, 2 * cc[0], 2 * cc[1], 2 * cc[2]);
-        double s = 0.0;
-#pragma unroll
-        for (int j = 0; j < MlDim<D>::CELLS; j++) {
-            int dx = j % 3 - 1, dy = (j / 3) % 3 - 1, dz = D == 3 ? j / 9 - 1 : 0;
-            double w = (dx ? 0.5 : 1.0) * (dy ? 0.5 : 1.0) * (dz ? 0.5 : 1.0);
-            s = fma(w, __ldcg(&src[fo + dx + f.s1 * dy + f.s2 * dz]), s);
-        }
-        v.b[o] = s;
-        v.x[o] = __ldg(&v.dinv[t]) * s;
-    }
-}
-
-// x_f += I src, src on the coarser grid c.
-template <int D>
-__device__ __forceinline__ void ml_prolong(const MlVecs &v, const double *src, const MlGrid &f, const MlGrid &c,
-                                           int lo, int hi, int t0, int step)
-{
-    for (int t = lo + t0; t < hi; t += step) {
-        int o = __ldg(&v.act[t]);
-        int fc[3];
-        ml_coords<D>(f, o, fc);
-        double s = 0.0;
-#pragma unroll
-        for (int j = 0; j < (1 << D); j++) {
-            int q = ml_at(c, (fc[0] + (j & 1)) / 2, (fc[1] + ((j >> 1) & 1)) / 2, D == 3 ? (fc[2] + (j >> 2)) / 2 : 0);
-            s += __ldcg(&src[q]);
-        }
-        v.x[o] = __ldcg(&v.x[o]) + s * (1.0 / (1 << D));
-    }
-}
-
+// b_1 = P^T r from the cells' parts, x_1 = E b_1.
 template <int D>
 __global__ void __launch_bounds__(CG_BLOCK) k_ml_nodes1(MlVecs v, const CGScalars *sc)
 {
     pdl_trigger();
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    bool in = t < v.na1;
+    int c[1 << D];
+#pragma unroll
+    for (int k = 0; k < (1 << D); k++) c[k] = in ? __ldg(&v.ncell[(size_t)k * v.na1 + t]) : -1;
+    int o = in ? __ldg(&v.act[t]) : 0;
+    double di = in ? __ldg(&v.dinv[t]) : 0.0;
     pdl_wait();
-    if (sc->done) return;
-    ml_nodes1<D>(v, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    if (!in || sc->done) return;
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < (1 << D); k++)
+        if (c[k] >= 0) s += v.csum[(size_t)c[k] * (1 << D) + k];
+    if (v.ld == 0) {
+        v.bd[t] = s;
+    } else {
+        v.b[o] = s;
+        v.x[o] = di * s;
+    }
 }
 
-template <int D, bool POST>
-__global__ void __launch_bounds__(CG_BLOCK) k_ml_residual(MlVecs v, MlGrid g, int lo, int hi, const CGScalars *sc)
-{
-    pdl_trigger();
-    pdl_wait();
-    if (sc->done) return;
-    ml_residual<D, POST>(v, g, lo, hi, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-}
-
+// Down one grid: b_{l+1} = C b_l, x_{l+1} = E b_{l+1} (a warp per coarse node,
+// the first blocks) and y_l = 2 x_l - E A x_l (eight lanes per node),
+// independent of each other.  Operators are read before the wait.
 template <int D>
 __global__ void __launch_bounds__(CG_BLOCK)
-k_ml_restrict(MlVecs v, const double *src, MlGrid f, MlGrid c, int lo, int hi, const CGScalars *sc)
+k_ml_down(MlVecs v, MlGrid f, int l, int lo, int mid, int hi, const CGScalars *sc)
 {
+    using L = MlDim<D>;
+    constexpr int NW = CG_BLOCK / 32;
+    __shared__ int off5[L::ST], off7[L::W7];
     pdl_trigger();
+    int lane = threadIdx.x & 31;
+    int nc = hi - mid, nf = mid - lo;
+    int cb = (nc + NW - 1) / NW;   // blocks of the coarse part
+    if ((int)blockIdx.x < cb) {
+        for (int e = threadIdx.x; e < L::W7; e += CG_BLOCK)
+            off7[e] = e % 7 - 3 + f.s1 * ((e / 7) % 7 - 3) + (D == 3 ? f.s2 * (e / 49 - 3) : 0);
+        int w = blockIdx.x * NW + (threadIdx.x >> 5);
+        bool in = w < nc;
+        constexpr int NE = (L::W7 + 31) / 32;
+        double ca[NE];
+        const double *C = v.C + (size_t)(mid + (in ? w : 0) - v.na1) * L::W7P;
+#pragma unroll
+        for (int j = 0; j < NE; j++) {
+            int e = lane + 32 * j;
+            ca[j] = in && e < L::W7 ? __ldg(&C[e]) : 0.0;
+        }
+        int o = in ? __ldg(&v.act[mid + w]) : 0, fo = in ? __ldg(&v.under[mid + w]) : f.base;
+        double di = in ? __ldg(&v.dinv[mid + w]) : 0.0;
+        __syncthreads();
+        pdl_wait();
+        if (sc->done) return;
+        double s = 0.0;
+#pragma unroll
+        for (int j = 0; j < NE; j++) {
+            int e = lane + 32 * j;
+            s = fma(ca[j], v.b[fo + off7[e < L::W7 ? e : 0]], s);
+        }
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+        if (in && lane == 0) {
+            if (v.ld == l + 1) {
+                v.bd[w] = s;
+            } else {
+                v.b[o] = s;
+                v.x[o] = di * s;
+            }
+        }
+        return;
+    }
+    for (int e = threadIdx.x; e < L::ST; e += CG_BLOCK) off5[e] = ml_offset<D>(f, e);
+    int t = (blockIdx.x - cb) * (CG_BLOCK / 8) + (threadIdx.x >> 3), k0 = threadIdx.x & 7;
+    bool in = t < nf;
+    constexpr int NE = L::STP / 8;
+    double a[NE];
+    const double *A = v.A + (size_t)(lo + (in ? t : 0)) * L::STP;
+#pragma unroll
+    for (int j = 0; j < NE; j++) a[j] = in ? __ldg(&A[k0 + 8 * j]) : 0.0;   // zero beyond the stencil
+    int o = in ? __ldg(&v.act[lo + t]) : f.base;
+    double di = in ? __ldg(&v.dinv[lo + t]) : 0.0;
+    __syncthreads();
     pdl_wait();
     if (sc->done) return;
-    ml_restrict<D>(v, src, f, c, lo, hi, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < NE; j++) {
+        int k = k0 + 8 * j;
+        s = fma(a[j], v.x[o + off5[k < L::ST ? k : 0]], s);
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    if (in && k0 == 0) v.y[o] = 2.0 * v.x[o] - di * s;
 }
 
+// Up one grid: y_l += C^T cx, eight lanes per node; cx is the coarser grid's
+// result.
 template <int D>
 __global__ void __launch_bounds__(CG_BLOCK)
-k_ml_prolong_add(MlVecs v, const double *src, MlGrid f, MlGrid c, int lo, int hi, const CGScalars *sc)
+k_ml_up(MlVecs v, MlGrid c, int lo, int nf, const double *cx, const CGScalars *sc)
 {
+    using L = MlDim<D>;
     pdl_trigger();
+    int t = blockIdx.x * (CG_BLOCK / 8) + (threadIdx.x >> 3), lane = threadIdx.x & 7;
+    bool in = t < nf;
+    int o = in ? __ldg(&v.act[lo + t]) : 0, q0 = in ? __ldg(&v.above[lo + t]) : c.base;
+    int par = in ? __ldg(&v.parity[lo + t]) : 0;
+    constexpr int NE = D == 3 ? 8 : 2;
+    double ca[NE];
+    int q[NE];
+#pragma unroll
+    for (int j = 0; j < NE; j++) {
+        int off, w = ml_cand<D>(c, par, lane + 8 * j, off);
+        q[j] = q0 + off;
+        int a = in && w >= 0 ? __ldg(&v.amap[q[j]]) : -1;
+        if (a < 0) q[j] = c.base;
+        ca[j] = a >= 0 ? __ldg(&v.C[(size_t)(a - v.na1) * L::W7P + w]) : 0.0;
+    }
     pdl_wait();
     if (sc->done) return;
-    ml_prolong<D>(v, src, f, c, lo, hi, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < NE; j++) s = fma(ca[j], cx[q[j]], s);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    if (in && lane == 0) v.y[o] += s;
 }
 
-// The V-cycle from grid l0 down and back, in one cluster of ML_CL CTAs: the
-// grids there are small, so what bounds a step is the time between dependent
-// steps, and a cluster barrier costs a fraction of a kernel boundary.
-// first_src: l0 == 0, the cells' parts; else the vector restricted to grid l0.
-// The result is in y on grids with a smoothing step after the correction, in
-// x on the coarsest and on an additive first grid.
-constexpr int ML_CL = 8;
-constexpr int ML_CL_THREADS = 512;
-
-__device__ __forceinline__ void cluster_sync()
+// The additive first grid: b_2 = I^T b_1, x_2 = E b_2, and y_1 = x_1 + I cx.
+template <int D>
+__global__ void __launch_bounds__(CG_BLOCK)
+k_ml_add_down(MlVecs v, MlGrid f, int mid, int hi, const CGScalars *sc)
 {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    pdl_trigger();
+    int t = mid + blockIdx.x * blockDim.x + threadIdx.x;
+    bool in = t < hi;
+    int o = in ? __ldg(&v.act[t]) : 0, fo = in ? __ldg(&v.under[t]) : 0;
+    double di = in ? __ldg(&v.dinv[t]) : 0.0;
+    pdl_wait();
+    if (!in || sc->done) return;
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < MlDim<D>::CELLS; j++) {
+        int dx = j % 3 - 1, dy = (j / 3) % 3 - 1, dz = D == 3 ? j / 9 - 1 : 0;
+        double w = (dx ? 0.5 : 1.0) * (dy ? 0.5 : 1.0) * (dz ? 0.5 : 1.0);
+        s = fma(w, v.b[fo + dx + f.s1 * dy + f.s2 * dz], s);
+    }
+    if (v.ld == 1) {
+        v.bd[t - mid] = s;
+    } else {
+        v.b[o] = s;
+        v.x[o] = di * s;
+    }
 }
 
 template <int D>
-__global__ void __cluster_dims__(ML_CL, 1, 1) __launch_bounds__(ML_CL_THREADS)
-k_ml_cycle(MlVecs v, const __grid_constant__ MlLevels lv, int l0, const double *src, bool additive,
-           const CGScalars *sc)
+__global__ void __launch_bounds__(CG_BLOCK) k_ml_add_up(MlVecs v, MlGrid c, const double *cx, const CGScalars *sc)
 {
     pdl_trigger();
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    bool in = t < v.na1;
+    int o = in ? __ldg(&v.act[t]) : 0, q0 = in ? __ldg(&v.above[t]) : 0, par = in ? __ldg(&v.parity[t]) : 0;
     pdl_wait();
-    if (sc->done) return;   // uniform over the cluster
-    int t0 = blockIdx.x * ML_CL_THREADS + threadIdx.x;
-    constexpr int step = ML_CL * ML_CL_THREADS;
-    int nl = lv.nl;
-    if (l0 == 0) ml_nodes1<D>(v, t0, step);
-    else ml_restrict<D>(v, src, lv.g[l0 - 1], lv.g[l0], lv.lo[l0], lv.lo[l0 + 1], t0, step);
-    cluster_sync();
-    for (int l = l0; l + 1 < nl; l++) {
-        bool add = additive && l == 0;
-        if (!add) {
-            ml_residual<D, false>(v, lv.g[l], lv.lo[l], lv.lo[l + 1], t0, step);
-            cluster_sync();
+    if (!in || sc->done) return;
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < (1 << D); j++) {
+        // parents: node (i + bit) / 2, above[] being at i / 2 - 1
+        int px = 1 + ((par & 1) & (j & 1)), py = 1 + (((par >> 1) & 1) & ((j >> 1) & 1));
+        int pz = D == 3 ? 1 + ((par >> 2) & (j >> 2)) : 0;
+        s += cx[q0 + px + c.s1 * py + c.s2 * pz];
+    }
+    v.y[o] = v.x[o] + s * (1.0 / (1 << D));
+}
+
+// The dense grid: x = M b, a warp per node; the matrix row is read before the
+// wait.
+__global__ void __launch_bounds__(CG_BLOCK) k_ml_matvec(MlVecs v, int lo, int n, const CGScalars *sc)
+{
+    pdl_trigger();
+    int lane = threadIdx.x & 31;
+    int t = blockIdx.x * (CG_BLOCK / 32) + (threadIdx.x >> 5);
+    bool in = t < n;
+    const double *M = v.M + (size_t)(in ? t : 0) * n;
+    constexpr int U = 8;
+    double m[U];
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+        int e = lane + 32 * j;
+        m[j] = in && e < n ? __ldg(&M[e]) : 0.0;
+    }
+    int o = in ? __ldg(&v.act[lo + t]) : 0;
+    pdl_wait();
+    if (!in || sc->done) return;   // warp-uniform
+    double s = 0.0;
+    for (int e0 = 0; e0 < n; e0 += 32 * U) {
+        if (e0) {
+#pragma unroll
+            for (int j = 0; j < U; j++) {
+                int e = e0 + lane + 32 * j;
+                m[j] = e < n ? __ldg(&M[e]) : 0.0;
+            }
         }
-        ml_restrict<D>(v, add ? v.b : v.y, lv.g[l], lv.g[l + 1], lv.lo[l + 1], lv.lo[l + 2], t0, step);
-        cluster_sync();
-    }
-    {
-        // coarsest grid: x = inverse b, eight lanes per node
-        int lo = lv.lo[nl - 1], n = lv.lo[nl] - lo;
-        int lane = threadIdx.x & 7;
-        int nrow = (n + 3) & ~3;
-        for (int t = t0 >> 3; t < nrow; t += step >> 3) {
-            double s = 0.0;
-            if (t < n)
-                for (int j = lane; j < n; j += 8)
-                    s = fma(__ldg(&v.inv[t * n + j]), __ldcg(&v.b[__ldg(&v.act[lo + j])]), s);
-            s += __shfl_xor_sync(0xffffffffu, s, 4);
-            s += __shfl_xor_sync(0xffffffffu, s, 2);
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            if (t < n && lane == 0) v.x[__ldg(&v.act[lo + t])] = s;
+#pragma unroll
+        for (int j = 0; j < U; j++) {
+            int e = e0 + lane + 32 * j;
+            s = fma(m[j], e < n ? v.bd[e] : 0.0, s);
         }
-        cluster_sync();
     }
-    for (int l = nl - 2; l >= l0; l--) {
-        const double *cx = l + 1 == nl - 1 ? v.x : v.y;
-        ml_prolong<D>(v, cx, lv.g[l], lv.g[l + 1], lv.lo[l], lv.lo[l + 1], t0, step);
-        if (additive && l == 0) continue;
-        cluster_sync();
-        ml_residual<D, true>(v, lv.g[l], lv.lo[l], lv.lo[l + 1], t0, step);
-        cluster_sync();
-    }
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+    if (lane == 0) v.x[o] = s;
 }
 
 }  // namespace mps

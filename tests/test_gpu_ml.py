@@ -3,9 +3,9 @@
 Both solve the same system, the IC(0) form (MPS_SWEEP=0) being pinned to the
 oracle elsewhere; the pressures agree to the solver's rounding.  Cases: both
 dimensions and precision forms, the additive and the multiplicative first
-grid (MPS_ML_ADD), every grid but the coarsest as kernels of its own and all of
-them in the cluster kernel (MPS_ML_CLUSTER), grids of odd and even extents, and
-cells with up to ~90 unknowns.  Tolerances: pressure 1e-8, velocity 1e-10 and
+grid (MPS_ML_ADD), the V-cycle dense from the coarsest grid on and from the
+first grid of at most 1,024 nodes on (MPS_ML_DENSE), grids of odd and even
+extents, and cells with up to ~90 unknowns.  Tolerances: pressure 1e-8, velocity 1e-10 and
 position 1e-14 relative L2 after one step, as for a step against the oracle.
 
 A wall region that no known pressure bounds and no source reaches keeps the
@@ -34,7 +34,7 @@ def _rel(a, b):
 
 def _step(monkeypatch, wl, precision, steps=1, **env):
     from mps_b200.session import start
-    for k in ("MPS_SWEEP", "MPS_ML_ADD", "MPS_ML_CLUSTER"):
+    for k in ("MPS_SWEEP", "MPS_ML_ADD", "MPS_ML_DENSE"):
         monkeypatch.delenv(k, raising=False)
     for k, v in env.items():
         monkeypatch.setenv(k, v)
@@ -73,8 +73,8 @@ def test_multilevel_matches_ic0(name, precision, monkeypatch):
     wl = CASES[name]()
     ref, mref = _step(monkeypatch, wl, precision, MPS_SWEEP="0")
     for add in ("0", "1000000"):
-        for cluster in ("0", "4096"):
-            g, m = _step(monkeypatch, wl, precision, MPS_ML_ADD=add, MPS_ML_CLUSTER=cluster)
+        for dense in ("0", "150", "1024"):
+            g, m = _step(monkeypatch, wl, precision, MPS_ML_ADD=add, MPS_ML_DENSE=dense)
             assert m["converged"] == 1
             for f in ("n", "on_surface", "type"):
                 assert np.array_equal(g[f], ref[f]), f
