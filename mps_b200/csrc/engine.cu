@@ -365,6 +365,19 @@ private:
     int win_ = CELL_WIN;
     bool win_valid_ = false;               // the window tables match the current factor and win_
     std::vector<int> inv_col_off_;         // block-inverse offsets at the colour boundaries
+    // CG buffers: the matrix and the factor stored as TM (double in the FP64
+    // form, float in the mixed form), the vectors always FP64
+    template <class TM>
+    struct PcgBufs {
+        const TM *A, *xf_lo, *xf_up, *pkv_lo, *pkv_up, *dinv, *inv_cm, *inv_rm;
+        double *x, *r, *z, *p, *Ap, *y, *part;
+        const double *b;
+        const double *A64 = nullptr;   // if set, the SpMV reads this FP64 matrix instead of A
+        const double *dsum = nullptr;  // if set, the SpMV is in difference form with these row sums
+        // FP32 only: packed (value bits, column) words of the matrix and of
+        // the cross runs; if set, the SpMV and the colour sweeps read these
+        const uint2 *ac = nullptr, *xfc_lo = nullptr, *xfc_up = nullptr;
+    };
     // ---- multilevel preconditioner
     MlLevels ml_{};                        // grids of the cell grid; lo of the current structure
     MlLevels mlc_{};                       // those the current solve uses
@@ -377,6 +390,22 @@ private:
     // iterations, which pays where an iteration is a chain of short launches;
     // and nodes up to which a grid's V-cycle is dense (MPS_ML_DENSE)
     int ml_add_rows_ = 60000, ml_dense_ = ML_DENSE;
+    // unknowns up to which the loop runs in one cluster (MPS_ML_SMALL); measured
+    // per iteration, launches against cluster: 1,617 unknowns (2-D) 27 / 11 us,
+    // 2,842 (3-D) 29 / 21, 5,487 (2-D) 31 / 19, 13,334 (3-D) 35 / 37
+    int ml_small_rows_ = 8192;
+    bool ml_small_ = false;                // the current solve does
+    int ml_clusters_ = -1;                 // clusters of that size the device can hold (-1: not asked yet)
+    int ml_clusters();
+    // entries of the vectors the cluster loop keeps in shared memory
+    size_t ml_small_vectors() const
+    {
+        return (size_t)n_eq_ + mlc_.lo[1] + (ml_add_ ? mlc_.lo[2] - mlc_.lo[1] : 0);
+    }
+    template <class TM>
+    bool ml_small_solve(const PcgBufs<TM> &v, double tol, int maxit, const double *zprev);
+    DevArray<int> mlcellnode_, mlfine_, mlparent_;
+    DevArray<double> mlxd_;
     DevArray<int> mlflag_, mlpos_, mlmap_, mlact_, mlcell_, mlncell_, mlcnode_, mlunder_, mlabove_, ufpar_, ufkeep_, mlscan_;
     DevArray<unsigned char> bounded_, mlpar_;
     DevArray<float> mlfrac_;
@@ -452,19 +481,6 @@ private:
     void sort();
     void unsort();
     void ppe(bool clamp);
-    // CG buffers: the matrix and the factor stored as TM (double in the FP64
-    // form, float in the mixed form), the vectors always FP64
-    template <class TM>
-    struct PcgBufs {
-        const TM *A, *xf_lo, *xf_up, *pkv_lo, *pkv_up, *dinv, *inv_cm, *inv_rm;
-        double *x, *r, *z, *p, *Ap, *y, *part;
-        const double *b;
-        const double *A64 = nullptr;   // if set, the SpMV reads this FP64 matrix instead of A
-        const double *dsum = nullptr;  // if set, the SpMV is in difference form with these row sums
-        // FP32 only: packed (value bits, column) words of the matrix and of
-        // the cross runs; if set, the SpMV and the colour sweeps read these
-        const uint2 *ac = nullptr, *xfc_lo = nullptr, *xfc_up = nullptr;
-    };
     template <class TM>
     void pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc, int n_eq, long long nnz,
                    const double *zprev = nullptr);
@@ -533,6 +549,7 @@ Engine<D>::Engine(const mps_params_t &p, int capacity)
         sweep_mode_ = (v == 0 || v == 1 || v == 3) ? v : 2;
     }
     if (const char *e = std::getenv("MPS_ML_ADD")) ml_add_rows_ = std::max(0, std::atoi(e));
+    if (const char *e = std::getenv("MPS_ML_SMALL")) ml_small_rows_ = std::max(0, std::atoi(e));
     if (const char *e = std::getenv("MPS_ML_DENSE")) ml_dense_ = std::min(ML_DENSE, std::max(0, std::atoi(e)));
     if (const char *e = std::getenv("MPS_SWEEP_HB")) head_batch_ = std::atoi(e) == 8 ? 8 : 4;
     if (const char *e = std::getenv("MPS_SWEEP_OCC")) sweep_occ_ = std::atoi(e) == 8 ? 8 : 6;
@@ -1364,7 +1381,7 @@ void Engine<D>::ml_build(int n_eq)
     mlA_.reserve((size_t)nall * L::STP);
     mlC_.reserve((size_t)(nall - na1) * L::W7P + 1);
     mldinv_.reserve((size_t)nall);
-    mlcsum_.reserve((size_t)nact * L::NC);
+    mlcsum_.reserve((size_t)nact * L::NC * 2);
     mlbd_.reserve((size_t)std::max(ML_DENSE, ML_COARSEST));
     mlunder_.reserve((size_t)nall);
     mlabove_.reserve((size_t)nall);
@@ -1417,7 +1434,119 @@ void Engine<D>::ml_build(int n_eq)
         cur ^= 1;
     }
     mlM_last_ = mlM_[cur].p;
+    ml_small_ = n_eq <= ml_small_rows_ && (ml_ld_ == 0 || (ml_ld_ == 1 && ml_add_)) &&
+                sizeof(double) * ml_small_vectors() <= ML_CL_SMEM && ml_clusters() > 0;
+    if (ml_small_) {
+        int nd = mlc_.lo[ml_ld_ + 1] - mlc_.lo[ml_ld_];
+        mlcellnode_.reserve((size_t)nact * L::NC);
+        mlfine_.reserve((size_t)nd * L::CELLS);
+        mlparent_.reserve((size_t)na1 * L::NC);
+        mlxd_.reserve((size_t)ML_DENSE);
+        launch(k_ml_small_tables<D>, nblk(std::max(nact, std::max(na1, nd)), TPB), TPB, 0, st_, nact, na1, nd, ml_add_,
+               mlc_.g[0], mlc_.g[ml_ld_], (const int *)mlcnode_.p, (const int *)mlmap_.p, (const int *)mlunder_.p,
+               (const int *)mlabove_.p, (const unsigned char *)mlpar_.p, mlcellnode_.p, mlfine_.p, mlparent_.p);
+    }
     MPS_CUDA(cudaGetLastError());
+}
+
+// The attributes of a launch of the cluster loop, one cluster.
+static void ml_cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, size_t smem, cudaStream_t st)
+{
+    cfg = {};
+    cfg.gridDim = dim3(ML_CL);
+    cfg.blockDim = dim3(ML_CL_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ML_CL;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+}
+
+// Whether the device can place a cluster of the loop's size (asked once per
+// session; it is beyond the portable eight CTAs).
+template <int D>
+int Engine<D>::ml_clusters()
+{
+    if (ml_clusters_ >= 0) return ml_clusters_;
+    ml_clusters_ = 1;
+    auto ask = [&](auto kern) {
+        int nc = 0;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[1];
+        ml_cluster_config(cfg, attr, ML_CL_SMEM, st_);
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ML_CL_SMEM) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) != cudaSuccess || nc < 1) {
+            (void)cudaGetLastError();
+            ml_clusters_ = 0;
+        }
+    };
+    ask(k_ml_small<D, double, 4, 16>);
+    ask(k_ml_small<D, double, 8, 32>);
+    ask(k_ml_small<D, double, 8, 64>);
+    ask(k_ml_small<D, float, 4, 16>);
+    ask(k_ml_small<D, float, 8, 32>);
+    ask(k_ml_small<D, float, 8, 64>);
+    return ml_clusters_;
+}
+
+// The whole loop in one cluster; false where this solve's matrix form has no
+// such kernel.
+template <int D>
+template <class TM>
+bool Engine<D>::ml_small_solve(const PcgBufs<TM> &v, double tol, int maxit, const double *zprev)
+{
+    if (sizeof(TM) == 4 && !(v.ac && v.dsum && !v.A64)) return false;
+    MlSmall a{};
+    a.n_eq = n_eq_;
+    a.nact = act_off_[1 << D];
+    a.na1 = mlc_.lo[1];
+    a.nd = mlc_.lo[ml_ld_ + 1] - mlc_.lo[ml_ld_];
+    a.additive = ml_add_;
+    a.stride = cap_;
+    a.resume = zprev != nullptr;
+    a.maxit = maxit;
+    a.tol = tol;
+    a.desc = adesc_.p;
+    a.frac = mlfrac_.p;
+    a.row_ptr = row_ptr_.p;
+    a.col = col_.p;
+    if constexpr (sizeof(TM) == 8) a.A = v.A;
+    a.dsum = v.dsum;
+    a.ac = v.ac;
+    a.dinv = jdinv_.p;
+    a.b = v.b;
+    a.zprev = zprev;
+    a.ncell = mlncell_.p;
+    a.cellnode = mlcellnode_.p;
+    a.fine = mlfine_.p;
+    a.parent = mlparent_.p;
+    a.dinv1 = mldinv_.p;
+    a.M = mlM_last_;
+    a.x = v.x;
+    a.r = v.r;
+    a.z = v.z;
+    a.p = v.p;
+    a.Ap = v.Ap;
+    a.csum = mlcsum_.p;
+    a.xd = mlxd_.p;
+    a.sc = sc_.p;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    // the rest of the shared memory for the matrix, at a margin over an even share
+    size_t vec = sizeof(double) * ml_small_vectors(), entry = sizeof(TM) == 8 ? 12 : 8;
+    size_t room = (ML_CL_SMEM - vec) / entry, share = (size_t)nnz_ / ML_CL + (size_t)nnz_ / (4 * ML_CL) + 64;
+    a.cache = (int)(std::min(room, share) & ~(size_t)1);
+    ml_cluster_config(cfg, attr, vec + entry * (size_t)a.cache, st_);
+    // short rows and small cells (2-D, small radii) take fewer lanes
+    if (nnz_ < 48LL * n_eq_) MPS_CUDA(cudaLaunchKernelEx(&cfg, k_ml_small<D, TM, 4, 16>, a));
+    else if (n_eq_ < 24LL * a.nact) MPS_CUDA(cudaLaunchKernelEx(&cfg, k_ml_small<D, TM, 8, 32>, a));
+    else MPS_CUDA(cudaLaunchKernelEx(&cfg, k_ml_small<D, TM, 8, 64>, a));
+    ++launch_counter();
+    return true;
 }
 
 // x += alpha p, r -= alpha Ap, r.r and the cells' parts of P^T r (the last
@@ -1850,6 +1979,11 @@ void Engine<D>::pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc,
     using T = double;
     const int RB = red_grid(n_eq, CG_BLOCK);
     int iter_before = 0;
+    if (icc && ml_on_ && ml_small_ && !profiling && ml_small_solve<TM>(v, tol, maxit, zprev)) {
+        MPS_CUDA(cudaMemcpyAsync(sc_host_, sc_.p, sizeof(CGScalars), cudaMemcpyDeviceToHost, st_));
+        MPS_CUDA(cudaStreamSynchronize(st_));
+        return;
+    }
     if (!zprev) {
         CGScalars init{};
         init.tol = tol;

@@ -308,13 +308,14 @@ __global__ void k_ml_rows(State<D> s, Grid<D> cg, int n_eq, int stride, const in
     dinv[r] = a > 0.0 ? 1.0 / a : (a <= 0.0 ? 1.0e30 : a);   // NaN stays NaN
 }
 
-// Weights of a row on its cell's corners, all zero for a row left out of P.
+// Weights of a position in a cell on the cell's corners, all zero for a row
+// left out of P.
 template <int D>
-__device__ __forceinline__ void ml_weights(const float *__restrict__ frac, int stride, int r, double *w)
+__device__ __forceinline__ void ml_weights_of(const float *f32, double *w)
 {
     double f[D];
 #pragma unroll
-    for (int d = 0; d < D; d++) f[d] = (double)__ldg(&frac[(size_t)d * stride + r]);
+    for (int d = 0; d < D; d++) f[d] = (double)f32[d];
     double on = f[0] < 0.0 ? 0.0 : 1.0;
     double x0 = on * (1.0 - f[0]), x1 = on * f[0];
     double y0 = 1.0 - f[1], y1 = f[1];
@@ -330,6 +331,15 @@ __device__ __forceinline__ void ml_weights(const float *__restrict__ frac, int s
             w[k] = w[k] * z0;
         }
     }
+}
+
+template <int D>
+__device__ __forceinline__ void ml_weights(const float *__restrict__ frac, int stride, int r, double *w)
+{
+    float f[D];
+#pragma unroll
+    for (int d = 0; d < D; d++) f[d] = __ldg(&frac[(size_t)d * stride + r]);
+    ml_weights_of<D>(f, w);
 }
 
 // ---- Galerkin operators -------------------------------------------------------------------
@@ -748,14 +758,13 @@ k_ml_dense(MlGrid f, MlGrid c, int lo, int nf, int loc, int na1, const int *__re
 
 // ---- one application -------------------------------------------------------------------------
 
-// Reduces NV = 8 or 4 values per lane over the warp; afterwards lane
-// (corner << (5 - log2 NV)) holds the sum of value `corner`.
-template <int NV>
-__device__ __forceinline__ double ml_warp_reduce(double *v, int lane)
+// Reduces NV = 8 or 4 values per lane over groups of W lanes; afterwards the
+// group's lanes [v W / NV, (v + 1) W / NV) hold the sum of value v.
+template <int NV, int W = 32>
+__device__ __forceinline__ double ml_group_reduce(double *v, int lane)
 {
-    int n = NV;
 #pragma unroll
-    for (int o = 16, h = NV / 2; h >= 1; o >>= 1, h >>= 1) {
+    for (int o = W / 2, h = NV / 2; h >= 1; o >>= 1, h >>= 1) {
         bool up = lane & o;
 #pragma unroll
         for (int i = 0; i < NV / 2; i++) {
@@ -764,12 +773,10 @@ __device__ __forceinline__ double ml_warp_reduce(double *v, int lane)
                 v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
         }
-        n = h;
     }
     double s = v[0];
-    (void)n;
 #pragma unroll
-    for (int o = 16 / NV; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    for (int o = W / NV / 2; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     return s;
 }
 
@@ -810,7 +817,7 @@ k_ml_update(int nact, const int2 *__restrict__ desc, const float *__restrict__ f
 #pragma unroll
             for (int k = 0; k < NC; k++) s[k] = fma(w[k], ri, s[k]);
         }
-        double v = ml_warp_reduce<NC>(s, lane);
+        double v = ml_group_reduce<NC>(s, lane);
         constexpr int SH = D == 3 ? 2 : 3;
         if ((lane & ((1 << SH) - 1)) == 0) csum[(size_t)kk * NC + (lane >> SH)] = v;
     }
@@ -1103,6 +1110,401 @@ __global__ void __launch_bounds__(CG_BLOCK) k_ml_matvec(MlVecs v, int lo, int n,
 #pragma unroll
     for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
     if (lane == 0) v.x[o] = s;
+}
+
+// ---- small systems: the whole loop in one cluster ------------------------------------
+//
+// Below some ten thousand unknowns an iteration of the launched kernels is
+// six or seven launches of 3-9 us, nearly all of it launch and drain.  Here
+// one cluster of ML_CL CTAs runs the loop to its end, four cluster barriers an
+// iteration (the product, the update, the coarse correction, its
+// interpolation).  A barrier costs about 1,700 cycles and a load from L2 about
+// 700, so what counts is the number of dependent ones: the direction and the
+// CTA's rows of the matrix (where they fit) sit in shared memory, loads go out
+// in predicated batches, the dot products' parts are stored into every CTA's
+// shared memory, and every CTA forms the direction, the first grid's
+// right-hand side and the additive form's second whole.
+
+constexpr int ML_CL = 16;
+constexpr int ML_CL_THREADS = 1024;
+constexpr size_t ML_CL_SMEM = 216 * 1024;        // dynamic shared memory at most
+
+struct MlSmall {
+    int n_eq, nact, na1, nd, additive, stride, resume, maxit;
+    int cache;   // matrix entries a CTA can hold in shared memory
+    double tol;
+    const int2 *desc;
+    const float *frac;
+    const int *row_ptr, *col;
+    const double *A, *dsum;
+    const uint2 *ac;
+    const double *dinv, *b, *zprev;
+    const int *ncell, *cellnode, *fine, *parent;   // node numbers: corners of a cell, I^T's and I's entries
+    const double *dinv1, *M;
+    double *x, *r, *z, *p, *Ap, *csum, *xd;
+    CGScalars *sc;
+};
+
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+struct MlTotals {
+    double part[3][ML_CL];
+    double sh[ML_CL_THREADS / 32];
+};
+
+// This CTA's part of a dot product, into every CTA's table; the cluster
+// barrier that follows makes it readable.
+__device__ __forceinline__ void ml_cluster_part(double v, int slot, MlTotals &t)
+{
+    v = block_sum<ML_CL_THREADS>(v, t.sh);
+    if (threadIdx.x < 32) {
+        v = __shfl_sync(0xffffffffu, v, 0);
+        if (threadIdx.x < ML_CL) {
+            unsigned local = smem_u32(&t.part[slot][blockIdx.x]), remote;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(threadIdx.x));
+            asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(v) : "memory");
+        }
+    }
+}
+
+// The sum of a slot's parts, the same bits in every thread of the cluster.
+__device__ __forceinline__ double ml_cluster_total(int slot, const MlTotals &t)
+{
+    double s = 0.0;
+    const volatile double *p = t.part[slot];
+#pragma unroll
+    for (int c = 0; c < ML_CL; c++) s += p[c];
+    return s;
+}
+
+// TM = float: the packed FP32 matrix in difference form (k_cg_spmv).
+//
+// Rows are taken cell by cell, W lanes per cell (64: two warps, each with its
+// own part of the cell's sums).  A lane's first row, the only one in most
+// cells, lives in registers with its weights: an acquire at the cluster
+// barrier empties L1, so anything read again comes from L2.
+template <int D, class TM, int LPR, int W>
+__global__ void __launch_bounds__(ML_CL_THREADS) k_ml_small(const __grid_constant__ MlSmall a)
+{
+    constexpr int NC = 1 << D, CELLS = MlDim<D>::CELLS;
+    constexpr int NW = ML_CL * ML_CL_THREADS / 32;
+    extern __shared__ __align__(16) double dyn[];
+    __shared__ MlTotals tot;
+    // shared: the direction, b_1, b_2, the CTA's matrix entries (values and columns, or words)
+    double *ps = dyn, *b1 = ps + a.n_eq, *b2 = b1 + a.na1;
+    double *mval = b2 + (a.additive ? a.nd : 0);
+    uint2 *mac = reinterpret_cast<uint2 *>(mval);
+    int *mcol = reinterpret_cast<int *>(mval + a.cache);
+    constexpr int PARTS = W > 32 ? W / 32 : 1, WL = W < 32 ? W : 32;   // warps of a cell; lanes of one in a warp
+    constexpr int CELLS_PASS = NW * 32 / W;
+    int tid = threadIdx.x, lane = tid & 31;
+    int warp = blockIdx.x * (ML_CL_THREADS / 32) + (tid >> 5);
+    int wl = lane & (WL - 1), part = warp & (PARTS - 1);
+    int hl = wl + 32 * part;
+    int first = W < 32 ? warp * (32 / WL) + lane / WL : warp / PARTS;   // this lane's first cell
+
+    // the CTA's rows of the product
+    int rb = (int)((long long)a.n_eq * blockIdx.x / ML_CL), re = (int)((long long)a.n_eq * (blockIdx.x + 1) / ML_CL);
+    int e0 = __ldg(&a.row_ptr[rb]), ne = __ldg(&a.row_ptr[re]) - e0;
+    bool cached = ne <= a.cache;
+    if (cached) {
+        for (int e = tid; e < ne; e += ML_CL_THREADS) {
+            if (sizeof(TM) == 8) {
+                mval[e] = __ldg(&a.A[e0 + e]);
+                mcol[e] = __ldg(&a.col[e0 + e]);
+            } else {
+                mac[e] = __ldg(&a.ac[e0 + e]);
+            }
+        }
+    }
+
+    // this lane's first row
+    int rounds = (a.nact + CELLS_PASS - 1) / CELLS_PASS;
+    int kk0 = first;
+    int2 dd0 = kk0 < a.nact ? __ldg(&a.desc[kk0]) : make_int2(0, 0);
+    int nd0 = kk0 < a.nact && wl < NC ? __ldg(&a.cellnode[(size_t)kk0 * NC + wl]) : 0;
+    bool own = hl < dd0.y;
+    int i0 = dd0.x + hl;
+    float f0[D];
+#pragma unroll
+    for (int d = 0; d < D; d++) f0[d] = own ? __ldg(&a.frac[(size_t)d * a.stride + i0]) : -1.0f;
+    double r0 = 0.0, x0 = 0.0;
+    if (own) {
+        r0 = a.resume ? a.r[i0] : a.b[i0];
+        x0 = a.resume ? a.x[i0] : 0.0;
+    }
+
+    // x += alpha p, r -= alpha Ap where `step`; r.r and the cells' parts of P^T r
+    auto update = [&](bool step, double alpha) {
+        double rr = 0.0;
+        for (int q = 0; q < rounds; q++) {
+            int kk = first + q * CELLS_PASS;
+            bool in = kk < a.nact;
+            int2 dd = q == 0 ? dd0 : in ? __ldg(&a.desc[kk]) : make_int2(0, 0);
+            double s[NC];
+#pragma unroll
+            for (int k = 0; k < NC; k++) s[k] = 0.0;
+            for (int i = dd.x + hl; i < dd.x + dd.y; i += W) {
+                double ri, w[NC];
+                if (q == 0 && i == i0) {
+                    if (step) {
+                        x0 = fma(alpha, ps[i], x0);
+                        r0 = fma(-alpha, __ldcg(&a.Ap[i]), r0);
+                    }
+                    ri = r0;
+                    ml_weights_of<D>(f0, w);
+                } else {
+                    if (step) {
+                        a.x[i] = fma(alpha, ps[i], a.x[i]);
+                        ri = fma(-alpha, __ldcg(&a.Ap[i]), a.r[i]);
+                        a.r[i] = ri;
+                    } else if (a.resume) {
+                        ri = a.r[i];
+                    } else {
+                        ri = a.b[i];
+                        a.x[i] = 0.0;
+                        a.r[i] = ri;
+                    }
+                    ml_weights<D>(a.frac, a.stride, i, w);
+                }
+                rr = fma(ri, ri, rr);
+#pragma unroll
+                for (int k = 0; k < NC; k++) s[k] = fma(w[k], ri, s[k]);
+            }
+            double v = ml_group_reduce<NC, WL>(s, lane);
+            if (in && wl % (WL / NC) == 0) a.csum[((size_t)kk * PARTS + part) * NC + wl / (WL / NC)] = v;
+        }
+        ml_cluster_part(rr, 1, tot);
+    };
+
+    // z = D^-1 r + P M P^T r for the cluster's rows from the cells' parts, and r.z
+    auto precondition = [&]() {
+        for (int t = tid; t < a.na1; t += ML_CL_THREADS) {
+            double s = 0.0;
+#pragma unroll
+            for (int k = 0; k < NC; k++) {
+                int c = __ldg(&a.ncell[(size_t)k * a.na1 + t]);
+#pragma unroll
+                for (int u = 0; u < PARTS; u++)
+                    s += c >= 0 ? __ldcg(&a.csum[((size_t)c * PARTS + u) * NC + k]) : 0.0;
+            }
+            b1[t] = s;
+        }
+        __syncthreads();
+        const double *bd = b1;
+        if (a.additive) {
+            for (int t = tid; t < a.nd; t += ML_CL_THREADS) {
+                double s = 0.0;
+#pragma unroll
+                for (int j = 0; j < CELLS; j++) {
+                    int f = __ldg(&a.fine[(size_t)j * a.nd + t]);
+                    double w = (j % 3 != 1 ? 0.5 : 1.0) * ((j / 3) % 3 != 1 ? 0.5 : 1.0) *
+                               (D == 3 && j / 9 != 1 ? 0.5 : 1.0);
+                    s = fma(w, f >= 0 ? b1[f] : 0.0, s);
+                }
+                b2[t] = s;
+            }
+            __syncthreads();
+            bd = b2;
+        }
+        for (int t = warp; t < a.nd; t += NW) {
+            const double *M = a.M + (size_t)t * a.nd;
+            double s = 0.0;
+            constexpr int U = 8;
+            for (int j0 = lane; j0 < a.nd; j0 += 32 * U) {
+                double m[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) m[u] = j0 + 32 * u < a.nd ? __ldg(&M[j0 + 32 * u]) : 0.0;
+#pragma unroll
+                for (int u = 0; u < U; u++) s = fma(m[u], j0 + 32 * u < a.nd ? bd[j0 + 32 * u] : 0.0, s);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) a.xd[t] = s;
+        }
+        cluster_sync();
+        double rz = 0.0;
+        for (int q = 0; q < rounds; q++) {
+            int kk = first + q * CELLS_PASS;
+            bool in = kk < a.nact;
+            int2 dd = q == 0 ? dd0 : in ? __ldg(&a.desc[kk]) : make_int2(0, 0);
+            double c = 0.0;
+            if (in && wl < NC) {
+                int nd = q == 0 ? nd0 : __ldg(&a.cellnode[(size_t)kk * NC + wl]);
+                if (a.additive) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int j = 0; j < NC; j++) s += __ldcg(&a.xd[__ldg(&a.parent[(size_t)nd * NC + j])]);
+                    c = fma(__ldg(&a.dinv1[nd]), b1[nd], s * (1.0 / NC));
+                } else {
+                    c = __ldcg(&a.xd[nd]);
+                }
+            }
+            double xc[NC];
+#pragma unroll
+            for (int k = 0; k < NC; k++) xc[k] = __shfl_sync(0xffffffffu, c, k, WL);
+            for (int i = dd.x + hl; i < dd.x + dd.y; i += W) {
+                double ri, w[NC];
+                double zi = __ldg(&a.dinv[i]);
+                if (q == 0 && i == i0) {
+                    ri = r0;
+                    ml_weights_of<D>(f0, w);
+                } else {
+                    ri = a.r[i];
+                    ml_weights<D>(a.frac, a.stride, i, w);
+                }
+                zi *= ri;
+#pragma unroll
+                for (int k = 0; k < NC; k++) zi = fma(w[k], xc[k], zi);
+                a.z[i] = zi;
+                rz = fma(ri, zi, rz);
+            }
+        }
+        ml_cluster_part(rz, 2, tot);
+    };
+
+    cluster_sync();   // every CTA runs before its shared memory is stored to
+    int iter = a.resume ? a.sc->iter : 0;
+    update(false, 0.0);
+    cluster_sync();
+    double rr = ml_cluster_total(1, tot);
+    precondition();
+    cluster_sync();
+    double rz = ml_cluster_total(2, tot);
+    for (int j = tid; j < a.n_eq; j += ML_CL_THREADS) {
+        double z = __ldcg(&a.z[j]);
+        ps[j] = a.resume ? a.p[j] + (z - a.zprev[j]) : z;
+    }
+    __syncthreads();
+    bool breakdown = false;
+    double pAp = 0.0, alpha = 0.0, beta = 0.0;
+    for (;;) {
+        // the loop head of k_cg_spmv; every thread holds the same scalars
+        if (sqrt(rr) < a.tol || iter >= a.maxit) break;
+        if (isnan(rr)) {
+            breakdown = true;
+            break;
+        }
+        double acc = 0.0;
+        for (int t = tid; t < (((re - rb) * LPR + 31) & ~31); t += ML_CL_THREADS) {
+            int r = rb + t / LPR;
+            bool in = r < re;
+            int q0 = in ? __ldg(&a.row_ptr[r]) - e0 : 0, q1 = in ? __ldg(&a.row_ptr[r + 1]) - e0 : 0;
+            double pr = in ? ps[r] : 0.0;
+            double s = 0.0;
+            constexpr int U = 8;
+            for (int q = q0 + (t & (LPR - 1)); q < q1; q += LPR * U) {
+                double v[U];
+                int c[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    int e = q + u * LPR;
+                    v[u] = 0.0;
+                    c[u] = r;
+                    if (e < q1) {
+                        if (sizeof(TM) == 8) {
+                            v[u] = cached ? mval[e] : __ldg(&a.A[e0 + e]);
+                            c[u] = cached ? mcol[e] : __ldg(&a.col[e0 + e]);
+                        } else {
+                            uint2 w = cached ? mac[e] : __ldg(&a.ac[e0 + e]);
+                            v[u] = (double)__uint_as_float(w.x);
+                            c[u] = (int)w.y;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) s = fma(v[u], sizeof(TM) == 8 ? ps[c[u]] : ps[c[u]] - pr, s);
+            }
+#pragma unroll
+            for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (in && (t & (LPR - 1)) == 0) {
+                if (sizeof(TM) == 4) s = fma(__ldg(&a.dsum[r]), pr, s);
+                a.Ap[r] = s;
+                acc = fma(pr, s, acc);
+            }
+        }
+        ml_cluster_part(acc, 0, tot);
+        cluster_sync();
+        pAp = ml_cluster_total(0, tot);
+        if (fabs(pAp) < 1.0e-30) {
+            breakdown = true;
+            break;
+        }
+        alpha = rz / pAp;
+        update(true, alpha);
+        cluster_sync();
+        rr = ml_cluster_total(1, tot);
+        precondition();
+        cluster_sync();
+        double rz_new = ml_cluster_total(2, tot);
+        if (fabs(rz) < 1.0e-60) {
+            breakdown = true;
+            break;
+        }
+        beta = rz_new / rz;
+        rz = rz_new;
+        for (int j = tid; j < a.n_eq; j += ML_CL_THREADS) ps[j] = fma(beta, ps[j], __ldcg(&a.z[j]));
+        __syncthreads();
+        iter++;
+    }
+    // what a resumed loop and the caller read
+    if (own) {
+        a.x[i0] = x0;
+        a.r[i0] = r0;
+    }
+    for (int j = rb + tid; j < re; j += ML_CL_THREADS) a.p[j] = ps[j];
+    if (blockIdx.x == 0 && tid == 0) {
+        CGScalars *sc = a.sc;
+        sc->rr = rr;
+        sc->rz = rz;
+        sc->pAp = pAp;
+        sc->alpha = alpha;
+        sc->beta = beta;
+        sc->tol = a.tol;
+        sc->maxit = a.maxit;
+        sc->iter = iter;
+        sc->done = 1;
+        sc->breakdown = breakdown;
+    }
+}
+
+// Node numbers the cluster loop needs: the corners of every active cell, and,
+// with an additive first grid, the fine nodes under every coarse node ([entry]
+// [node], -1 where there is none) and the 2^D parents of every fine node.
+template <int D>
+__global__ void k_ml_small_tables(int nact, int na1, int nd, bool additive, MlGrid f, MlGrid c,
+                                  const int *__restrict__ cnode, const int *__restrict__ amap,
+                                  const int *__restrict__ under, const int *__restrict__ above,
+                                  const unsigned char *__restrict__ parity, int *__restrict__ cellnode,
+                                  int *__restrict__ fine, int *__restrict__ parent)
+{
+    constexpr int NC = 1 << D, CELLS = MlDim<D>::CELLS;
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < nact) {
+#pragma unroll
+        for (int k = 0; k < NC; k++)
+            cellnode[(size_t)t * NC + k] = amap[cnode[t] + (k & 1) + f.s1 * ((k >> 1) & 1) + f.s2 * (k >> 2)];
+    }
+    if (!additive) return;
+    if (t < nd) {
+        int o = under[na1 + t];
+#pragma unroll
+        for (int j = 0; j < CELLS; j++)
+            fine[(size_t)j * nd + t] =
+                amap[o + j % 3 - 1 + f.s1 * ((j / 3) % 3 - 1) + (D == 3 ? f.s2 * (j / 9 - 1) : 0)];
+    }
+    if (t < na1) {
+        int q0 = above[t], par = parity[t];
+#pragma unroll
+        for (int j = 0; j < NC; j++) {
+            int px = 1 + ((par & 1) & (j & 1)), py = 1 + (((par >> 1) & 1) & ((j >> 1) & 1));
+            int pz = D == 3 ? 1 + ((par >> 2) & (j >> 2)) : 0;
+            parent[(size_t)t * NC + j] = amap[q0 + px + c.s1 * py + c.s2 * pz] - na1;
+        }
+    }
 }
 
 }  // namespace mps

@@ -5,7 +5,8 @@ oracle elsewhere; the pressures agree to the solver's rounding.  Cases: both
 dimensions and precision forms, the additive and the multiplicative first
 grid (MPS_ML_ADD), the V-cycle dense from the coarsest grid on and from the
 first grid of at most 1,024 nodes on (MPS_ML_DENSE), grids of odd and even
-extents, and cells with up to ~90 unknowns.  Tolerances: pressure 1e-8, velocity 1e-10 and
+extents, cells with up to ~90 unknowns, and the loop as launches and in one
+cluster (MPS_ML_SMALL).  Tolerances: pressure 1e-8, velocity 1e-10 and
 position 1e-14 relative L2 after one step, as for a step against the oracle.
 
 A wall region that no known pressure bounds and no source reaches keeps the
@@ -34,7 +35,7 @@ def _rel(a, b):
 
 def _step(monkeypatch, wl, precision, steps=1, **env):
     from mps_b200.session import start
-    for k in ("MPS_SWEEP", "MPS_ML_ADD", "MPS_ML_DENSE"):
+    for k in ("MPS_SWEEP", "MPS_ML_ADD", "MPS_ML_DENSE", "MPS_ML_SMALL"):
         monkeypatch.delenv(k, raising=False)
     for k, v in env.items():
         monkeypatch.setenv(k, v)
@@ -74,17 +75,18 @@ def test_multilevel_matches_ic0(name, precision, monkeypatch):
     ref, mref = _step(monkeypatch, wl, precision, MPS_SWEEP="0")
     for add in ("0", "1000000"):
         for dense in ("0", "150", "1024"):
-            g, m = _step(monkeypatch, wl, precision, MPS_ML_ADD=add, MPS_ML_DENSE=dense)
-            assert m["converged"] == 1
-            for f in ("n", "on_surface", "type"):
-                assert np.array_equal(g[f], ref[f]), f
-            assert _rel(g["pressure"], ref["pressure"]) < 1e-8
-            assert _rel(g["vel"], ref["vel"]) < 1e-10
-            assert _rel(g["pos"], ref["pos"]) < 1e-14
-            if name == "droplet":
-                wall = g["type"] == T.WALL
-                assert np.abs(g["pressure"]).max() > 0.0
-                assert np.all(g["pressure"][wall] == 0.0) and np.all(ref["pressure"][wall] == 0.0)
+            for small in ("0", "1000000"):
+                g, m = _step(monkeypatch, wl, precision, MPS_ML_ADD=add, MPS_ML_DENSE=dense, MPS_ML_SMALL=small)
+                assert m["converged"] == 1
+                for f in ("n", "on_surface", "type"):
+                    assert np.array_equal(g[f], ref[f]), f
+                assert _rel(g["pressure"], ref["pressure"]) < 1e-8
+                assert _rel(g["vel"], ref["vel"]) < 1e-10
+                assert _rel(g["pos"], ref["pos"]) < 1e-14
+                if name == "droplet":
+                    wall = g["type"] == T.WALL
+                    assert np.abs(g["pressure"]).max() > 0.0
+                    assert np.all(g["pressure"][wall] == 0.0) and np.all(ref["pressure"][wall] == 0.0)
 
 
 def test_multilevel_reruns_are_bit_identical(monkeypatch):
