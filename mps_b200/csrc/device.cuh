@@ -291,7 +291,61 @@ struct NbrSource {
             f(j);
         }
     }
+
+    // for_each with the neighbours' data: use(j, load(j)) in list order, the
+    // loads of U neighbours issued together and the next U indices before
+    // them, so that a thread waits for memory once per U neighbours.
+    template <int U = 4, class Ld, class F>
+    __device__ __forceinline__ void for_each_with(int i, Ld &&load, F &&use) const
+    {
+        int c = __ldg(&cnt[i]);
+        if (c > pitch) {
+            cells.for_each(i, [&](int j) { use(j, load(j)); });
+            return;
+        }
+        const int *p = idx + (size_t)(i >> 5) * 32 * pitch + (i & 31);
+        int jn[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) jn[u] = u < c ? __ldg(p + 32 * u) : i;
+        for (int k = 0; k < c; k += U) {
+            int j[U];
+            decltype(load(0)) d[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) j[u] = jn[u];
+#pragma unroll
+            for (int u = 0; u < U; u++) d[u] = load(j[u]);   // past the end: the particle itself
+#pragma unroll
+            for (int u = 0; u < U; u++) jn[u] = k + U + u < c ? __ldg(p + 32 * (k + U + u)) : i;
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (k + u < c) use(j[u], d[u]);
+        }
+    }
 };
+
+// A neighbour's data, loaded together.
+template <int D>
+struct PosData {
+    double x[D];
+};
+template <int D>
+struct PosVelData {
+    double x[D], v[D];
+    int type;
+};
+template <int D>
+struct PosValData {
+    double x[D], p;
+};
+
+template <int D>
+__device__ __forceinline__ PosData<D> load_pos(const State<D> &s, int j)
+{
+    PosData<D> d;
+#pragma unroll
+    for (int k = 0; k < D; k++) d.x[k] = s.pos[k][j];
+    return d;
+}
 
 // Neighbours from a caller-supplied list (CSR of the reference's
 // NeighborList, entries in engine indices).
@@ -304,6 +358,12 @@ struct ListSource {
     {
         int e = ptr[i + 1];
         for (int k = ptr[i]; k < e; k++) f(idx[k]);
+    }
+
+    template <int U = 1, class Ld, class F>
+    __device__ __forceinline__ void for_each_with(int i, Ld &&load, F &&use) const
+    {
+        for_each(i, [&](int j) { use(j, load(j)); });
     }
 };
 

@@ -474,6 +474,10 @@ private:
     int nbr_pitch_ = 0;
     // bytes the lists may take; beyond, operators walk the cells
     static constexpr double kNbrBytes = 24.0e9;
+    // particles below which a list is built by several lanes each (MPS_NBR_LANES);
+    // measured, a thread against eight lanes: 6,606 particles 122 / 55 us, 28 k
+    // 53 / 30, 118 k 168 / 206
+    int nbr_lanes_below_ = 60000;
 
     void alloc_state();
     void build_grid();
@@ -549,6 +553,7 @@ Engine<D>::Engine(const mps_params_t &p, int capacity)
         sweep_mode_ = (v == 0 || v == 1 || v == 3) ? v : 2;
     }
     if (const char *e = std::getenv("MPS_ML_ADD")) ml_add_rows_ = std::max(0, std::atoi(e));
+    if (const char *e = std::getenv("MPS_NBR_LANES")) nbr_lanes_below_ = std::max(0, std::atoi(e));
     if (const char *e = std::getenv("MPS_ML_SMALL")) ml_small_rows_ = std::max(0, std::atoi(e));
     if (const char *e = std::getenv("MPS_ML_DENSE")) ml_dense_ = std::min(ML_DENSE, std::max(0, std::atoi(e)));
     if (const char *e = std::getenv("MPS_SWEEP_HB")) head_batch_ = std::atoi(e) == 8 ? 8 : 4;
@@ -1020,8 +1025,12 @@ NbrSource<D> Engine<D>::near()
         for (int d = 0; d < D; d++) ext = std::max(ext, g_.dims[d]);
         float band = ext > 1000000 ? 1.0e30f : 8.0f * 1.1920929e-7f * (float)ext + 4.0e-6f;
         launch(k_key_cells<D>, nblk(n, TPB), TPB, 0, st_, S(), g_, n, keyf_.p);
-        launch(k_nbr_list<D>, nblk(n, 128), 128, 0, st_, cells(), n, (const float4 *)keyf_.p, band, nbr_pitch_,
-               nbr_idx_.p, nbr_cnt_.p);
+        if (n < nbr_lanes_below_)
+            launch(k_nbr_list_lanes<D>, nblk((long long)n * NBR_LANES, 128), 128, 0, st_, cells(), n,
+                   (const float4 *)keyf_.p, band, nbr_pitch_, nbr_idx_.p, nbr_cnt_.p);
+        else
+            launch(k_nbr_list<D>, nblk(n, 128), 128, 0, st_, cells(), n, (const float4 *)keyf_.p, band, nbr_pitch_,
+                   nbr_idx_.p, nbr_cnt_.p);
         nbr_valid_ = true;
     }
     src.idx = nbr_idx_.p;
@@ -1396,7 +1405,9 @@ void Engine<D>::ml_build(int n_eq)
     launch(k_cell_desc, nblk(nact, TPB), TPB, 0, st_, nact, (const int *)acells_.p, (const int *)cell_row0_.p,
            (const int *)ucount_.p, adesc_.p, err_.p);
     launch(k_uf_init, nblk(n_eq, TPB), TPB, 0, st_, n_eq, rp, dp, ci, A, ufpar_.p, ufkeep_.p);
-    launch(k_uf_hook, nblk((long long)n_eq * 8, TPB), TPB, 0, st_, n_eq, rp, dp, ci, A, ufpar_.p);
+    launch(k_uf_sample, nblk(n_eq, TPB), TPB, 0, st_, n_eq, rp, dp, ci, A, ufpar_.p);
+    launch(k_uf_flatten, nblk(n_eq, TPB), TPB, 0, st_, n_eq, ufpar_.p);
+    launch(k_uf_hook, nblk((long long)n_eq * 8, TPB), TPB, 0, st_, n_eq, rp, ci, A, ufpar_.p);
     launch(k_uf_keep, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const double *)b_.p, (const unsigned char *)bounded_.p,
            ufpar_.p, ufkeep_.p);
     launch(k_ml_rows<D>, nblk(n_eq, TPB), TPB, 0, st_, s, g_, n_eq, cap_, (const int *)part_of_row_.p, dp, A,

@@ -52,10 +52,10 @@ namespace mps {
 
 constexpr int ML_MAXL = 26;       // grids at most: 2^30 cells, even in one direction, reach the coarsest size
 constexpr int ML_BOX = 64;        // the grids end when their box holds at most this many nodes ...
-// ... and a solve's at the first with at most this many nodes in use: its
-// explicit inverse costs 128 pivots once and ends the chain of dependent
-// steps two or three grids earlier.
-constexpr int ML_COARSEST = 128;
+// ... and a solve's at the first with at most this many nodes in use, whose
+// inverse starts the dense V-cycle (128 took 175 us to invert, a pivot at a
+// time; one more grid costs 30).
+constexpr int ML_COARSEST = 64;
 // Nodes up to which a grid's V-cycle is held as a dense matrix: 8 MB at most,
 // read from L2 in about 3 us, against three dependent launches per grid for
 // the steps it replaces.
@@ -248,28 +248,49 @@ __global__ void k_uf_init(int n, const int *__restrict__ row_ptr, const int *__r
     keep[r] = 0;
 }
 
-// Eight lanes per row take its lower entries.
-__global__ void k_uf_hook(int n, const int *__restrict__ row_ptr, const int *__restrict__ diagpos,
-                          const int *__restrict__ col, const double *__restrict__ A, int *parent)
+// Joins the trees of rows i and j: the larger root goes under the smaller.
+__device__ __forceinline__ void uf_join(int *parent, int i, int j)
+{
+    int a = uf_find(parent, i), b = uf_find(parent, j);
+    while (a != b) {
+        if (a < b) { int t = a; a = b; b = t; }
+        int old = atomicCAS(&parent[a], a, b);
+        if (old == a) break;
+        a = uf_find(parent, old);
+        b = uf_find(parent, b);
+    }
+}
+
+// Most rows belong to one tree after a few of their entries (Sutton, Ben-Nun,
+// Barak 2018, "Optimizing parallel graph connectivity computation via
+// subgraph sampling"): three entries of every row first, then all entries of
+// the rows that are not in the first row's tree.
+__global__ void k_uf_sample(int n, const int *__restrict__ row_ptr, const int *__restrict__ diagpos,
+                            const int *__restrict__ col, const double *__restrict__ A, int *parent)
+{
+    int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    int a = row_ptr[r], d = diagpos[r], e = row_ptr[r + 1];
+    int q[3] = {(a + d) / 2, d - 1, e - 1};
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        if (q[k] >= a && q[k] != d && A[q[k]] != 0.0) uf_join(parent, r, col[q[k]]);
+}
+
+__global__ void k_uf_flatten(int n, int *parent)
+{
+    int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < n) parent[r] = uf_find(parent, r);
+}
+
+// Eight lanes per row.
+__global__ void k_uf_hook(int n, const int *__restrict__ row_ptr, const int *__restrict__ col,
+                          const double *__restrict__ A, int *parent)
 {
     int r = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 3);
-    if (r >= n) return;
-    int last = -1;
-    for (int q = row_ptr[r] + (threadIdx.x & 7); q < diagpos[r]; q += 8) {
-        int j = col[q];
-        if (A[q] == 0.0) continue;
-        int b = uf_find(parent, j);
-        if (b == last) continue;
-        int a = uf_find(parent, r);
-        while (a != b) {
-            if (a < b) { int t = a; a = b; b = t; }
-            int old = atomicCAS(&parent[a], a, b);   // the larger root under the smaller
-            if (old == a) break;
-            a = uf_find(parent, old);
-            b = uf_find(parent, b);
-        }
-        last = b;
-    }
+    if (r >= n || uf_find(parent, r) == uf_find(parent, 0)) return;
+    for (int q = row_ptr[r] + (threadIdx.x & 7); q < row_ptr[r + 1]; q += 8)
+        if (A[q] != 0.0) uf_join(parent, r, col[q]);
 }
 
 __global__ void k_uf_keep(int n, const double *__restrict__ b, const unsigned char *__restrict__ bounded,
@@ -571,7 +592,7 @@ k_ml_galerkin(MlGrid f, MlGrid c, int lof, int loc, const int *__restrict__ act,
 }
 
 // Inverse of the coarsest operator (n <= ML_COARSEST nodes), one CTA, the
-// matrix in registers (16 entries a thread): Gauss-Jordan without pivoting on
+// matrix in registers (4 entries a thread): Gauss-Jordan without pivoting on
 // the symmetric matrix, one barrier per pivot.  A pivot that cancellation has
 // emptied (below 1e-9 of its diagonal: a constant on a region no known
 // pressure bounds, or a node no row reaches) is dropped, which keeps the

@@ -38,13 +38,19 @@ __global__ void k_viscosity(Src src, State<D> s, Consts k, int n, int accumulate
     load_vec<D>(vi, s.vel, i);
 #pragma unroll
     for (int d = 0; d < D; d++) lap[d] = 0.0;
-    src.for_each(i, [&](int j) {
-        double pj[D];
-        load_vec<D>(pj, s.pos, j);
-        double w = kweight(sqrt(dist2<D>(pi, pj)), k.re_lap, k.rmin);
+    src.for_each_with(
+        i,
+        [&](int j) {
+            PosVelData<D> q;
+            load_vec<D>(q.x, s.pos, j);
+            load_vec<D>(q.v, s.vel, j);
+            return q;
+        },
+        [&](int, const PosVelData<D> &q) {
+            double w = kweight(sqrt(dist2<D>(pi, q.x)), k.re_lap, k.rmin);
 #pragma unroll
-        for (int d = 0; d < D; d++) lap[d] += (s.vel[d][j] - vi[d]) * w;
-    });
+            for (int d = 0; d < D; d++) lap[d] += (q.v[d] - vi[d]) * w;
+        });
 #pragma unroll
     for (int d = 0; d < D; d++) {
         double a = accumulate ? s.acc[d][i] : k.gravity[d];
@@ -301,13 +307,14 @@ __global__ void k_collision_list(Src src, State<D> s, Consts k, int n, double *_
     if (s.type[i] == FLUID) {
         double pi[D];
         load_vec<D>(pi, s.pos, i);
-        src.for_each(i, [&](int j) {
-            if (s.type[j] == GHOST) return;
-            double pj[D], vj[D];
-            load_vec<D>(pj, s.pos, j);
-            load_vec<D>(vj, s.vel, j);
-            collide<D>(vi, pi, pj, vj, k);
-        });
+        // few pairs are close enough to collide: only those load more than a position
+        src.for_each_with(i, [&](int j) { return load_pos(s, j); },
+                          [&](int j, const PosData<D> &q) {
+                              if (dist2<D>(pi, q.x) >= k.col2 || s.type[j] == GHOST) return;
+                              double vj[D];
+                              load_vec<D>(vj, s.vel, j);
+                              collide<D>(vi, pi, q.x, vj, k);
+                          });
     }
 #pragma unroll
     for (int d = 0; d < D; d++) vafter[(size_t)d * n + i] = vi[d];
@@ -380,14 +387,13 @@ __global__ void k_density(Src src, State<D> s, Consts k, int n, unsigned *err, i
     load_vec<D>(pi, s.pos, i);
     double sum = 0.0;
     int len = 0, cnt = 0;
-    src.for_each(i, [&](int j) {
-        double pj[D];
-        load_vec<D>(pj, s.pos, j);
-        double r2 = dist2<D>(pi, pj);
-        sum += kweight(sqrt(r2), k.re_n, k.rmin);
-        cnt += (r2 < k.re_n2);
-        len++;
-    });
+    src.for_each_with(i, [&](int j) { return load_pos(s, j); },
+                      [&](int, const PosData<D> &q) {
+                          double r2 = dist2<D>(pi, q.x);
+                          sum += kweight(sqrt(r2), k.re_n, k.rmin);
+                          cnt += (r2 < k.re_n2);
+                          len++;
+                      });
     if (check_overflow && len > k.max_nb) atomicOr(err, ERR_NEIGHBOR_OVERFLOW);
     s.n[i] = sum;
     if (!set_flags) return;
@@ -434,10 +440,10 @@ __global__ void k_pmin(Src src, State<D> s, int n, double *__restrict__ pmin)
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double m = s.p[i];
-    src.for_each(i, [&](int j) {
-        double pj = s.p[j];
-        if (pj < m) m = pj;
-    });
+    src.for_each_with(i, [&](int j) { return s.p[j]; },
+                      [&](int, double pj) {
+                          if (pj < m) m = pj;
+                      });
     pmin[i] = m;
 }
 
@@ -452,19 +458,26 @@ __global__ void k_gradient(Src src, State<D> s, Consts k, int n, const double *_
     double pim = pmin ? pmin[i] : 0.0;
 #pragma unroll
     for (int d = 0; d < D; d++) g[d] = 0.0;
-    src.for_each(i, [&](int j) {
-        double pj[D], dr[D];
-        load_vec<D>(pj, s.pos, j);
-        double r2 = dist2v<D>(pi, pj, dr);
-        if (r2 < k.grad_r2min) return;
-        double w = kweight(sqrt(r2), k.re_lap, k.rmin);
-        double dp;
-        if (k.cmps == 1)      dp = Pi + s.p[j] - pim - pmin[j];
-        else if (k.cmps == 2) dp = Pi + s.p[j];
-        else                  dp = s.p[j] - pim;
+    src.for_each_with(
+        i,
+        [&](int j) {
+            PosValData<D> q;
+            load_vec<D>(q.x, s.pos, j);
+            q.p = s.p[j];
+            return q;
+        },
+        [&](int j, const PosValData<D> &q) {
+            double dr[D];
+            double r2 = dist2v<D>(pi, q.x, dr);
+            if (r2 < k.grad_r2min) return;
+            double w = kweight(sqrt(r2), k.re_lap, k.rmin);
+            double dp;
+            if (k.cmps == 1)      dp = Pi + q.p - pim - pmin[j];
+            else if (k.cmps == 2) dp = Pi + q.p;
+            else                  dp = q.p - pim;
 #pragma unroll
-        for (int d = 0; d < D; d++) g[d] += dp / r2 * dr[d] * w;
-    });
+            for (int d = 0; d < D; d++) g[d] += dp / r2 * dr[d] * w;
+        });
 #pragma unroll
     for (int d = 0; d < D; d++) s.acc[d][i] = k.neg_grad * g[d] / k.density;
 }

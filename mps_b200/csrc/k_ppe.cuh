@@ -177,16 +177,16 @@ k_row_count(NbrSource<D> src, State<D> s, const int *__restrict__ part_of_row, c
     int ci = s.cell[i];
     const Grid<D> &g = src.cells.g;
     int prev = ci, nb = CELLS / 2, below = 0;
-    src.for_each(i, [&](int j) {
-        if (row_of[j] < 0) return;
-        int c = s.cell[j];
-        if (c != prev) {
-            prev = c;
-            nb = neighbour_cell<D>(g, c - ci);
-        }
-        cnt[nb][threadIdx.x]++;
-        below += c == ci && j < i;
-    });
+    src.for_each_with(i, [&](int j) { return make_int2(row_of[j], s.cell[j]); },
+                      [&](int j, int2 q) {
+                          if (q.x < 0) return;
+                          if (q.y != prev) {
+                              prev = q.y;
+                              nb = neighbour_cell<D>(g, q.y - ci);
+                          }
+                          cnt[nb][threadIdx.x]++;
+                          below += q.y == ci && j < i;
+                      });
     cnt[CELLS / 2][threadIdx.x]++;
     int par = cell_parity<D>(g, ci);
     int off = 0;
@@ -273,30 +273,40 @@ k_fill(NbrSource<D> src, State<D> s, Consts k, const int *__restrict__ part_of_r
     int prev = -1, pos = base, placed = 1;
     double sum_w = 0.0;
     bool known = k.diag_scale != k.coeff;   // the row sum is not zero
-    src.for_each(i, [&](int j) {
-        if (s.type[j] == DUMMY) return;
-        double pj[D];
-        load_vec<D>(pj, s.pos, j);
-        double w = kweight(sqrt(dist2<D>(pi, pj)), k.re_lap, k.rmin);
-        sum_w += w;
-        int rj = row_of[j];
-        if (rj < 0) {
-            known = known || w > 0.0;
-            return;
-        }
-        int c = s.cell[j];
-        if (c != prev) {
-            prev = c;
-            pos = base + runs[(size_t)visit_rank<D>(par, neighbour_cell<D>(g, c - ci)) * stride + r];
-        }
-        if (pos == dpos) pos++;
-        if (pos < end) {
-            col[pos] = rj;
-            val[pos] = k.neg_coeff * w;
-        }
-        pos++;
-        placed++;
-    });
+    struct Data {
+        double x[D];
+        int type, row, cell;
+    };
+    src.for_each_with(
+        i,
+        [&](int j) {
+            Data q;
+            load_vec<D>(q.x, s.pos, j);
+            q.type = s.type[j];
+            q.row = row_of[j];
+            q.cell = s.cell[j];
+            return q;
+        },
+        [&](int, const Data &q) {
+            if (q.type == DUMMY) return;
+            double w = kweight(sqrt(dist2<D>(pi, q.x)), k.re_lap, k.rmin);
+            sum_w += w;
+            if (q.row < 0) {
+                known = known || w > 0.0;
+                return;
+            }
+            if (q.cell != prev) {
+                prev = q.cell;
+                pos = base + runs[(size_t)visit_rank<D>(par, neighbour_cell<D>(g, q.cell - ci)) * stride + r];
+            }
+            if (pos == dpos) pos++;
+            if (pos < end) {
+                col[pos] = q.row;
+                val[pos] = k.neg_coeff * w;
+            }
+            pos++;
+            placed++;
+        });
     bounded[r] = known;
     diagpos[r] = dpos;
     col[dpos] = r;

@@ -203,6 +203,76 @@ __global__ void k_nbr_list(CellSource<D> src, int n, const float4 *__restrict__ 
     cnt[i] = k;
 }
 
+// The same lists with NBR_LANES lanes per particle, for systems too small to
+// fill the device with a thread each: the lanes take consecutive candidates
+// of a run and a ballot keeps the accepted ones in order.
+constexpr int NBR_LANES = 8;
+
+template <int D>
+__global__ void k_nbr_list_lanes(CellSource<D> src, int n, const float4 *__restrict__ kf, float band, int pitch,
+                                 int *__restrict__ idx, int *__restrict__ cnt)
+{
+    int i = (blockIdx.x * blockDim.x + threadIdx.x) / NBR_LANES;
+    int lane = threadIdx.x & 31, l = lane % NBR_LANES;
+    unsigned group = ((1u << NBR_LANES) - 1u) << (lane - l);
+    if (i >= n) return;   // whole groups
+    int c = src.cell[i];
+    int k = 0;
+    if (c >= 0) {
+        const Grid<D> &g = src.g;
+        float4 me = kf[i];
+        double ki[D];
+#pragma unroll
+        for (int d = 0; d < D; d++) ki[d] = src.key[d][i];
+        int cc[D];
+        int rem = c;
+#pragma unroll
+        for (int d = 0; d < D; d++) { cc[d] = rem % g.dims[d]; rem /= g.dims[d]; }
+        int x0 = cc[0] > 0 ? cc[0] - 1 : 0;
+        int x1 = cc[0] < g.dims[0] - 1 ? cc[0] + 1 : g.dims[0] - 1;
+        int y0 = cc[1] > 0 ? cc[1] - 1 : 0;
+        int y1 = cc[1] < g.dims[1] - 1 ? cc[1] + 1 : g.dims[1] - 1;
+        int z0 = 0, z1 = 0;
+        if (D == 3) {
+            z0 = cc[D - 1] > 0 ? cc[D - 1] - 1 : 0;
+            z1 = cc[D - 1] < g.dims[D - 1] - 1 ? cc[D - 1] + 1 : g.dims[D - 1] - 1;
+        }
+        int *out = idx + (size_t)(i >> 5) * 32 * pitch + (i & 31);
+        for (int z = z0; z <= z1; z++) {
+            for (int y = y0; y <= y1; y++) {
+                int base = (D == 3) ? (z * g.dims[1] + y) * g.dims[0] : y * g.dims[0];
+                int t0 = g.start[base + x0], t1 = g.start[base + x1 + 1];
+#pragma unroll 2
+                for (int tb = t0; tb < t1; tb += NBR_LANES) {
+                    int t = tb + l;
+                    bool hit = false;
+                    if (t < t1) {
+                        float4 o = __ldg(&kf[t]);
+                        float dx = o.x - me.x, dy = o.y - me.y;
+                        float d2 = fmaf(dx, dx, dy * dy);
+                        if (D == 3) {
+                            float dz = o.z - me.z;
+                            d2 = fmaf(dz, dz, d2);
+                        }
+                        hit = d2 < 1.0f + band && t != i;
+                        if (hit && d2 >= 1.0f - band) {
+                            double kt[D];
+#pragma unroll
+                            for (int d = 0; d < D; d++) kt[d] = src.key[d][t];
+                            hit = dist2<D>(ki, kt) < src.re2;
+                        }
+                    }
+                    unsigned m = __ballot_sync(group, hit) >> (lane - l);
+                    int at = k + __popc(m & ((1u << l) - 1u));
+                    if (hit && at < pitch) out[(size_t)at * 32] = t;
+                    k += __popc(m);
+                }
+            }
+        }
+    }
+    if (l == 0) cnt[i] = k;
+}
+
 // Neighbour list in the reference's layout (rows by reference index,
 // entries as reference indices, reference order).  Row r starts at
 // out_nb[r * pitch]; rows longer than max_nb raise the overflow flag.

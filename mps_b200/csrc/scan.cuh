@@ -14,7 +14,8 @@ constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
 template <class T>
-__global__ void k_scan_tile(const T *__restrict__ in, T *__restrict__ out, T *__restrict__ sums, int n)
+__global__ void k_scan_tile(const T *__restrict__ in, T *__restrict__ out, T *__restrict__ sums, T *__restrict__ tot,
+                            int n)
 {
     __shared__ T warp_tot[SCAN_THREADS / 32];
     int base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
@@ -46,6 +47,7 @@ __global__ void k_scan_tile(const T *__restrict__ in, T *__restrict__ out, T *__
         }
         if (lane < SCAN_THREADS / 32) warp_tot[lane] = ti - t;   // exclusive
         if (lane == SCAN_THREADS / 32 - 1 && sums) sums[blockIdx.x] = ti;
+        if (lane == SCAN_THREADS / 32 - 1 && tot) *tot = ti;   // the only tile
     }
     __syncthreads();
     T off = warp_tot[w] + (inc - run);
@@ -55,10 +57,11 @@ __global__ void k_scan_tile(const T *__restrict__ in, T *__restrict__ out, T *__
 }
 
 template <class T>
-__global__ void k_scan_add(T *__restrict__ out, const T *__restrict__ offs, int n)
+__global__ void k_scan_add(T *__restrict__ out, const T *__restrict__ offs, int nb, int n)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] += offs[i / SCAN_TILE];
+    if (i == 0) out[n] = offs[nb];
 }
 
 // out[0..n) = exclusive scan of in[0..n); out[n] = total.  `ws` needs
@@ -75,30 +78,28 @@ inline size_t scan_workspace(int n)
 }
 
 template <class T>
-__global__ void k_scan_total(const T *in, const T *out, T *tot, int n)
+__global__ void k_scan_empty(T *tot)
 {
-    if (n == 0) { *tot = 0; return; }
-    *tot = out[n - 1] + in[n - 1];
+    *tot = T(0);
 }
 
 template <class T>
 void scan_exclusive(const T *in, T *out, int n, T *ws, cudaStream_t st)
 {
     if (n <= 0) {
-        launch(k_scan_total<T>, 1, 1, 0, st, in, out, out, 0);
+        launch(k_scan_empty<T>, 1, 1, 0, st, out);
         return;
     }
     int nb = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (nb == 1) {
-        launch(k_scan_tile<T>, 1, SCAN_THREADS, 0, st, in, out, nullptr, n);
+        launch(k_scan_tile<T>, 1, SCAN_THREADS, 0, st, in, out, (T *)nullptr, out + n, n);
     } else {
         T *sums = ws;
         T *sums_scan = ws + nb;   // nb + 1 entries via the recursion
-        launch(k_scan_tile<T>, nb, SCAN_THREADS, 0, st, in, out, sums, n);
+        launch(k_scan_tile<T>, nb, SCAN_THREADS, 0, st, in, out, sums, (T *)nullptr, n);
         scan_exclusive<T>(sums, sums_scan, nb, ws + 2 * nb + 1, st);
-        launch(k_scan_add<T>, (n + 255) / 256, 256, 0, st, out, sums_scan, n);
+        launch(k_scan_add<T>, (n + 255) / 256, 256, 0, st, out, (const T *)sums_scan, nb, n);
     }
-    launch(k_scan_total<T>, 1, 1, 0, st, in, out, out + n, n);
 }
 
 }  // namespace mps
