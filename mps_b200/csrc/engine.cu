@@ -27,6 +27,7 @@
 #include <numeric>
 
 #include "engine.cuh"
+#include "hostcopy.cuh"
 #include "k_ops.cuh"
 #include "k_ppe.cuh"
 #include "k_pcg.cuh"
@@ -448,6 +449,9 @@ private:
     DevArray<unsigned char> aos_;
     DevArray<double> soa_in_;
     DevArray<int> int_in_;
+    HostPipe pipe_;
+    void copy_to_host(void *host, const void *dev, size_t bytes);     // and wait
+    void copy_to_device(void *dev, const void *host, size_t bytes);   // queued on st_
     CGScalars *sc_host_ = nullptr;
     int *int_host_ = nullptr;
     cudaEvent_t ev_[6];
@@ -902,13 +906,31 @@ void Engine<D>::check_err()
 // ---- state transfer ---------------------------------------------------------
 
 template <int D>
+void Engine<D>::copy_to_host(void *host, const void *dev, size_t bytes)
+{
+    if (HostPipe::wanted(host, bytes)) {
+        pipe_.to_host(host, dev, bytes, st_);
+    } else {
+        MPS_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st_));
+        MPS_CUDA(cudaStreamSynchronize(st_));
+    }
+}
+
+template <int D>
+void Engine<D>::copy_to_device(void *dev, const void *host, size_t bytes)
+{
+    if (HostPipe::wanted(host, bytes)) pipe_.to_device(dev, host, bytes, st_);
+    else MPS_CUDA(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st_));
+}
+
+template <int D>
 void Engine<D>::upload_aos(const void *aos, int num)
 {
     if (num < 0 || num > cap_) throw CudaError("particle count exceeds capacity", MPS_ERR_INVALID);
     n_ = num;
     size_t bytes = (size_t)num * AosLayout<D>::size;
     aos_.reserve(bytes + 8);
-    MPS_CUDA(cudaMemcpyAsync(aos_.p, aos, bytes, cudaMemcpyHostToDevice, st_));
+    copy_to_device(aos_.p, aos, bytes);
     if (num) launch(k_unpack<D>, nblk(num, TPB), TPB, 0, st_, aos_.p, S(), num);
     if (num) launch(k_set_rest<D>, nblk(num, TPB), TPB, 0, st_, S(), num, cap_, rest_.p);
     MPS_CUDA(cudaGetLastError());
@@ -927,8 +949,7 @@ void Engine<D>::download_aos(void *aos, int num)
     aos_.reserve(bytes + 8);
     if (num) launch(k_pack<D>, nblk(num, TPB), TPB, 0, st_, aos_.p, S(), num);
     MPS_CUDA(cudaGetLastError());
-    MPS_CUDA(cudaMemcpyAsync(aos, aos_.p, bytes, cudaMemcpyDeviceToHost, st_));
-    MPS_CUDA(cudaStreamSynchronize(st_));
+    copy_to_host(aos, aos_.p, bytes);
 }
 
 template <int D>
@@ -938,9 +959,8 @@ void Engine<D>::upload_soa(const double *pos, const double *vel, const int *type
     n_ = num;
     soa_in_.reserve((size_t)2 * D * num + 2);
     int_in_.reserve((size_t)num + 1);
-    MPS_CUDA(cudaMemcpyAsync(soa_in_.p, pos, sizeof(double) * D * num, cudaMemcpyHostToDevice, st_));
-    MPS_CUDA(cudaMemcpyAsync(soa_in_.p + (size_t)D * num, vel, sizeof(double) * D * num,
-                             cudaMemcpyHostToDevice, st_));
+    copy_to_device(soa_in_.p, pos, sizeof(double) * D * num);
+    copy_to_device(soa_in_.p + (size_t)D * num, vel, sizeof(double) * D * num);
     MPS_CUDA(cudaMemcpyAsync(int_in_.p, type, sizeof(int) * num, cudaMemcpyHostToDevice, st_));
     if (num)
         launch(k_unpack_soa<D>, nblk(num, TPB), TPB, 0, st_, soa_in_.p, soa_in_.p + (size_t)D * num, int_in_.p, S(),
@@ -960,8 +980,7 @@ void Engine<D>::download_pressure(double *p, int num)
     if (num != n_) throw CudaError("download count differs from the uploaded count", MPS_ERR_INVALID);
     soa_in_.reserve((size_t)num + 2);
     if (num) launch(k_pressure_ref<D>, nblk(num, TPB), TPB, 0, st_, S(), num, soa_in_.p);
-    MPS_CUDA(cudaMemcpyAsync(p, soa_in_.p, sizeof(double) * num, cudaMemcpyDeviceToHost, st_));
-    MPS_CUDA(cudaStreamSynchronize(st_));
+    copy_to_host(p, soa_in_.p, sizeof(double) * num);
 }
 
 // ---- neighbour search -------------------------------------------------------
@@ -1169,17 +1188,21 @@ void Engine<D>::set_initial_params(double n0, double lambda, int n0_count)
 // ---- the step -------------------------------------------------------------------
 
 // The caller's list (reference layout: row i at nb[i * max_nb], count[i]
-// entries) to CSR on the device: one pitched copy of the used columns, a
-// scan of the counts and a compaction kernel.
+// entries) to CSR on the device: a scan of the counts, and the used entries
+// gathered on the way (by the host threads of a large pageable list, by a
+// kernel reading page-locked memory, else by one pitched copy of the used
+// columns and a compaction kernel).
 template <int D>
 void Engine<D>::upload_list(const int *nb, const int *cnt, int max_nb)
 {
     int n = n_;
     if (max_nb <= 0) throw CudaError("max_neighbors must be positive", MPS_ERR_INVALID);
     int mc = 0;
+    long long used = 0;
     for (int i = 0; i < n; i++) {
         if (cnt[i] < 0 || cnt[i] > max_nb) throw CudaError("bad neighbour count", MPS_ERR_INVALID);
         mc = std::max(mc, cnt[i]);
+        used += cnt[i];
     }
     lcnt_.reserve((size_t)n + 1);
     lptr_.reserve((size_t)n + 1);
@@ -1198,6 +1221,33 @@ void Engine<D>::upload_list(const int *nb, const int *cnt, int max_nb)
         lidx_.reserve((size_t)n * mc);
         launch(k_gather_host_list, nblk((long long)n * 32, TPB), TPB, 0, st_, (const int *)pa.devicePointer,
                max_nb, (const int *)lcnt_.p, (const int *)lptr_.p, n, lidx_.p, err_.p);
+    } else if (used < 0x7fffffffLL && (size_t)mc * sizeof(int) <= HostPipe::kChunk &&
+               HostPipe::wanted(nb, sizeof(int) * (size_t)used)) {
+        lidx_.reserve((size_t)used);
+        // chunks of whole rows: first row and first entry of each
+        constexpr long long room = HostPipe::kChunk / sizeof(int);
+        std::vector<int> row{0};
+        std::vector<long long> at{0};
+        long long pos = 0;
+        for (int i = 0; i < n; i++) {
+            if (pos + cnt[i] - at.back() > room) {
+                row.push_back(i);
+                at.push_back(pos);
+            }
+            pos += cnt[i];
+        }
+        row.push_back(n);
+        at.push_back(pos);
+        pipe_.chunks_to_device(row.size() - 1, st_, [&](size_t c, void *buf, void *&dst) {
+            int *o = (int *)buf;
+            for (int i = row[c]; i < row[c + 1]; i++) {
+                std::memcpy(o, nb + (size_t)i * max_nb, sizeof(int) * (size_t)cnt[i]);
+                o += cnt[i];
+            }
+            dst = lidx_.p + at[c];
+            return sizeof(int) * (size_t)(at[c + 1] - at[c]);
+        });
+        launch(k_check_list, nblk(used, TPB), TPB, 0, st_, (int)used, n, lidx_.p, err_.p);
     } else if (mc > 0 && n > 0) {
         lout_.reserve((size_t)n * mc);
         lidx_.reserve((size_t)n * mc);
@@ -2730,8 +2780,25 @@ void Engine<D>::get_neighbor_list(int *nb, int *cnt, int max_nb)
     lout_.reserve((size_t)n * mc);
     launch(k_build_list<D>, nblk(n, TPB), TPB, 0, st_, near(), (const int *)S().id, n, max_nb, mc, lout_.p,
            lcnt_.p, err_.p);
-    MPS_CUDA(cudaMemcpy2DAsync(nb, sizeof(int) * (size_t)max_nb, lout_.p, sizeof(int) * mc, sizeof(int) * mc, n,
-                               cudaMemcpyDeviceToHost, st_));
+    size_t row_bytes = sizeof(int) * (size_t)mc;
+    if (row_bytes <= HostPipe::kChunk && HostPipe::wanted(nb, row_bytes * (size_t)n)) {
+        size_t rows = HostPipe::kChunk / row_bytes, nc = ((size_t)n + rows - 1) / rows;
+        pipe_.chunks_to_host(
+            nc, st_,
+            [&](size_t c, const void *&src, size_t &bytes) {
+                src = lout_.p + c * rows * mc;
+                bytes = row_bytes * std::min(rows, (size_t)n - c * rows);
+            },
+            [&](size_t c, const void *buf, size_t bytes) {
+                const int *in = (const int *)buf;
+                size_t r0 = c * rows, m = bytes / row_bytes;
+                for (size_t i = 0; i < m; i++)
+                    std::memcpy(nb + (r0 + i) * (size_t)max_nb, in + i * mc, sizeof(int) * (size_t)hcnt[r0 + i]);
+            });
+    } else {
+        MPS_CUDA(cudaMemcpy2DAsync(nb, sizeof(int) * (size_t)max_nb, lout_.p, row_bytes, row_bytes, n,
+                                   cudaMemcpyDeviceToHost, st_));
+    }
     check_err();
 }
 

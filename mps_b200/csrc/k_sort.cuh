@@ -296,6 +296,18 @@ __global__ void k_build_list(NbrSource<D> src, const int *__restrict__ id, int n
     out_cnt[row] = cnt;
 }
 
+// Entries of an uploaded list outside the particles are reported.
+__global__ void k_check_list(int used, int n, int *__restrict__ idx, unsigned *err)
+{
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= used) return;
+    int j = idx[k];
+    if (j < 0 || j >= n) {
+        atomicOr(err, ERR_LIST_MISMATCH);
+        idx[k] = 0;
+    }
+}
+
 // Rows of a pitched host list (already on the device) into CSR.
 __global__ void k_compact_list(const int *__restrict__ rows, int pitch, const int *__restrict__ cnt,
                                const int *__restrict__ ptr, int n, int *__restrict__ idx, unsigned *err)
