@@ -410,7 +410,7 @@ private:
     DevArray<int> mlflag_, mlpos_, mlmap_, mlact_, mlcell_, mlncell_, mlcnode_, mlunder_, mlabove_, ufpar_, ufkeep_, mlscan_;
     DevArray<unsigned char> bounded_, mlpar_;
     DevArray<float> mlfrac_;
-    DevArray<double> mlcm_, mlA_, mlC_, mldinv_, mlb_, mlx_, mly_, mlbd_, mlM_[2], mlMC_, mlcsum_, jdinv_;
+    DevArray<double> mlcm_, mlB_, mlA_, mlC_, mldinv_, mlb_, mlx_, mly_, mlbd_, mlM_[2], mlMC_, mlcsum_, jdinv_;
     const double *mlM_last_ = nullptr;     // the dense V-cycle of the current solve
     void ml_levels();
     void ml_nodes(int nact);
@@ -1464,10 +1464,13 @@ void Engine<D>::ml_build(int n_eq)
            ufpar_.p, (const int *)ufkeep_.p, mlfrac_.p, jdinv_.p);
     launch(k_ml_node_cells<D>, nblk(na1, TPB), TPB, 0, st_, na1, (const int *)mlact_.p, ml_.g[0], g_,
            (const int *)mlcell_.p, mlncell_.p);
-    launch(k_ml_cellmat<D>, nact, D == 3 ? 256 : 128, 0, st_, (const int *)acells_.p, (const int2 *)adesc_.p, g_, rp,
-           (const unsigned short *)runs_.p, ci, A, (const float *)mlfrac_.p, cap_, mlcm_.p);
-    launch(k_ml_a1<D>, na1, L::STP, 0, st_, na1, (const int *)mlncell_.p, (const double *)mlcm_.p,
-           ml_add_, mlA_.p, mldinv_.p);
+    launch(k_ml_cellmat<D>, nblk(nact, ML_CW), 32 * ML_CW, 0, st_, nact, (const int *)acells_.p,
+           (const int2 *)adesc_.p, g_, rp, dp, (const unsigned short *)runs_.p, ci, A, (const float *)mlfrac_.p, cap_,
+           mlcm_.p);
+    mlB_.reserve((size_t)na1 * L::STP);
+    launch(k_ml_b1<D>, na1, L::STP, 0, st_, na1, (const int *)mlncell_.p, (const double *)mlcm_.p, mlB_.p);
+    launch(k_ml_a1<D>, na1, L::STP, 0, st_, mlc_.g[0], (const int *)mlact_.p, (const int *)mlmap_.p,
+           (const double *)mlB_.p, ml_add_, mlA_.p, mldinv_.p);
     for (int l = 0; l + 1 < nl; l++) {
         int lof = mlc_.lo[l], loc = mlc_.lo[l + 1], nc = mlc_.lo[l + 2] - loc;
         launch(k_ml_galerkin<D>, nc, L::STP, 0, st_, mlc_.g[l], mlc_.g[l + 1], lof, loc, (const int *)mlact_.p,

@@ -365,92 +365,146 @@ __device__ __forceinline__ void ml_weights(const float *__restrict__ frac, int s
 
 // ---- Galerkin operators -------------------------------------------------------------------
 
-// Part of one cell's rows in A_1 = P^T A P, a CTA per active cell, ML_RB rows
-// at a time: a thread per (row, neighbour cell) sums the row's entries there
-// weighted onto that cell's corners, the corner sums are added up on the 4^D
-// nodes of the cell and its neighbours, and the rows of that product are
-// spread over the cell's own corners: out[cell][own corner][node].
-// (A thread per neighbour cell and corner, every entry read by 2^D threads,
-// took 14.7 ms at 2.2 M rows.)
-constexpr int ML_RB = 8;
+// Part of one cell's rows in B = P^T (L + D / 2) P, with A = L + D + L^T, a
+// warp per active cell and a lane per row (32 rows at a time): a lane walks
+// its row's run in each neighbour cell in turn, sums the entries times the
+// eight monomials of the column's position in its cell (half the arithmetic
+// of eight weights), turns them into the sums on that cell's corners and adds
+// those to its own row of nodes of the cell and its neighbours in shared
+// memory.  The rows of nodes are then spread over the cell's own corners:
+// out[cell][own corner][node].  Runs of one cell's rows are of similar length,
+// so the lanes stay together; what bounds it is the latency of the entries,
+// which are therefore read a batch ahead, across the ends of runs.
+constexpr int ML_CW = 2;   // cells per block
 
 template <int D>
-__global__ void __launch_bounds__(D == 3 ? 256 : 128)
-k_ml_cellmat(const int *__restrict__ acells, const int2 *__restrict__ desc, Grid<D> cg,
-             const int *__restrict__ row_ptr, const unsigned short *__restrict__ runs, const int *__restrict__ col,
-             const double *__restrict__ A, const float *__restrict__ frac, int stride, double *__restrict__ out)
+__global__ void __launch_bounds__(32 * ML_CW)
+k_ml_cellmat(int nact, const int *__restrict__ acells, const int2 *__restrict__ desc, Grid<D> cg,
+             const int *__restrict__ row_ptr, const int *__restrict__ diagpos,
+             const unsigned short *__restrict__ runs, const int *__restrict__ col, const double *__restrict__ A,
+             const float *__restrict__ frac, int stride, double *__restrict__ out)
 {
     using L = MlDim<D>;
-    constexpr int BLOCK = D == 3 ? 256 : 128;
-    constexpr int ITEMS = (L::NC * L::W4 + BLOCK - 1) / BLOCK;
-    __shared__ double sp[ML_RB][L::CELLS][L::NC];
-    __shared__ double sn[ML_RB][L::W4];
-    __shared__ double sw[ML_RB][L::NC];
-    int kk = blockIdx.x, t = threadIdx.x;
+    constexpr int NC = L::NC, LN = 33, U = 4;
+    constexpr int NPL = (L::W4 + 31) / 32;   // nodes of a lane
+    __shared__ double snode[ML_CW][L::W4 * LN];
+    __shared__ double sw[ML_CW][32 * NC];
+    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int kk = blockIdx.x * ML_CW + w;
+    if (kk >= nact) return;   // whole warps; no block barrier below
+    double *node = snode[w], *wt = sw[w];
     int2 dd = desc[kk];
     int par = cell_parity<D>(cg, acells[kk]);
-    double acc[ITEMS];
+    int qc = visit_rank<D>(par, L::CELLS / 2);   // the own cell: the last with lower entries
+    double acc[NPL][NC];
 #pragma unroll
-    for (int j = 0; j < ITEMS; j++) acc[j] = 0.0;
-    for (int i0 = 0; i0 < dd.y; i0 += ML_RB) {
-        int nr = min(ML_RB, dd.y - i0);
-        for (int w = t; w < nr * L::CELLS; w += BLOCK) {
-            int i = w / L::CELLS, q = w % L::CELLS;
-            int r = dd.x + i0 + i;
-            int base = row_ptr[r];
-            int e = base + runs[(size_t)q * stride + r];
-            int end = q + 1 < L::CELLS ? base + runs[(size_t)(q + 1) * stride + r] : row_ptr[r + 1];
-            double s[L::NC];
+    for (int j = 0; j < NPL; j++)
 #pragma unroll
-            for (int k = 0; k < L::NC; k++) s[k] = 0.0;
-            for (; e < end; e++) {
-                double a = __ldg(&A[e]);
-                double wt[L::NC];
-                ml_weights<D>(frac, stride, __ldg(&col[e]), wt);
+        for (int k = 0; k < NC; k++) acc[j][k] = 0.0;
+    for (int i0 = 0; i0 < dd.y; i0 += 32) {
+        int nr = min(32, dd.y - i0);
+        bool in = lane < nr;
+        int r = dd.x + i0 + (in ? lane : 0);
+        int base = row_ptr[r], diag = diagpos[r];
+        int last = in ? diag + 1 : base;
+        int end = qc > 0 ? min(last, base + runs[(size_t)stride + r]) : last;
+        int e = base;
+        int cn[U];
+        double an[U];
 #pragma unroll
-                for (int k = 0; k < L::NC; k++) s[k] = fma(a, wt[k], s[k]);
-            }
-            int nb = visit_cell<D>(par, q);
-#pragma unroll
-            for (int k = 0; k < L::NC; k++) sp[i][nb][k] = s[k];
+        for (int u = 0; u < U; u++) {
+            cn[u] = e + u < last ? __ldg(&col[e + u]) : r;
+            an[u] = e + u < last ? __ldg(&A[e + u]) : 0.0;
         }
-        if (t < nr) {
-            double w[L::NC];
-            ml_weights<D>(frac, stride, dd.x + i0 + t, w);
+#pragma unroll 8
+        for (int nd = 0; nd < L::W4; nd++) node[nd * LN + lane] = 0.0;
+        double own[NC];
+        ml_weights<D>(frac, stride, r, own);
 #pragma unroll
-            for (int j = 0; j < L::NC; j++) sw[t][j] = w[j];
-        }
-        __syncthreads();
-        // the (cell, corner) pairs that name one node, in a fixed order
-        for (int w = t; w < nr * L::W4; w += BLOCK) {
-            int i = w / L::W4, nd = w % L::W4;
-            int nx = nd % 4, ny = (nd / 4) % 4, nz = nd / 16;
-            double s = 0.0;
+        for (int k = 0; k < NC; k++) wt[lane * NC + k] = own[k];
+        for (int q = 0; q <= qc; q++) {
+            int end1 = q + 1 < qc ? min(last, base + runs[(size_t)(q + 2) * stride + r]) : last;   // the next run's end
+            double s[NC];
 #pragma unroll
-            for (int kz = 0; kz < (D == 3 ? 2 : 1); kz++)
+            for (int k = 0; k < NC; k++) s[k] = 0.0;
+            bool any = false;
+            while (__any_sync(0xffffffffu, e < end)) {
+                any = true;
+                double a[U];
+                float f[U][D];
+                int ne = min(e + U, end);
 #pragma unroll
-                for (int ky = 0; ky < 2; ky++)
+                for (int u = 0; u < U; u++) {
+                    a[u] = e + u < end ? (e + u == diag ? 0.5 * an[u] : an[u]) : 0.0;
 #pragma unroll
-                    for (int kx = 0; kx < 2; kx++) {
-                        int qx = nx - kx, qy = ny - ky, qz = D == 3 ? nz - kz : 0;
-                        if (qx < 0 || qx > 2 || qy < 0 || qy > 2 || qz < 0 || qz > 2) continue;
-                        s += sp[i][qx + 3 * qy + 9 * qz][kx + 2 * ky + 4 * kz];
+                    for (int d = 0; d < D; d++) f[u][d] = __ldg(&frac[(size_t)d * stride + cn[u]]);
+                }
+                if (ne != e) {   // a lane at the end of its run keeps what it has read ahead
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        cn[u] = ne + u < last ? __ldg(&col[ne + u]) : r;
+                        an[u] = ne + u < last ? __ldg(&A[ne + u]) : 0.0;
                     }
-            sn[i][nd] = s;
-        }
-        __syncthreads();
+                }
+                e = ne;
 #pragma unroll
-        for (int j = 0; j < ITEMS; j++) {
-            int w = t + j * BLOCK;
-            if (w < L::NC * L::W4)
-                for (int i = 0; i < nr; i++) acc[j] = fma(sw[i][w / L::W4], sn[i][w % L::W4], acc[j]);
+                for (int u = 0; u < U; u++) {
+                    double x = (double)f[u][0], y = (double)f[u][1];
+                    double v = f[u][0] < 0.0f ? 0.0 : a[u];
+                    double vx = v * x;
+                    s[0] += v;
+                    s[1] += vx;
+                    s[2] = fma(v, y, s[2]);
+                    s[3] = fma(vx, y, s[3]);
+                    if (D == 3) {
+                        double z = (double)f[u][D - 1];
+                        double vz = v * z, vxz = vx * z;
+                        s[4 & (NC - 1)] += vz;
+                        s[5 & (NC - 1)] += vxz;
+                        s[6 & (NC - 1)] = fma(vz, y, s[6 & (NC - 1)]);
+                        s[7 & (NC - 1)] = fma(vxz, y, s[7 & (NC - 1)]);
+                    }
+                }
+            }
+            end = end1;
+            if (!any) continue;
+            // monomials to corners: along each axis, (1 - f) and f
+#pragma unroll
+            for (int d = 0; d < D; d++)
+#pragma unroll
+                for (int k = 0; k < NC; k++)
+                    if (!(k >> d & 1)) s[k] -= s[k | (1 << d)];
+            int nb = visit_cell<D>(par, q);
+            int n0 = nb % 3 + 4 * ((nb / 3) % 3) + (D == 3 ? 16 * (nb / 9) : 0);
+#pragma unroll
+            for (int k = 0; k < NC; k++) {
+                int nd = n0 + (k & 1) + 4 * ((k >> 1) & 1) + 16 * (k >> 2);
+                node[nd * LN + lane] += s[k];
+            }
         }
-        __syncthreads();
+        __syncwarp();
+        for (int i = 0; i < nr; i++) {
+            double wi[NC];
+#pragma unroll
+            for (int k = 0; k < NC; k++) wi[k] = wt[i * NC + k];
+#pragma unroll
+            for (int j = 0; j < NPL; j++) {
+                int nd = lane + 32 * j;
+                if (nd < L::W4) {
+                    double v = node[nd * LN + i];
+#pragma unroll
+                    for (int k = 0; k < NC; k++) acc[j][k] = fma(wi[k], v, acc[j][k]);
+                }
+            }
+        }
+        __syncwarp();
     }
 #pragma unroll
-    for (int j = 0; j < ITEMS; j++) {
-        int w = t + j * BLOCK;
-        if (w < L::NC * L::W4) out[(size_t)kk * (L::NC * L::W4) + w] = acc[j];
+    for (int j = 0; j < NPL; j++) {
+        int nd = lane + 32 * j;
+        if (nd < L::W4)
+#pragma unroll
+            for (int k = 0; k < NC; k++) out[(size_t)kk * (NC * L::W4) + k * L::W4 + nd] = acc[j][k];
     }
 }
 
@@ -476,14 +530,12 @@ __device__ __forceinline__ void ml_row_factor(double v, int k, double *sh, bool 
     }
 }
 
-// A_1 rows from the cells' parts: a block per node, a thread per stencil entry.
+// B's rows from the cells' parts: a block per node, a thread per stencil entry.
 template <int D>
 __global__ void __launch_bounds__(MlDim<D>::STP)
-k_ml_a1(int na, const int *__restrict__ ncell, const double *__restrict__ cellmat, bool additive,
-        double *__restrict__ Ac, double *__restrict__ dinv)
+k_ml_b1(int na, const int *__restrict__ ncell, const double *__restrict__ cellmat, double *__restrict__ B)
 {
     using L = MlDim<D>;
-    __shared__ double sh[4];
     int t = blockIdx.x, k = threadIdx.x;
     double s = 0.0;
     if (k < L::ST) {
@@ -503,6 +555,24 @@ k_ml_a1(int na, const int *__restrict__ ncell, const double *__restrict__ cellma
             }
             if (in) s += cellmat[(size_t)c * (L::NC * L::W4) + j * L::W4 + nd];
         }
+    }
+    B[(size_t)t * L::STP + k] = s;
+}
+
+// A_1 = B + B^T and its smoother factor: entry k of node t is also entry
+// ST - 1 - k of the node at that offset.
+template <int D>
+__global__ void __launch_bounds__(MlDim<D>::STP)
+k_ml_a1(MlGrid g, const int *__restrict__ act, const int *__restrict__ amap, const double *__restrict__ B,
+        bool additive, double *__restrict__ Ac, double *__restrict__ dinv)
+{
+    using L = MlDim<D>;
+    __shared__ double sh[4];
+    int t = blockIdx.x, k = threadIdx.x;
+    double s = 0.0;
+    if (k < L::ST) {
+        int o = amap[act[t] + ml_offset<D>(g, k)];
+        s = B[(size_t)t * L::STP + k] + (o >= 0 ? B[(size_t)o * L::STP + L::ST - 1 - k] : 0.0);
     }
     Ac[(size_t)t * L::STP + k] = s;
     ml_row_factor<D>(s, k, sh, additive, &dinv[t]);

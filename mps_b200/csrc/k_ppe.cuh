@@ -1576,6 +1576,7 @@ __global__ void k_refine_residual(int n_eq, const int *__restrict__ row_ptr, con
         double s = 0.0, sa = 0.0;
         if (i < n_eq) {
             int q1 = __ldg(&row_ptr[i + 1]);
+#pragma unroll 4
             for (int q = __ldg(&row_ptr[i]) + lane; q < q1; q += LPR) {
                 double t = __ldg(&A[q]) * x[__ldg(&col[q])];
                 s += t;
@@ -1631,6 +1632,7 @@ __global__ void k_true_residual(int n_eq, const int *__restrict__ row_ptr, const
         double s = 0.0, sa = 0.0;
         if (i < n_eq) {
             int q1 = __ldg(&row_ptr[i + 1]);
+#pragma unroll 4
             for (int q = __ldg(&row_ptr[i]) + lane; q < q1; q += LPR) {
                 double t = __ldg(&A[q]) * x[__ldg(&col[q])];
                 s += t;
