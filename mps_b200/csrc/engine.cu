@@ -272,7 +272,7 @@ private:
     bool structure_ = false;   // cell structure valid for S_[cur_]
 
     // ---- sort
-    DevArray<int> kcell_, count_, start_, cursor_, excl_, exoff_, tmp_, perm_, where_, scanws_;
+    DevArray<int> kcell_, count_, start_, excl_, exoff_, tmp_, perm_, where_, scanws_;
     DevArray<long long> scanws64_;
 
     // ---- block colouring
@@ -475,6 +475,7 @@ private:
     DevArray<int> nbr_idx_, nbr_cnt_;
     DevArray<float4> keyf_;
     bool nbr_valid_ = false;
+    bool keyf_valid_ = false;   // keyf_ belongs to the current structure
     int nbr_pitch_ = 0;
     // bytes the lists may take; beyond, operators walk the cells
     static constexpr double kNbrBytes = 24.0e9;
@@ -719,15 +720,13 @@ void Engine<D>::build_grid()
     if (total <= 0 || total > (1LL << 30)) throw CudaError("cell grid too large", MPS_ERR_INVALID);
     g_.total = (int)total;
     g_.cs_inv = 1.0 / re;
-    count_.reserve(total + 1);
-    cursor_.reserve(total + 1);
+    count_.reserve(2 * (total + 1));   // and the scatter's cursors
     start_.reserve(total + 2);
     ucount_.reserve(total);
     ucol_.reserve(total);
     rs_.reserve(total + 1);
     cell_row0_.reserve(total);
-    size_t ws = std::max(scan_workspace((int)std::max<long long>(total + 1, cap_ + 1)), (size_t)64);
-    scanws_.reserve(ws);
+    scanws_.reserve(scan_workspace((int)total + 1) + scan_workspace(std::max((int)total, cap_) + 1) + 64);   // a pair's
     g_.start = start_.p;
 
     // cells sorted by (colour, linear index)
@@ -991,23 +990,24 @@ void Engine<D>::sort()
     int n = n_, total = g_.total;
     State<D> &src = S_[cur_];
     State<D> &dst = S_[cur_ ^ 1];
-    MPS_CUDA(cudaMemsetAsync(count_.p, 0, sizeof(int) * (total + 1), st_));
-    MPS_CUDA(cudaMemsetAsync(cursor_.p, 0, sizeof(int) * (total + 1), st_));
+    MPS_CUDA(cudaMemsetAsync(count_.p, 0, 2 * sizeof(int) * ((size_t)total + 1), st_));
+    int *cursor = count_.p + total + 1;
+    keyf_.reserve((size_t)cap_);
     if (n) launch(k_bin<D>, nblk(n, TPB), TPB, 0, st_, src, g_, n, kcell_.p, count_.p, excl_.p);
-    scan_exclusive<int>(count_.p, start_.p, total, scanws_.p, st_);
-    scan_exclusive<int>(excl_.p, exoff_.p, n, scanws_.p, st_);
+    scan_exclusive2<int>(count_.p, start_.p, total, excl_.p, exoff_.p, n, scanws_.p, st_);
     if (n) {
-        launch(k_scatter, nblk(n, TPB), TPB, 0, st_, n, total, kcell_.p, start_.p, cursor_.p, exoff_.p, tmp_.p,
+        launch(k_scatter, nblk(n, TPB), TPB, 0, st_, n, total, kcell_.p, start_.p, cursor, exoff_.p, tmp_.p,
                                                  perm_.p);
         // ranks for the binned prefix [0, start[total])
         launch(k_rank, nblk(n, TPB), TPB, 0, st_, start_.p + total, tmp_.p, kcell_.p, start_.p, src.id, perm_.p);
-        launch(k_gather<D>, nblk(n, TPB), TPB, 0, st_, dst, src, perm_.p, kcell_.p, n, where_.p);
+        launch(k_gather<D>, nblk(n, TPB), TPB, 0, st_, dst, src, perm_.p, kcell_.p, n, where_.p, g_, keyf_.p);
     }
     MPS_CUDA(cudaGetLastError());
     cur_ ^= 1;
     g_.start = start_.p;
     structure_ = true;
     nbr_valid_ = false;
+    keyf_valid_ = n > 0;
     ppe_valid_ = false;
 }
 
@@ -1043,7 +1043,8 @@ NbrSource<D> Engine<D>::near()
         int ext = 1;
         for (int d = 0; d < D; d++) ext = std::max(ext, g_.dims[d]);
         float band = ext > 1000000 ? 1.0e30f : 8.0f * 1.1920929e-7f * (float)ext + 4.0e-6f;
-        launch(k_key_cells<D>, nblk(n, TPB), TPB, 0, st_, S(), g_, n, keyf_.p);
+        if (!keyf_valid_) launch(k_key_cells<D>, nblk(n, TPB), TPB, 0, st_, S(), g_, n, keyf_.p);
+        keyf_valid_ = true;
         if (n < nbr_lanes_below_)
             launch(k_nbr_list_lanes<D>, nblk((long long)n * NBR_LANES, 128), 128, 0, st_, cells(), n,
                    (const float4 *)keyf_.p, band, nbr_pitch_, nbr_idx_.p, nbr_cnt_.p);
@@ -1431,9 +1432,10 @@ void Engine<D>::ml_build(int n_eq)
     ml_ld_ = 0;
     while (ml_ld_ + 1 < nl && mlc_.lo[ml_ld_ + 1] - mlc_.lo[ml_ld_] > ml_dense_) ml_ld_++;
     ml_add_ = ml_add_ && ml_ld_ > 0;
+    // zero around the nodes in use (the dense grid alone reads no neighbours)
     for (auto *v : {&mlb_, &mlx_, &mly_}) {
         v->reserve((size_t)ml_total_);
-        MPS_CUDA(cudaMemsetAsync(v->p, 0, sizeof(double) * (size_t)ml_total_, st_));
+        if (ml_ld_ > 0) MPS_CUDA(cudaMemsetAsync(v->p, 0, sizeof(double) * (size_t)ml_total_, st_));
     }
     mlncell_.reserve((size_t)L::NC * na1);
     mlcm_.reserve((size_t)nact * L::NC * L::W4);
@@ -1849,13 +1851,11 @@ void Engine<D>::ppe(bool clamp)
     int n = n_, total = g_.total;
     int ncol = 1 << D;
     State<D> &s = S();
-    launch(k_cell_unknowns<D>, nblk(total, TPB), TPB, 0, st_, s, start_.p, total, ucount_.p);
-    launch(k_color_gather, nblk(total, TPB), TPB, 0, st_, ccells_.p, ucount_.p, total, ucol_.p);
-    scan_exclusive<int>(ucol_.p, rs_.p, total, scanws_.p, st_);
+    launch(k_cell_unknowns<D>, nblk(total, TPB), TPB, 0, st_, s, (const int *)start_.p, (const int *)ccells_.p, total,
+           ucount_.p, ucol_.p, aflag_.p);
+    scan_exclusive2<int>(ucol_.p, rs_.p, total, aflag_.p, apos_.p, total, scanws_.p, st_);
     launch(k_assign_rows<D>, nblk(total, TPB), TPB, 0, st_, s, (const int *)start_.p, (const int *)ccells_.p,
            (const int *)rs_.p, total, cell_row0_.p, row_of_.p, part_of_row_.p);
-    launch(k_active_flag, nblk(total, TPB), TPB, 0, st_, (const int *)ucol_.p, total, aflag_.p);
-    scan_exclusive<int>(aflag_.p, apos_.p, total, scanws_.p, st_);
     launch(k_active_scatter, nblk(total, TPB), TPB, 0, st_, (const int *)ccells_.p, (const int *)ucol_.p,
            (const int *)apos_.p, total, acells_.p);
     launch(k_ppe_sizes, 1, 1, 0, st_, (const int *)rs_.p, (const int *)apos_.p, (const int *)start_.p, total,
@@ -2527,7 +2527,7 @@ void Engine<D>::state_load(const void *src)
     tstep_ = h.tstep;
     g_.start = start_.p;
     structure_ = true;
-    nbr_valid_ = false;
+    nbr_valid_ = keyf_valid_ = false;
     ppe_valid_ = false;
 }
 

@@ -81,30 +81,23 @@ __device__ __forceinline__ bool is_unknown(int type, int surf)
 
 // ---- numbering -------------------------------------------------------------
 
+// Unknowns of every cell, taken in colour order: by cell, by position in that
+// order, and whether there are any.
 template <int D>
-__global__ void k_cell_unknowns(State<D> s, const int *__restrict__ start, int total, int *__restrict__ ucount)
+__global__ void k_cell_unknowns(State<D> s, const int *__restrict__ start, const int *__restrict__ ccells, int total,
+                                int *__restrict__ ucount, int *__restrict__ ucol, int *__restrict__ flag)
 {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= total) return;
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= total) return;
+    int c = ccells[k];
     int u = 0;
     for (int t = start[c]; t < start[c + 1]; t++) u += is_unknown(s.type[t], s.surf[t]);
     ucount[c] = u;
+    ucol[k] = u;
+    flag[k] = u > 0;
 }
 
-__global__ void k_color_gather(const int *__restrict__ ccells, const int *__restrict__ ucount, int total,
-                               int *__restrict__ ucol)
-{
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < total) ucol[k] = ucount[ccells[k]];
-}
-
-// Cells holding unknowns, in colour order: flag, scan, scatter.
-__global__ void k_active_flag(const int *__restrict__ ucol, int total, int *__restrict__ flag)
-{
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < total) flag[k] = ucol[k] > 0;
-}
-
+// Cells holding unknowns, in colour order.
 __global__ void k_active_scatter(const int *__restrict__ ccells, const int *__restrict__ ucol,
                                  const int *__restrict__ apos, int total, int *__restrict__ acells)
 {

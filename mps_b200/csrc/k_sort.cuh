@@ -67,14 +67,17 @@ __global__ void k_rank(const int *__restrict__ nbinned, const int *__restrict__ 
 
 template <int D>
 __global__ void k_gather(State<D> dst, State<D> src, const int *__restrict__ perm,
-                         const int *__restrict__ kcell, int n, int *__restrict__ where)
+                         const int *__restrict__ kcell, int n, int *__restrict__ where, Grid<D> g,
+                         float4 *__restrict__ kf)
 {
     int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n) return;
     int i = perm[q];
+    float f[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // the key in cell units, as k_key_cells
 #pragma unroll
     for (int d = 0; d < D; d++) {
         double x = src.pos[d][i];
+        f[d] = (float)((x - g.origin[d]) * g.cs_inv);
         dst.pos[d][q] = x;
         dst.key[d][q] = x;
         dst.vel[d][q] = src.vel[d][i];
@@ -89,6 +92,7 @@ __global__ void k_gather(State<D> dst, State<D> src, const int *__restrict__ per
     dst.id[q] = id;
     dst.cell[q] = kcell[i];
     where[id] = q;
+    kf[q] = make_float4(f[0], f[1], f[2], f[3]);
 }
 
 // Reorder to reference order (engine index == reference index).
