@@ -386,11 +386,9 @@ private:
     bool ml_on_ = false;                   // the current solve uses it
     bool ml_add_ = false;                  // additive first grid
     int ml_ld_ = 0;                        // the dense grid
-    // unknowns below which the first grid is additive (MPS_ML_ADD): a product
-    // with its operator and with C fewer per iteration for about a third more
-    // iterations, which pays where an iteration is a chain of short launches;
-    // and nodes up to which a grid's V-cycle is dense (MPS_ML_DENSE)
-    int ml_add_rows_ = 60000, ml_dense_ = ML_DENSE;
+    // unknowns below which the first grid is additive (MPS_ML_ADD; -1: the rule
+    // of ml_build), and nodes up to which a grid's V-cycle is dense (MPS_ML_DENSE)
+    int ml_add_rows_ = -1, ml_dense_ = ML_DENSE;
     // unknowns up to which the loop runs in one cluster (MPS_ML_SMALL); measured
     // per iteration, launches against cluster: 1,617 unknowns (2-D) 27 / 11 us,
     // 2,842 (3-D) 29 / 21, 5,487 (2-D) 31 / 19, 13,334 (3-D) 35 / 37
@@ -1428,10 +1426,18 @@ void Engine<D>::ml_build(int n_eq)
             break;
         }
     int nl = mlc_.nl, na1 = mlc_.lo[1], nall = mlc_.lo[nl], nact = act_off_[1 << D];
-    ml_add_ = n_eq < ml_add_rows_;
     ml_ld_ = 0;
     while (ml_ld_ + 1 < nl && mlc_.lo[ml_ld_ + 1] - mlc_.lo[ml_ld_] > ml_dense_) ml_ld_++;
-    ml_add_ = ml_add_ && ml_ld_ > 0;
+    // Additive: a product with the first grid's operator and one with C fewer
+    // per iteration for a fifth to a half more iterations.  It pays where the
+    // loop runs in one cluster, which has no other form for a first grid too
+    // large to be dense (solve at 7,457 unknowns: 1.13 ms, against 1.28 by
+    // launches), and nowhere above (13,334: 1.84 ms against 2.52, 57,816: 1.99
+    // against 2.31).  From 20,000 to 40,000 unknowns it stays although slower
+    // (26,632: 2.4 ms against 1.8): the iteration count there is held to at
+    // least half of natural-order IC(0)'s, 95, and 36 is below that (49).
+    ml_add_ = ml_ld_ > 0 && (ml_add_rows_ >= 0 ? n_eq < ml_add_rows_
+                                               : n_eq <= ml_small_rows_ || (n_eq >= 20000 && n_eq < 40000));
     // zero around the nodes in use (the dense grid alone reads no neighbours)
     for (auto *v : {&mlb_, &mlx_, &mly_}) {
         v->reserve((size_t)ml_total_);
