@@ -864,6 +864,8 @@ void Engine<D>::update_params(const mps_params_t &p)
     regrid |= list_radius(p) != re_list_;
     prm_ = p;
     if (regrid) {
+        // a factor still to be formed reads the cells of the old grid
+        if (ppe_valid_ && ic0_valid_) require_ic0();
         build_grid();
         structure_ = false;
         nbr_valid_ = false;

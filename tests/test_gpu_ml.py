@@ -98,3 +98,31 @@ def test_multilevel_reruns_are_bit_identical(monkeypatch):
         assert ma["ppe_iterations"] == mb["ppe_iterations"]
         for f in ("pressure", "pos", "vel"):
             assert np.array_equal(a[f], b[f]), f
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_ic0_survives_a_larger_grid(dim):
+    """The IC(0) factor is formed on request; a domain enlarged in between
+    (the grid's arrays are allocated anew) leaves it as it was."""
+    _cuda()
+    from mps_b200 import _lib
+    from mps_b200.session import start
+    wl = CASES["small3d" if dim == 3 else "dam2d"]()
+    got = []
+    for grow in (False, True):
+        hp = T.HostParticles(dim, wl.pos, wl.vel, wl.types)
+        s = start(wl.config(), dim, hp)
+        try:
+            s.step(1)
+            if grow:
+                for d in range(dim):
+                    s.params.domain_max[d] *= 4.0
+                s._check(s.lib.mps_update_params(s.h, _lib.C.byref(s.params)))
+            got.append((s.ic0(), s.cell_blocks()))
+        finally:
+            s.close()
+    (f0, c0), (f1, c1) = got
+    for k in f0:
+        assert np.array_equal(f0[k], f1[k]), k
+    for a, b in zip(c0, c1):
+        assert np.array_equal(a, b)
