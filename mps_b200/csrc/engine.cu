@@ -271,6 +271,10 @@ private:
     int cur_ = 0;
     bool structure_ = false;   // cell structure valid for S_[cur_]
 
+    // storage of the arrays sized by the capacity, by the grid, and by a solve's
+    // grids (the last for the loop in one cluster)
+    DevGroup state_group_, grid_group_, ml_group_, ml_small_group_;
+
     // ---- sort
     DevArray<int> kcell_, count_, start_, excl_, exoff_, tmp_, perm_, where_, scanws_;
     DevArray<long long> scanws64_;
@@ -658,9 +662,25 @@ template <int D>
 void Engine<D>::alloc_state()
 {
     size_t nd = (size_t)(4 * D + 2), ni = 5;
+    state_group_.reserve([&](auto add) {
+        size_t cap = cap_;
+        for (int b = 0; b < 2; b++) {
+            add(dbuf_[b], nd * cap);
+            add(ibuf_[b], ni * cap);
+        }
+        for (auto *v : {&kcell_, &excl_, &tmp_, &perm_, &where_, &row_of_, &part_of_row_, &diagpos_, &nbr_cnt_,
+                        &ufpar_, &ufkeep_})
+            add(*v, cap);
+        for (auto *v : {&exoff_, &rcount_, &row_ptr_}) add(*v, cap + 1);
+        for (auto *v : {&vafter_, &rest_}) add(*v, D * cap);
+        for (auto *v : {&pmin_, &b_, &x_, &r_, &z_, &p_, &Ap_, &y_, &part_, &p2_, &dinv_, &jdinv_}) add(*v, cap);
+        add(diagoff_, cap);
+        add(runs_, (D == 3 ? 27 : 9) * cap);
+        add(keyf_, cap);
+        add(mlfrac_, D * cap);
+        add(bounded_, cap);
+    });
     for (int b = 0; b < 2; b++) {
-        dbuf_[b].reserve(nd * cap_);
-        ibuf_[b].reserve(ni * cap_);
         double *dp = dbuf_[b].p;
         int *ip = ibuf_[b].p;
         State<D> &s = S_[b];
@@ -678,27 +698,6 @@ void Engine<D>::alloc_state()
         s.id = ip + 3 * (size_t)cap_;
         s.cell = ip + 4 * (size_t)cap_;
     }
-    kcell_.reserve(cap_);
-    excl_.reserve(cap_);
-    exoff_.reserve(cap_ + 1);
-    tmp_.reserve(cap_);
-    perm_.reserve(cap_);
-    where_.reserve(cap_);
-    vafter_.reserve((size_t)D * cap_);
-    pmin_.reserve(cap_);
-    rest_.reserve((size_t)D * cap_);
-    row_of_.reserve(cap_);
-    part_of_row_.reserve(cap_);
-    rcount_.reserve(cap_ + 1);
-    row_ptr_.reserve(cap_ + 1);
-    diagpos_.reserve(cap_);
-    diagoff_.reserve(cap_);
-    runs_.reserve((size_t)(D == 3 ? 27 : 9) * cap_);
-    inpos_.reserve(cap_);
-    outpos_.reserve(cap_);
-    for (auto *v : {&pk_len_lo_, &pk_len_up_, &pk_off_lo_, &pk_off_up_}) v->reserve((size_t)cap_ + 1);
-    dinv_.reserve(cap_);
-    for (auto *v : {&b_, &x_, &r_, &z_, &p_, &Ap_, &y_, &part_, &p2_}) v->reserve(cap_);
 }
 
 // cell_list_create (neighbor_search.c:92-122) with cell size = list radius.
@@ -718,13 +717,19 @@ void Engine<D>::build_grid()
     if (total <= 0 || total > (1LL << 30)) throw CudaError("cell grid too large", MPS_ERR_INVALID);
     g_.total = (int)total;
     g_.cs_inv = 1.0 / re;
-    count_.reserve(2 * (total + 1));   // and the scatter's cursors
-    start_.reserve(total + 2);
-    ucount_.reserve(total);
-    ucol_.reserve(total);
-    rs_.reserve(total + 1);
-    cell_row0_.reserve(total);
-    scanws_.reserve(scan_workspace((int)total + 1) + scan_workspace(std::max((int)total, cap_) + 1) + 64);   // a pair's
+    ml_levels();
+    grid_group_.reserve([&](auto add) {
+        size_t t = (size_t)total, mt = (size_t)ml_total_;
+        add(count_, 2 * (t + 1));   // and the scatter's cursors
+        add(start_, t + 2);
+        for (auto *v : {&ucount_, &ucol_, &cell_row0_, &ccells_}) add(*v, t);
+        for (auto *v : {&rs_, &aflag_, &apos_, &acells_}) add(*v, t + 1);
+        add(scanws_, scan_workspace((int)total + 1) + scan_workspace(std::max((int)total, cap_) + 1) + 64);   // a pair's
+        add(mlscan_, scan_workspace(ml_total_ + 1));
+        for (auto *v : {&mlflag_, &mlpos_, &mlmap_, &mlact_}) add(*v, mt + 1);
+        for (auto *v : {&mlcnode_, &mlcell_}) add(*v, t + 1);
+        for (auto *v : {&mlb_, &mlx_, &mly_}) add(*v, mt);
+    });
     g_.start = start_.p;
 
     // cells sorted by (colour, linear index)
@@ -744,15 +749,10 @@ void Engine<D>::build_grid()
     color_off_ = cnt;
     std::vector<int> fill(cnt.begin(), cnt.end() - 1);
     for (long long l = 0; l < total; l++) cc[(size_t)fill[color_of(l)]++] = (int)l;
-    ccells_.reserve(total);
     MPS_CUDA(cudaMemcpy(ccells_.p, cc.data(), sizeof(int) * (size_t)total, cudaMemcpyHostToDevice));
     color_off_dev_.reserve(ncol + 1);
     MPS_CUDA(cudaMemcpy(color_off_dev_.p, color_off_.data(), sizeof(int) * (ncol + 1), cudaMemcpyHostToDevice));
-    aflag_.reserve(total + 1);
-    apos_.reserve(total + 1);
-    acells_.reserve(total + 1);
     sizes_.reserve(64);
-    ml_levels();
 }
 
 // The nested grids over the cell grid: nodes on the cell corners, then every
@@ -782,7 +782,6 @@ void Engine<D>::ml_levels()
         for (int d = 0; d < D; d++) n[d] = n[d] / 2 + 1;
     }
     ml_total_ = (int)first;
-    mlscan_.reserve(scan_workspace(ml_total_ + 1));
 }
 
 // Constants evaluated with the reference's expressions.
@@ -992,7 +991,6 @@ void Engine<D>::sort()
     State<D> &dst = S_[cur_ ^ 1];
     MPS_CUDA(cudaMemsetAsync(count_.p, 0, 2 * sizeof(int) * ((size_t)total + 1), st_));
     int *cursor = count_.p + total + 1;
-    keyf_.reserve((size_t)cap_);
     if (n) launch(k_bin<D>, nblk(n, TPB), TPB, 0, st_, src, g_, n, kcell_.p, count_.p, excl_.p);
     scan_exclusive2<int>(count_.p, start_.p, total, excl_.p, exoff_.p, n, scanws_.p, st_);
     if (n) {
@@ -1016,7 +1014,6 @@ NbrSource<D> Engine<D>::near()
 {
     NbrSource<D> src{cells(), nullptr, nullptr, 0};
     int n = n_;
-    nbr_cnt_.reserve((size_t)cap_);
     if (!nbr_valid_ && n) {
         // room for 1.4 times the neighbours of the rest lattice; a particle
         // with more (a blow-up) walks the cells in every operator
@@ -1036,7 +1033,6 @@ NbrSource<D> Engine<D>::near()
                 nbr_pitch_ = 0;
             }
         }
-        keyf_.reserve((size_t)cap_);
         // FP32 coordinates are off by at most 2^-24 of the grid's extent (in
         // cells); a squared distance near 1 by less than 8 times that (on
         // wider grids FP32 decides nothing)
@@ -1368,9 +1364,6 @@ template <int D>
 void Engine<D>::ml_nodes(int nact)
 {
     int total = ml_total_, nl = ml_.nl;
-    for (auto *v : {&mlflag_, &mlpos_, &mlmap_, &mlact_}) v->reserve((size_t)total + 1);
-    mlcnode_.reserve((size_t)nact + 1);
-    mlcell_.reserve((size_t)g_.total);
     MPS_CUDA(cudaMemsetAsync(mlflag_.p, 0, sizeof(int) * (size_t)total, st_));
     launch(k_ml_flag1<D>, nblk(nact, TPB), TPB, 0, st_, nact, (const int *)acells_.p, g_, ml_.g[0], mlflag_.p,
            mlcnode_.p);
@@ -1441,24 +1434,31 @@ void Engine<D>::ml_build(int n_eq)
     ml_add_ = ml_ld_ > 0 && (ml_add_rows_ >= 0 ? n_eq < ml_add_rows_
                                                : n_eq <= ml_small_rows_ || (n_eq >= 20000 && n_eq < 40000));
     // zero around the nodes in use (the dense grid alone reads no neighbours)
-    for (auto *v : {&mlb_, &mlx_, &mly_}) {
-        v->reserve((size_t)ml_total_);
-        if (ml_ld_ > 0) MPS_CUDA(cudaMemsetAsync(v->p, 0, sizeof(double) * (size_t)ml_total_, st_));
+    if (ml_ld_ > 0)
+        for (auto *v : {&mlb_, &mlx_, &mly_})
+            MPS_CUDA(cudaMemsetAsync(v->p, 0, sizeof(double) * (size_t)ml_total_, st_));
+    size_t msize = (size_t)ML_COARSEST * ML_COARSEST, mcsize = 0;   // of the dense V-cycle
+    for (int l = ml_ld_; l < nl; l++) {
+        size_t nf = mlc_.lo[l + 1] - mlc_.lo[l], nc = l + 1 < nl ? mlc_.lo[l + 2] - mlc_.lo[l + 1] : 0;
+        msize = std::max(msize, nf * nf);
+        mcsize = std::max(mcsize, nf * nc);
     }
-    mlncell_.reserve((size_t)L::NC * na1);
-    mlcm_.reserve((size_t)nact * L::NC * L::W4);
-    mlA_.reserve((size_t)nall * L::STP);
-    mlC_.reserve((size_t)(nall - na1) * L::W7P + 1);
-    mldinv_.reserve((size_t)nall);
-    mlcsum_.reserve((size_t)nact * L::NC * 2);
-    mlbd_.reserve((size_t)std::max(ML_DENSE, ML_COARSEST));
-    mlunder_.reserve((size_t)nall);
-    mlabove_.reserve((size_t)nall);
-    mlpar_.reserve((size_t)nall);
-    mlfrac_.reserve((size_t)D * cap_);
-    jdinv_.reserve((size_t)cap_);
-    ufpar_.reserve((size_t)cap_);
-    ufkeep_.reserve((size_t)cap_);
+    ml_group_.reserve([&](auto add) {
+        size_t n1 = na1, n = nall, a = nact;
+        add(mlncell_, L::NC * n1);
+        add(mlcm_, a * L::NC * L::W4);
+        add(mlA_, n * L::STP);
+        add(mlB_, n1 * L::STP);
+        add(mlC_, (n - n1) * L::W7P + 1);
+        add(mldinv_, n);
+        add(mlcsum_, a * L::NC * 2);
+        add(mlbd_, std::max(ML_DENSE, ML_COARSEST));
+        add(mlxd_, ML_DENSE);
+        for (auto *v : {&mlunder_, &mlabove_}) add(*v, n);
+        add(mlpar_, n);
+        for (auto &m : mlM_) add(m, msize);
+        add(mlMC_, mcsize);
+    });
     const int *rp = row_ptr_.p, *dp = diagpos_.p, *ci = col_.p;
     const double *A = A_.p;
     adesc_.reserve((size_t)nact + 1);
@@ -1477,7 +1477,6 @@ void Engine<D>::ml_build(int n_eq)
     launch(k_ml_cellmat<D>, nblk(nact, ML_CW), 32 * ML_CW, 0, st_, nact, (const int *)acells_.p,
            (const int2 *)adesc_.p, g_, rp, dp, (const unsigned short *)runs_.p, ci, A, (const float *)mlfrac_.p, cap_,
            mlcm_.p);
-    mlB_.reserve((size_t)na1 * L::STP);
     launch(k_ml_b1<D>, na1, L::STP, 0, st_, na1, (const int *)mlncell_.p, (const double *)mlcm_.p, mlB_.p);
     launch(k_ml_a1<D>, na1, L::STP, 0, st_, mlc_.g[0], (const int *)mlact_.p, (const int *)mlmap_.p,
            (const double *)mlB_.p, ml_add_, mlA_.p, mldinv_.p);
@@ -1490,14 +1489,11 @@ void Engine<D>::ml_build(int n_eq)
     }
     launch(k_ml_tables<D>, nblk(nall, TPB), TPB, 0, st_, mlc_, (const int *)mlact_.p, mlunder_.p, mlabove_.p, mlpar_.p);
     int lo = mlc_.lo[nl - 1], n = nall - lo;
-    mlM_[0].reserve((size_t)ML_COARSEST * ML_COARSEST);
     launch(k_ml_inverse<D>, 1, 1024, sizeof(double) * ML_COARSEST * ML_COARSEST, st_, mlc_.g[nl - 1], lo, n,
            (const int *)mlact_.p, (const int *)mlmap_.p, (const double *)mlA_.p + (size_t)lo * L::STP, mlM_[0].p);
     int cur = 0;
     for (int l = nl - 2; l >= ml_ld_; l--) {
         int lof = mlc_.lo[l], loc = mlc_.lo[l + 1], nf = loc - lof, nc = mlc_.lo[l + 2] - loc;
-        mlMC_.reserve((size_t)nf * nc);
-        mlM_[cur ^ 1].reserve((size_t)nf * nf);
         launch(k_ml_dense_mc<D>, nf, 128, 0, st_, mlc_.g[l + 1], lof, nf, loc, nc, na1, (const int *)mlmap_.p,
                (const int *)mlabove_.p, (const unsigned char *)mlpar_.p, (const double *)mlC_.p,
                (const double *)mlM_[cur].p, mlMC_.p);
@@ -1512,10 +1508,11 @@ void Engine<D>::ml_build(int n_eq)
                 sizeof(double) * ml_small_vectors() <= ML_CL_SMEM && ml_clusters() > 0;
     if (ml_small_) {
         int nd = mlc_.lo[ml_ld_ + 1] - mlc_.lo[ml_ld_];
-        mlcellnode_.reserve((size_t)nact * L::NC);
-        mlfine_.reserve((size_t)nd * L::CELLS);
-        mlparent_.reserve((size_t)na1 * L::NC);
-        mlxd_.reserve((size_t)ML_DENSE);
+        ml_small_group_.reserve([&](auto add) {
+            add(mlcellnode_, (size_t)nact * L::NC);
+            add(mlfine_, (size_t)nd * L::CELLS);
+            add(mlparent_, (size_t)na1 * L::NC);
+        });
         launch(k_ml_small_tables<D>, nblk(std::max(nact, std::max(na1, nd)), TPB), TPB, 0, st_, nact, na1, nd, ml_add_,
                mlc_.g[0], mlc_.g[ml_ld_], (const int *)mlcnode_.p, (const int *)mlmap_.p, (const int *)mlunder_.p,
                (const int *)mlabove_.p, (const unsigned char *)mlpar_.p, mlcellnode_.p, mlfine_.p, mlparent_.p);
@@ -1684,6 +1681,9 @@ void Engine<D>::factor_ic0()
     size_t nnz = (size_t)nnz_;
     State<D> &s = S();
     F_.reserve(nnz);
+    inpos_.reserve(cap_);
+    outpos_.reserve(cap_);
+    for (auto *v : {&pk_len_lo_, &pk_len_up_, &pk_off_lo_, &pk_off_up_}) v->reserve((size_t)cap_ + 1);
     launch(k_row_splits, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)row_ptr_.p, (const int *)diagpos_.p,
            (const int *)col_.p, (const int *)part_of_row_.p, (const int *)s.cell, (const int *)cell_row0_.p,
            (const int *)ucount_.p, inpos_.p, outpos_.p);
@@ -1911,7 +1911,6 @@ void Engine<D>::ppe(bool clamp)
     met.nnz = nnz;
     col_.reserve(nnz);
     A_.reserve(nnz);
-    bounded_.reserve(cap_);
     launch(k_fill<D>, nblk(n_eq, ROW_BLOCK), ROW_BLOCK, 0, st_, src, s, k_, (const int *)part_of_row_.p,
            (const int *)row_of_.p, n_eq, cap_, (const int *)row_ptr_.p, (const unsigned short *)runs_.p,
            (const unsigned short *)diagoff_.p, col_.p, A_.p, diagpos_.p, b_.p, bounded_.p, err_.p);
