@@ -506,6 +506,12 @@ private:
     // adjoint: stop at kAdjRtol ||b|| (or the rounding floor) and leave the
     // step's metrics as they are
     void mixed_solve(int n_eq, long long nnz, bool icc, bool adjoint = false);
+    // packed words for the launch-per-colour loop; the persistent and the
+    // CTA-per-cell loops read the separate arrays
+    bool packed_spmv() const
+    {
+        return pack_ && mixed_spmv_ == 2 && (ml_on_ || (sweep_mode_ == 0 && head_batch_ == 4));
+    }
     void build_windows(bool fp32);
     void factor_ic0();      // IC(0) factor and sweep tables of the current matrix
     void convert_ic0();     // their FP32 copies
@@ -1911,11 +1917,19 @@ void Engine<D>::ppe(bool clamp)
     met.nnz = nnz;
     col_.reserve(nnz);
     A_.reserve(nnz);
-    launch(k_fill<D>, nblk(n_eq, ROW_BLOCK), ROW_BLOCK, 0, st_, src, s, k_, (const int *)part_of_row_.p,
-           (const int *)row_of_.p, n_eq, cap_, (const int *)row_ptr_.p, (const unsigned short *)runs_.p,
-           (const unsigned short *)diagoff_.p, col_.p, A_.p, diagpos_.p, b_.p, bounded_.p, err_.p);
-    MPS_CUDA(cudaEventRecord(ev_[2], st_));
     bool icc = prm_.solver_type == 1;
+    const bool mixed = prm_.precision == MPS_PREC_MIXED && mixed_spmv_ == 2, packed = mixed && packed_spmv();
+    if (mixed) dsum_.reserve((size_t)cap_);
+    if (packed) ac32_.reserve(nnz);
+    const bool sums = k_.hs_mode == 1 || k_.ppe_type == 1;   // the source term sums over neighbours
+    launch(mixed ? k_fill<D, true> : k_fill<D, false>, nblk((long long)n_eq * FILL_LANES, ROW_BLOCK), ROW_BLOCK, 0,
+           st_, src, s, k_, (const int *)part_of_row_.p, (const int *)row_of_.p, n_eq, cap_, (const int *)row_ptr_.p,
+           (const unsigned short *)runs_.p, (const unsigned short *)diagoff_.p, col_.p, A_.p,
+           packed ? ac32_.p : nullptr, dsum_.p, diagpos_.p, sums ? nullptr : b_.p, bounded_.p, err_.p);
+    if (sums)
+        launch(k_rhs<D>, nblk(n_eq, ROW_BLOCK), ROW_BLOCK, 0, st_, src, s, k_, (const int *)part_of_row_.p, n_eq,
+               b_.p);
+    MPS_CUDA(cudaEventRecord(ev_[2], st_));
     ic0_valid_ = icc;
     ic0_built_ = false;
     if (icc && ml_on_) ml_build(n_eq);
@@ -2378,15 +2392,10 @@ void Engine<D>::mixed_solve(int n_eq, long long nnz, bool icc, bool adjoint)
 {
     const int RB = RED_BLOCKS;
     size_t nz = (size_t)nnz;
-    // packed words for the launch-per-colour loop; the persistent and the
-    // CTA-per-cell loops read the separate arrays
-    const bool pk = pack_ && (ml_on_ || (sweep_mode_ == 0 && head_batch_ == 4));
-    const bool pk_spmv = pk && mixed_spmv_ == 2;
+    const bool pk_spmv = packed_spmv();
     zprev_.reserve((size_t)cap_);
-    if (pk_spmv) {
-        ac32_.reserve(nz);
-        launch(k_pack_fc, RB, CG_BLOCK, 0, st_, nz, (const double *)A_.p, (const int *)col_.p, ac32_.p);
-    } else {
+    if (!pk_spmv) {   // else the assembly has written the packed words
+
         A32_.reserve(nz);
         launch(k_convert<double, float>, RB, CG_BLOCK, 0, st_, nz, (const double *)A_.p, A32_.p);
     }
@@ -2411,12 +2420,7 @@ void Engine<D>::mixed_solve(int n_eq, long long nnz, bool icc, bool adjoint)
         v.xfc_lo = xfc32_lo_.p;
         v.xfc_up = xfc32_up_.p;
     }
-    if (mixed_spmv_ == 2) {
-        dsum_.reserve((size_t)cap_);
-        launch(k_row_sum, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)row_ptr_.p, (const double *)A_.p,
-               dsum_.p);
-        v.dsum = dsum_.p;
-    }
+    if (mixed_spmv_ == 2) v.dsum = dsum_.p;   // the assembly's
     const double *zsrc = icc ? z_.p : r_.p;   // the preconditioned residual
     // tolerance of the next inner solve from a true residual `rn`: a reduction
     // by rel_delta_, or, where that comes near the goal, well below it, since

@@ -192,7 +192,14 @@ k_row_count(NbrSource<D> src, State<D> s, const int *__restrict__ part_of_row, c
     rcount[r] = off;
 }
 
-// Right-hand side of one unknown row (pressure_solver.c:328-362, 524-529).
+// Right-hand side of one unknown row (pressure_solver.c:328-362, 524-529):
+// without sums over neighbours, and in general.
+template <int D>
+__device__ __forceinline__ double ppe_rhs_density(const State<D> &s, const Consts &k, int i)
+{
+    return s.type[i] == WALL ? 0.0 : k.rhs_k * (s.n[i] - k.n0) / k.n0;
+}
+
 template <int D, class Src>
 __device__ double ppe_rhs(const Src &src, const State<D> &s, const Consts &k, int i, const double *pi)
 {
@@ -238,23 +245,44 @@ __device__ double ppe_rhs(const Src &src, const State<D> &s, const Consts &k, in
         }
         return k.rhs_na * div + k.rhs_nb * (s.n[i] - n0) / n0;
     }
-    return k.rhs_k * (s.n[i] - n0) / n0;
+    return ppe_rhs_density<D>(s, k, i);
 }
 
-// One row of A and b: the row's neighbours in the reference's order for the
-// diagonal sum and the source term (bounded[row]: the row couples to a known
-// pressure), each off-diagonal at its place in its cell's run.  A neighbour's
-// weight is computed once, for the sum and the entry.
+// The source terms that sum over neighbours, a thread per row.
 template <int D>
+__global__ void __launch_bounds__(ROW_BLOCK)
+k_rhs(NbrSource<D> src, State<D> s, Consts k, const int *__restrict__ part_of_row, int n_eq, double *__restrict__ b)
+{
+    int r = blockIdx.x * ROW_BLOCK + threadIdx.x;
+    if (r >= n_eq) return;
+    int i = part_of_row[r];
+    double pi[D];
+    load_vec<D>(pi, s.pos, i);
+    b[r] = ppe_rhs<D>(src, s, k, i, pi);
+}
+
+// One row of A (and b, unless k_rhs forms it) by FILL_LANES lanes: the row's
+// neighbours in the reference's order for the diagonal sum (bounded[row]: the
+// row couples to a known pressure), each off-diagonal at its place in its
+// cell's run.  A neighbour's weight is computed once, for the sum and the
+// entry; every lane adds the group's weights one by one, so the sum is the
+// reference's bit for bit.  FC: the packed words of the FP32 product and the
+// rows' sums come out of the same pass.
+constexpr int FILL_LANES = 8;
+
+template <int D, bool MIXED>
 __global__ void __launch_bounds__(ROW_BLOCK)
 k_fill(NbrSource<D> src, State<D> s, Consts k, const int *__restrict__ part_of_row,
        const int *__restrict__ row_of, int n_eq, int stride, const int *__restrict__ row_ptr,
        const unsigned short *__restrict__ runs, const unsigned short *__restrict__ diagoff, int *__restrict__ col,
-       double *__restrict__ val, int *__restrict__ diagpos, double *__restrict__ b,
-       unsigned char *__restrict__ bounded, unsigned *err)
+       double *__restrict__ val, uint2 *__restrict__ fc, double *__restrict__ dsum, int *__restrict__ diagpos,
+       double *__restrict__ b, unsigned char *__restrict__ bounded, unsigned *err)
 {
-    int r = blockIdx.x * ROW_BLOCK + threadIdx.x;
-    if (r >= n_eq) return;
+    constexpr int L = FILL_LANES;
+    int r = (int)((blockIdx.x * (long long)ROW_BLOCK + threadIdx.x) / L);
+    if (r >= n_eq) return;   // whole groups
+    int lane = threadIdx.x & 31, l = lane % L;
+    unsigned group = ((1u << L) - 1u) << (lane - l);
     int i = part_of_row[r];
     double pi[D];
     load_vec<D>(pi, s.pos, i);
@@ -263,48 +291,86 @@ k_fill(NbrSource<D> src, State<D> s, Consts k, const int *__restrict__ part_of_r
     int par = cell_parity<D>(g, ci);
     int base = row_ptr[r], end = row_ptr[r + 1];
     int dpos = base + diagoff[r];
-    int prev = -1, pos = base, placed = 1;
-    double sum_w = 0.0;
+    int placed = 1;
+    double sum_w = 0.0, sum_off = 0.0;
     bool known = k.diag_scale != k.coeff;   // the row sum is not zero
-    struct Data {
-        double x[D];
-        int type, row, cell;
+    auto run_of = [&](int cell) {
+        return base + runs[(size_t)visit_rank<D>(par, neighbour_cell<D>(g, cell - ci)) * stride + r];
     };
-    src.for_each_with(
-        i,
-        [&](int j) {
-            Data q;
-            load_vec<D>(q.x, s.pos, j);
-            q.type = s.type[j];
-            q.row = row_of[j];
-            q.cell = s.cell[j];
-            return q;
-        },
-        [&](int, const Data &q) {
-            if (q.type == DUMMY) return;
-            double w = kweight(sqrt(dist2<D>(pi, q.x)), k.re_lap, k.rmin);
-            sum_w += w;
-            if (q.row < 0) {
-                known = known || w > 0.0;
-                return;
+    auto put = [&](int q, int c, double v) {
+        if (q >= end) return;
+        col[q] = c;
+        val[q] = v;
+        if (MIXED && fc) fc[q] = make_uint2(__float_as_uint((float)v), (unsigned)c);
+    };
+    int c = __ldg(&src.cnt[i]);
+    if (c > src.pitch) {   // more neighbours than the list holds: the first lane walks the cells
+        if (l == 0) {
+            int prev = -1, pos = base;
+            src.cells.for_each(i, [&](int j) {
+                int row = row_of[j], cell = s.cell[j];
+                if (s.type[j] == DUMMY) return;
+                double pj[D];
+                load_vec<D>(pj, s.pos, j);
+                double w = kweight(sqrt(dist2<D>(pi, pj)), k.re_lap, k.rmin);
+                sum_w += w;
+                if (row < 0) {
+                    known = known || w > 0.0;
+                    return;
+                }
+                if (cell != prev) {
+                    prev = cell;
+                    pos = run_of(cell);
+                }
+                if (pos == dpos) pos++;
+                put(pos, row, k.neg_coeff * w);
+                sum_off += k.neg_coeff * w;
+                pos++;
+                placed++;
+            });
+        }
+    } else {
+        const int *p = src.idx + (size_t)(i >> 5) * 32 * src.pitch + (i & 31);
+        int prev = -1, pos = base;   // the cell of the last neighbour so far, and the next place in its run
+        int jn = l < c ? __ldg(p + 32 * l) : i;
+        for (int k0 = 0; k0 < c; k0 += L) {
+            int j = jn;
+            bool in = k0 + l < c;
+            jn = k0 + L + l < c ? __ldg(p + 32 * (k0 + L + l)) : i;
+            double pj[D];
+            load_vec<D>(pj, s.pos, j);
+            int row = row_of[j], cell = s.cell[j];
+            in = in && s.type[j] != DUMMY;
+            double w = in ? kweight(sqrt(dist2<D>(pi, pj)), k.re_lap, k.rmin) : 0.0;
+            bool unk = in && row >= 0;
+            known = known || (in && row < 0 && w > 0.0);
+            unsigned um = __ballot_sync(group, unk) >> (lane - l);
+            // the list runs cell by cell: my run's first lane in this piece
+            int before = __shfl_up_sync(group, cell, 1, L);
+            if (l == 0) before = prev;
+            bool head = cell != before;
+            unsigned hm = (__ballot_sync(group, head) >> (lane - l)) & ((2u << l) - 1u);
+            int h = hm ? 31 - __clz(hm) : 0;
+            int at = (hm ? run_of(cell) : pos) + __popc(um & ((1u << l) - 1u) & ~((1u << h) - 1u));
+            if (unk) put(at + (cell == ci && row > r), row, k.neg_coeff * w);
+            pos = __shfl_sync(group, at + unk, L - 1, L);
+            prev = __shfl_sync(group, cell, L - 1, L);
+            placed += __popc(um);
+#pragma unroll
+            for (int u = 0; u < L; u++) {
+                double wu = __shfl_sync(group, w, u, L);
+                sum_w += wu;
+                if (MIXED && (um >> u & 1)) sum_off += k.neg_coeff * wu;
             }
-            if (q.cell != prev) {
-                prev = q.cell;
-                pos = base + runs[(size_t)visit_rank<D>(par, neighbour_cell<D>(g, q.cell - ci)) * stride + r];
-            }
-            if (pos == dpos) pos++;
-            if (pos < end) {
-                col[pos] = q.row;
-                val[pos] = k.neg_coeff * w;
-            }
-            pos++;
-            placed++;
-        });
+        }
+        known = __any_sync(group, known);
+    }
+    if (l) return;
     bounded[r] = known;
     diagpos[r] = dpos;
-    col[dpos] = r;
-    val[dpos] = k.diag_scale * sum_w;
-    b[r] = ppe_rhs<D>(src, s, k, i, pi);
+    put(dpos, r, k.diag_scale * sum_w);
+    if (MIXED) dsum[r] = sum_off + k.diag_scale * sum_w;
+    if (b) b[r] = ppe_rhs_density<D>(s, k, i);
     if (placed != end - base) atomicOr(err, ERR_COLORING);
 }
 
@@ -1482,17 +1548,6 @@ __global__ void k_convert(size_t n, const S *__restrict__ in, T *__restrict__ ou
 {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         out[i] = (T)in[i];
-}
-
-// dsum_i = sum_j A_ij in FP64, in entry order (the difference-form SpMV).
-__global__ void k_row_sum(int n_eq, const int *__restrict__ row_ptr, const double *__restrict__ A,
-                          double *__restrict__ dsum)
-{
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_eq) return;
-    double s = 0.0;
-    for (int q = row_ptr[r]; q < row_ptr[r + 1]; q++) s += A[q];
-    dsum[r] = s;
 }
 
 // x = 0, r = b, ||b||^2 into sc->rr_outer.
