@@ -24,9 +24,9 @@ would time broken flow.  The device-side checkpoint load is inside the
 timed region; the e2e arm restores its host arrays between the timed calls.
 --rollout times consecutive steps instead.
 
-Other keys: `roofline` for the dominant kernel (the IC(0) colour sweep
-k_sweep_colour, with the CG SpMV beside it; CUDA events on the library's
-stream in two profiled steps after the timed ones), `cpu_baseline` (the
+Other keys: `roofline` for the dominant kernel (the CG SpMV; with
+MPS_SWEEP=0 the IC(0) colour sweep k_sweep_colour first; CUDA events on the
+library's stream in two profiled steps after the timed ones), `cpu_baseline` (the
 reference compiled from source, OpenMP on all host cores, on a bounded
 sample of the same workload), `e2e` (the same metric through the C ABI with
 host buffers copied in and out every step), `clocks` (nvidia-smi sampled
