@@ -58,17 +58,28 @@ __device__ __forceinline__ int cell_parity(const Grid<D> &g, int c)
     return par;
 }
 
-// Number of a neighbouring cell from the difference of the linear indices.
+// Number of cell c as a neighbour of cell ci (1 + the coordinate differences,
+// x fastest).  The linear difference gives it where every direction but the
+// last has three cells or more; on a thinner grid (a domain narrower than the
+// margins around it) two neighbours can share a difference, so the coordinates
+// are compared.
 template <int D>
-__device__ __forceinline__ int neighbour_cell(const Grid<D> &g, int diff)
+__host__ __device__ __forceinline__ int neighbour_cell(const Grid<D> &g, int c, int ci)
 {
-    int nx = g.dims[0];
+    int nx = g.dims[0], ny = g.dims[1];
+    if (nx < 3 || (D == 3 && ny < 3)) {
+        int n = c % nx - ci % nx + 1;
+        c /= nx;
+        ci /= nx;
+        if (D == 2) return n + 3 * (c - ci + 1);
+        return n + 3 * (c % ny - ci % ny + 1) + 9 * (c / ny - ci / ny + 1);
+    }
     if (D == 2) {
-        int v = diff + nx + 1, y = v / nx;
+        int v = c - ci + nx + 1, y = v / nx;
         return v - y * nx + 3 * y;
     }
-    int nxy = nx * g.dims[1];
-    int v = diff + nxy + nx + 1, z = v / nxy;
+    int nxy = nx * ny;
+    int v = c - ci + nxy + nx + 1, z = v / nxy;
     v -= z * nxy;
     int y = v / nx;
     return v - y * nx + 3 * y + 9 * z;
@@ -175,7 +186,7 @@ k_row_count(NbrSource<D> src, State<D> s, const int *__restrict__ part_of_row, c
                           if (q.x < 0) return;
                           if (q.y != prev) {
                               prev = q.y;
-                              nb = neighbour_cell<D>(g, q.y - ci);
+                              nb = neighbour_cell<D>(g, q.y, ci);
                           }
                           cnt[nb][threadIdx.x]++;
                           below += q.y == ci && j < i;
@@ -295,7 +306,7 @@ k_fill(NbrSource<D> src, State<D> s, Consts k, const int *__restrict__ part_of_r
     double sum_w = 0.0, sum_off = 0.0;
     bool known = k.diag_scale != k.coeff;   // the row sum is not zero
     auto run_of = [&](int cell) {
-        return base + runs[(size_t)visit_rank<D>(par, neighbour_cell<D>(g, cell - ci)) * stride + r];
+        return base + runs[(size_t)visit_rank<D>(par, neighbour_cell<D>(g, cell, ci)) * stride + r];
     };
     auto put = [&](int q, int c, double v) {
         if (q >= end) return;
