@@ -912,7 +912,7 @@ void Engine<D>::check_err()
 template <int D>
 void Engine<D>::copy_to_host(void *host, const void *dev, size_t bytes)
 {
-    if (HostPipe::wanted(host, bytes)) {
+    if (pipe_.wanted(host, bytes)) {
         pipe_.to_host(host, dev, bytes, st_);
     } else {
         MPS_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st_));
@@ -923,7 +923,7 @@ void Engine<D>::copy_to_host(void *host, const void *dev, size_t bytes)
 template <int D>
 void Engine<D>::copy_to_device(void *dev, const void *host, size_t bytes)
 {
-    if (HostPipe::wanted(host, bytes)) pipe_.to_device(dev, host, bytes, st_);
+    if (pipe_.wanted(host, bytes)) pipe_.to_device(dev, host, bytes, st_);
     else MPS_CUDA(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st_));
 }
 
@@ -1225,7 +1225,7 @@ void Engine<D>::upload_list(const int *nb, const int *cnt, int max_nb)
         launch(k_gather_host_list, nblk((long long)n * 32, TPB), TPB, 0, st_, (const int *)pa.devicePointer,
                max_nb, (const int *)lcnt_.p, (const int *)lptr_.p, n, lidx_.p, err_.p);
     } else if (used < 0x7fffffffLL && (size_t)mc * sizeof(int) <= HostPipe::kChunk &&
-               HostPipe::wanted(nb, sizeof(int) * (size_t)used)) {
+               pipe_.wanted(nb, sizeof(int) * (size_t)used)) {
         lidx_.reserve((size_t)used);
         // chunks of whole rows: first row and first entry of each
         constexpr long long room = HostPipe::kChunk / sizeof(int);
@@ -2795,7 +2795,7 @@ void Engine<D>::get_neighbor_list(int *nb, int *cnt, int max_nb)
     launch(k_build_list<D>, nblk(n, TPB), TPB, 0, st_, near(), (const int *)S().id, n, max_nb, mc, lout_.p,
            lcnt_.p, err_.p);
     size_t row_bytes = sizeof(int) * (size_t)mc;
-    if (row_bytes <= HostPipe::kChunk && HostPipe::wanted(nb, row_bytes * (size_t)n)) {
+    if (row_bytes <= HostPipe::kChunk && pipe_.wanted(nb, row_bytes * (size_t)n)) {
         size_t rows = HostPipe::kChunk / row_bytes, nc = ((size_t)n + rows - 1) / rows;
         pipe_.chunks_to_host(
             nc, st_,

@@ -1,30 +1,14 @@
 // engine.cuh -- host-side engine of one device-resident particle system.
 #pragma once
 
-#include <cuda_runtime.h>
-
-#include <stdexcept>
 #include <string>
 #include <vector>
 
-#include "../../include/mps_b200.h"
 #include "device.cuh"
+#include "error.cuh"
 #include "k_ppe.cuh"
 
 namespace mps {
-
-struct CudaError : std::runtime_error {
-    int code;
-    CudaError(const std::string &m, int c) : std::runtime_error(m), code(c) {}
-};
-
-#define MPS_CUDA(call)                                                                         \
-    do {                                                                                       \
-        cudaError_t e_ = (call);                                                               \
-        if (e_ != cudaSuccess)                                                                 \
-            throw ::mps::CudaError(std::string(#call) + ": " + cudaGetErrorString(e_),         \
-                                   e_ == cudaErrorMemoryAllocation ? MPS_ERR_OOM : MPS_ERR_CUDA); \
-    } while (0)
 
 // Growable device array; contents are not preserved on growth.
 template <class T>

@@ -8,19 +8,19 @@
 // before between its buffer and the caller's memory, so the link and the
 // host copies overlap.  The threads live for one call; the buffers belong to
 // the engine, are made on its first large transfer and are given back with
-// it.
+// it.  Where they cannot be made, transfers stay plain copies, and the share
+// of a thread that cannot be started is done by the caller's.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
-#include <functional>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <vector>
 
-#include "engine.cuh"
+#include "error.cuh"
 
 namespace mps {
 
@@ -41,15 +41,15 @@ public:
     }
 
     // Whether a transfer of `bytes` with host memory `p` goes through the pipe.
-    static bool wanted(const void *p, size_t bytes)
+    bool wanted(const void *p, size_t bytes)
     {
         if (bytes < kLarge) return false;
         cudaPointerAttributes a{};
         if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
             (void)cudaGetLastError();
-            return true;
+            return ready();
         }
-        return a.type == cudaMemoryTypeUnregistered;
+        return a.type == cudaMemoryTypeUnregistered && ready();
     }
 
     // `dev` (bytes) to host memory; returns when the bytes are there.
@@ -128,27 +128,46 @@ private:
 
     char *buffer(int t, int b) const { return buf_ + (size_t)(2 * t + b) * kChunk; }
     cudaEvent_t event(int t, int b) const { return ev_[2 * t + b]; }
+
+    // Makes the events and the page-locked buffers on first use; false where
+    // the system has none to give.
+    bool ready()
+    {
+        if (buf_) return true;
+        for (auto &e : ev_)
+            if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+                e = nullptr;
+                (void)cudaGetLastError();
+                return false;
+            }
+        if (cudaMallocHost((void **)&buf_, 2 * kThreads * kChunk) != cudaSuccess) {
+            buf_ = nullptr;
+            (void)cudaGetLastError();
+            return false;
+        }
+        return true;
+    }
+
     static void ok(cudaError_t e)
     {
         if (e != cudaSuccess) throw CudaError(std::string("host transfer: ") + cudaGetErrorString(e), MPS_ERR_CUDA);
     }
 
     // body(t, threads) on each thread, the caller's being thread 0; the first
-    // failure is thrown after all have ended.
+    // failure is thrown after all have ended and every copy is out of the
+    // buffers.  Nothing is thrown past a running thread: what can fail between
+    // the first one's start and the last one's end is caught on the spot.
     template <class Body>
     void run(size_t n, Body body)
     {
         if (n == 0) return;
-        if (!buf_) {
-            for (auto &e : ev_)
-                if (!e) MPS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            MPS_CUDA(cudaMallocHost((void **)&buf_, 2 * kThreads * kChunk));
-        }
         int dev = 0;
         MPS_CUDA(cudaGetDevice(&dev));
         size_t threads = std::min<size_t>(std::min<size_t>(kThreads, n), std::max(1u, std::thread::hardware_concurrency()));
-        std::vector<std::exception_ptr> err(threads);
+        std::exception_ptr err[kThreads];
         std::vector<std::thread> pool;
+        pool.reserve(threads);
+        bool left[kThreads] = {};
         auto work = [&](int t) {
             try {
                 if (t) ok(cudaSetDevice(dev));
@@ -158,19 +177,22 @@ private:
             }
         };
         // a thread the system refuses to start does its share here instead
-        std::vector<int> left;
         for (size_t t = 1; t < threads; t++) {
             try {
                 pool.emplace_back(work, (int)t);
-            } catch (const std::system_error &) {
-                left.push_back((int)t);
+            } catch (...) {
+                left[t] = true;
             }
         }
         work(0);
-        for (int t : left) work(t);
+        for (size_t t = 1; t < threads; t++)
+            if (left[t]) work((int)t);
         for (auto &p : pool) p.join();
-        for (auto &e : err)
-            if (e) std::rethrow_exception(e);
+        for (size_t t = 0; t < threads; t++)
+            if (err[t]) {
+                for (auto &e : ev_) (void)cudaEventSynchronize(e);
+                std::rethrow_exception(err[t]);
+            }
     }
 };
 
