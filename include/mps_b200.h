@@ -171,7 +171,9 @@ const char *mps_error_string(int code);
 int  mps_session_create(mps_session **out, const mps_params_t *params, int capacity);
 int  mps_session_destroy(mps_session *s);
 /* Replace the parameters (a changed domain or radius rebuilds the grid and
- * requires a new neighbour search). */
+ * requires a new neighbour search).  On an error the parameters stay those of
+ * before; where the device had no memory for the new grid, the search has to
+ * be repeated all the same. */
 int  mps_update_params(mps_session *s, const mps_params_t *params);
 /* Select the precision form, MPS_PREC_FP64 or MPS_PREC_MIXED, from the next
  * step on, every other parameter kept; MPS_ERR_INVALID for any other value.

@@ -270,6 +270,7 @@ private:
     State<D> S_[2];
     int cur_ = 0;
     bool structure_ = false;   // cell structure valid for S_[cur_]
+    bool grid_ok_ = false;     // the grid's arrays are those of prm_ (false after a failed build_grid)
 
     // storage of the arrays sized by the capacity, by the grid, and by a solve's
     // grids (the last for the loop in one cluster)
@@ -488,6 +489,8 @@ private:
 
     void alloc_state();
     void build_grid();
+    void need_grid() { if (!grid_ok_) build_grid(); }
+    long long grid_of(const mps_params_t &p, Grid<D> &g) const;
     void compute_consts();
     void sort();
     void unsort();
@@ -706,23 +709,33 @@ void Engine<D>::alloc_state()
     }
 }
 
-// cell_list_create (neighbor_search.c:92-122) with cell size = list radius.
+// cell_list_create (neighbor_search.c:92-122) with cell size = list radius:
+// origin, cells per direction and in all of the grid that `p` asks for.
+template <int D>
+long long Engine<D>::grid_of(const mps_params_t &p, Grid<D> &g) const
+{
+    double re = list_radius(p), margin = 4.0 * re;
+    long long total = 1;
+    for (int d = 0; d < D; d++) {
+        g.origin[d] = p.domain_min[d] - margin;
+        double span = (p.domain_max[d] + margin) - g.origin[d];
+        g.dims[d] = (int)(span / re) + 2;
+        total *= g.dims[d];
+    }
+    if (total <= 0 || total > (1LL << 30)) throw CudaError("cell grid too large", MPS_ERR_INVALID);
+    g.total = (int)total;
+    g.cs_inv = 1.0 / re;
+    return total;
+}
+
 template <int D>
 void Engine<D>::build_grid()
 {
-    double re = list_radius(prm_);
-    re_list_ = re;
-    double margin = 4.0 * re;
-    long long total = 1;
-    for (int d = 0; d < D; d++) {
-        g_.origin[d] = prm_.domain_min[d] - margin;
-        double span = (prm_.domain_max[d] + margin) - g_.origin[d];
-        g_.dims[d] = (int)(span / re) + 2;
-        total *= g_.dims[d];
-    }
-    if (total <= 0 || total > (1LL << 30)) throw CudaError("cell grid too large", MPS_ERR_INVALID);
-    g_.total = (int)total;
-    g_.cs_inv = 1.0 / re;
+    Grid<D> g = g_;
+    long long total = grid_of(prm_, g);
+    grid_ok_ = false;
+    g_ = g;
+    re_list_ = list_radius(prm_);
     ml_levels();
     grid_group_.reserve([&](auto add) {
         size_t t = (size_t)total, mt = (size_t)ml_total_;
@@ -759,6 +772,7 @@ void Engine<D>::build_grid()
     color_off_dev_.reserve(ncol + 1);
     MPS_CUDA(cudaMemcpy(color_off_dev_.p, color_off_.data(), sizeof(int) * (ncol + 1), cudaMemcpyHostToDevice));
     sizes_.reserve(64);
+    grid_ok_ = true;
 }
 
 // The nested grids over the cell grid: nodes on the cell corners, then every
@@ -866,14 +880,30 @@ void Engine<D>::update_params(const mps_params_t &p)
     bool regrid = false;
     for (int d = 0; d < D; d++)
         regrid |= p.domain_min[d] != prm_.domain_min[d] || p.domain_max[d] != prm_.domain_max[d];
-    regrid |= list_radius(p) != re_list_;
-    prm_ = p;
+    regrid |= list_radius(p) != re_list_ || !grid_ok_;
+    mps_params_t old = prm_;
     if (regrid) {
+        Grid<D> g = g_;
+        grid_of(p, g);   // refused here, or not for its size: nothing has changed yet
         // a factor still to be formed reads the cells of the old grid
         if (ppe_valid_ && ic0_valid_) require_ic0();
-        build_grid();
         structure_ = false;
         nbr_valid_ = false;
+    }
+    prm_ = p;
+    if (regrid) {
+        try {
+            build_grid();
+        } catch (...) {
+            // the parameters stay those of before, with their grid: at the latest
+            // when it is next needed
+            prm_ = old;
+            try {
+                build_grid();
+            } catch (const std::exception &) {
+            }
+            throw;
+        }
     }
     compute_consts();
 }
@@ -992,6 +1022,7 @@ void Engine<D>::download_pressure(double *p, int num)
 template <int D>
 void Engine<D>::sort()
 {
+    need_grid();
     int n = n_, total = g_.total;
     State<D> &src = S_[cur_];
     State<D> &dst = S_[cur_ ^ 1];
@@ -2521,6 +2552,7 @@ template <int D>
 void Engine<D>::state_load(const void *src)
 {
     if (!src) throw CudaError("null checkpoint buffer", MPS_ERR_INVALID);
+    need_grid();
     StateHeader h{};
     MPS_CUDA(cudaMemcpyAsync(&h, src, sizeof h, cudaMemcpyDefault, st_));
     MPS_CUDA(cudaStreamSynchronize(st_));
