@@ -427,6 +427,12 @@ private:
     bool ppe_valid_ = false;
     bool ic0_valid_ = false;     // the last PPE was an ICCG one: its IC(0) factor can be had
     bool ic0_built_ = false;     // the factor and its sweep tables have been formed
+    // the numbering of the last PPE's cells, which a factor formed later reads:
+    // the grid's arrays, or copies once update_params has replaced the grid
+    struct PpeCells {
+        const int *act, *row0, *count;
+    } ppe_cells_{};
+    DevArray<int> ppe_cells_kept_;
     bool last_fp32_ = false;     // the last solve ran the mixed form (FP32 factor copies exist)
 
     // ---- driven walls
@@ -491,6 +497,7 @@ private:
     void build_grid();
     void need_grid() { if (!grid_ok_) build_grid(); }
     long long grid_of(const mps_params_t &p, Grid<D> &g) const;
+    void keep_ppe_cells();
     void compute_consts();
     void sort();
     void unsort();
@@ -885,8 +892,7 @@ void Engine<D>::update_params(const mps_params_t &p)
     if (regrid) {
         Grid<D> g = g_;
         grid_of(p, g);   // refused here, or not for its size: nothing has changed yet
-        // a factor still to be formed reads the cells of the old grid
-        if (ppe_valid_ && ic0_valid_) require_ic0();
+        keep_ppe_cells();
         structure_ = false;
         nbr_valid_ = false;
     }
@@ -906,6 +912,22 @@ void Engine<D>::update_params(const mps_params_t &p)
         }
     }
     compute_consts();
+}
+
+// Copies of the arrays in ppe_cells_ where a factor still to be formed needs
+// them after the grid's have been given back.
+template <int D>
+void Engine<D>::keep_ppe_cells()
+{
+    if (!ppe_valid_ || !ic0_valid_ || ic0_built_ || n_eq_ == 0 || ppe_cells_.act == ppe_cells_kept_.p) return;
+    size_t t = (size_t)g_.total;
+    ppe_cells_kept_.reserve(3 * t);
+    int *k = ppe_cells_kept_.p;
+    const int *from[3] = {ppe_cells_.act, ppe_cells_.row0, ppe_cells_.count};
+    for (int i = 0; i < 3; i++)
+        MPS_CUDA(cudaMemcpyAsync(k + i * t, from[i], sizeof(int) * t, cudaMemcpyDeviceToDevice, st_));
+    MPS_CUDA(cudaStreamSynchronize(st_));
+    ppe_cells_ = {k, k + t, k + 2 * t};
 }
 
 template <int D>
@@ -1722,8 +1744,8 @@ void Engine<D>::factor_ic0()
     outpos_.reserve(cap_);
     for (auto *v : {&pk_len_lo_, &pk_len_up_, &pk_off_lo_, &pk_off_up_}) v->reserve((size_t)cap_ + 1);
     launch(k_row_splits, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)row_ptr_.p, (const int *)diagpos_.p,
-           (const int *)col_.p, (const int *)part_of_row_.p, (const int *)s.cell, (const int *)cell_row0_.p,
-           (const int *)ucount_.p, inpos_.p, outpos_.p);
+           (const int *)col_.p, (const int *)part_of_row_.p, (const int *)s.cell, ppe_cells_.row0,
+           ppe_cells_.count, inpos_.p, outpos_.p);
     MPS_CUDA(cudaMemcpyAsync(F_.p, A_.p, sizeof(double) * nnz, cudaMemcpyDeviceToDevice, st_));
     for (int c = 0; c < ncol; c++) {
         int rb = row_off_[c], re = row_off_[c + 1];
@@ -1734,7 +1756,7 @@ void Engine<D>::factor_ic0()
         int kb = act_off_[c], ke = act_off_[c + 1];
         if (ke > kb)
             launch(k_ic0_incell, nblk(ke - kb, SWEEP_WARPS_IC), 32 * SWEEP_WARPS_IC, 0, st_, kb, ke,
-                   (const int *)acells_.p, (const int *)cell_row0_.p, (const int *)ucount_.p,
+                   ppe_cells_.act, ppe_cells_.row0, ppe_cells_.count,
                    (const int *)row_ptr_.p, (const int *)diagpos_.p, (const int *)inpos_.p,
                    (const int *)col_.p, (const double *)A_.p, F_.p);
     }
@@ -1750,7 +1772,7 @@ void Engine<D>::factor_ic0()
     pk_k_up_.reserve(in_cap);
     launch(k_pack_fill, nblk(n_eq, TPB), TPB, 0, st_, n_eq, (const int *)diagpos_.p, (const int *)inpos_.p,
            (const int *)outpos_.p, (const int *)col_.p, (const double *)F_.p, (const int *)part_of_row_.p,
-           (const int *)s.cell, (const int *)cell_row0_.p, (const int *)pk_off_lo_.p,
+           (const int *)s.cell, ppe_cells_.row0, (const int *)pk_off_lo_.p,
            (const int *)pk_off_up_.p, pk_val_lo_.p, pk_k_lo_.p, pk_val_up_.p, pk_k_up_.p, dinv_.p, err_.p);
     // packed cross-cell runs of the factor for the sweeps
     for (auto *v : {&xlen_lo_, &xlen_up_, &xp_lo_, &xp_up_, &xs_lo_, &xs_up_}) v->reserve((size_t)n_eq + 1);
@@ -1780,8 +1802,8 @@ void Engine<D>::factor_ic0()
     int nact = act_off_[ncol];
     adesc_.reserve((size_t)nact + 1);
     if (nact)
-        launch(k_cell_desc, nblk(nact, TPB), TPB, 0, st_, nact, (const int *)acells_.p,
-               (const int *)cell_row0_.p, (const int *)ucount_.p, adesc_.p, err_.p);
+        launch(k_cell_desc, nblk(nact, TPB), TPB, 0, st_, nact, ppe_cells_.act,
+               ppe_cells_.row0, ppe_cells_.count, adesc_.p, err_.p);
     if (ic_mode() != 0) {
         // the cross runs of each cell in jagged-diagonal order (k_sweep_cell, k_pcg)
         for (auto *v : {&jlen_, &jdc_lo_, &jdc_up_}) v->reserve((size_t)nact + 1);
@@ -1903,6 +1925,7 @@ void Engine<D>::ppe(bool clamp)
            (const int *)rs_.p, total, cell_row0_.p, row_of_.p, part_of_row_.p);
     launch(k_active_scatter, nblk(total, TPB), TPB, 0, st_, (const int *)ccells_.p, (const int *)ucol_.p,
            (const int *)apos_.p, total, acells_.p);
+    ppe_cells_ = {acells_.p, cell_row0_.p, ucount_.p};
     launch(k_ppe_sizes, 1, 1, 0, st_, (const int *)rs_.p, (const int *)apos_.p, (const int *)start_.p, total,
            (const int *)color_off_dev_.p, ncol, sizes_.p);
     MPS_CUDA(cudaMemcpyAsync(int_host_, sizes_.p, sizeof(int) * (2 * ncol + 4), cudaMemcpyDeviceToHost, st_));

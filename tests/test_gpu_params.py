@@ -3,7 +3,8 @@
 A refused change (a grid beyond 2^30 cells, or one the device has no memory
 for) leaves the parameters and the grid of before: the next search and step
 give the bits of a session that was never asked, the same change is refused
-again, and a change that can be made is made.
+again, and a change that can be made is made.  A changed domain forms no IC(0)
+factor; one asked for afterwards is the factor of the step before it.
 """
 import numpy as np
 import pytest
@@ -79,3 +80,26 @@ def test_refused_change_leaves_the_session_as_it_was(dim, why):
         s.neighbor_search()
         s.step(1)
         assert s.metrics()["converged"] == 1
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_changed_domain_forms_no_factor(precision):
+    _cuda()
+    got = []
+    for grow in (0, 1, 2):
+        with _session(3, precision=precision) as s:
+            s.step(1)
+            n0 = s.lib.mps_launch_count()
+            for _ in range(grow):
+                _domain(s, 3, 2.0)
+                _update(s)
+            assert s.lib.mps_launch_count() == n0
+            f = s.ic0()
+            r = np.random.default_rng(3).normal(size=len(f["b"]))
+            got.append((f, s.cell_blocks(), s.apply_preconditioner(r)))
+    for f, blocks, z in got[1:]:
+        for k in f:
+            assert np.array_equal(f[k], got[0][0][k]), k
+        for a, b in zip(blocks, got[0][1]):
+            assert np.array_equal(a, b)
+        assert np.array_equal(z, got[0][2])
