@@ -426,7 +426,7 @@ private:
 
     bool ppe_valid_ = false;
     bool ic0_valid_ = false;     // the last PPE was an ICCG one: its IC(0) factor can be had
-    bool ic0_built_ = false;     // the factor and its sweep tables have been formed
+    bool ic0_built_ = false;     // all of the factor, its sweep tables and their FP32 copies have been formed
     // the numbering of the last PPE's cells, which a factor formed later reads:
     // the grid's arrays, or copies once update_params has replaced the grid
     struct PpeCells {
@@ -1862,7 +1862,6 @@ void Engine<D>::factor_ic0()
     met.sweep_cross_lo = nx_lo_;
     met.sweep_cross_up = nx_up_;
     met.sweep_inverse_entries = ninv_;
-    ic0_built_ = true;
 }
 
 // FP32 copies of the IC(0) factor and its sweep data (mixed form): the cross
@@ -1908,6 +1907,7 @@ void Engine<D>::require_ic0()
     factor_ic0();
     if (last_fp32_) convert_ic0();
     check_err();
+    ic0_built_ = true;   // all of it: a failure above leaves it to the next call
 }
 
 // ---- PPE ------------------------------------------------------------------------
@@ -2013,6 +2013,7 @@ void Engine<D>::ppe(bool clamp)
     }
     launch(k_writeback<D>, nb, TPB, 0, st_, s, row_of_.p, x_.p, n, clamp);
     MPS_CUDA(cudaGetLastError());
+    ic0_built_ = icc && !ml_on_;
     ppe_valid_ = true;
 }
 
