@@ -359,7 +359,7 @@ private:
     // mixed form: residual reduction between reliable updates (MPS_RELIABLE_DELTA
     // overrides) and the SpMV of its inner loop (MPS_MIXED_SPMV): 0 the FP32
     // copy of A, 1 the FP64 matrix, 2 the FP32 copy in difference form
-    double rel_delta_ = kDelta;
+    double rel_delta_ = 0.0;   // MPS_RELIABLE_DELTA; 0: kDeltaMl or kDelta
     int mixed_spmv_ = 2;
     // CG-loop kernels launched as programmatic dependents (MPS_PDL_MASK): 2 the
     // colour sweep kernel, 4 SpMV and vector kernels
@@ -530,11 +530,16 @@ private:
     void convert_ic0();     // their FP32 copies
     void require_ic0();     // both, for callers that inspect them
     static constexpr int kMaxUpdates = 200;      // reliable updates of the mixed form, at most
-    // residual reduction between reliable updates (mixed form); measured at c2:
-    // 0.01 30.3 ms of solve, 0.001 28.9, 0.0001 26.9, 0.00001 27.6
-    static constexpr double kDelta = 0.0001;
-    static constexpr double kNear = 16.0;        // an inner solve that would end within this of the goal
-    static constexpr double kAim = 0.25;         // aims at this part of it instead
+    // Residual reduction between reliable updates (mixed form).  Multilevel
+    // form, dam break of 2.85 M particles: 30.3 ms of solve at 0.01, 28.9 at
+    // 0.001, 26.9 at 0.0001, 27.6 at 0.00001; an inner solve that would end
+    // within kNear of the goal aims at kAim of it instead, which saves it a
+    // whole stretch for a few iterations.  Where iterations come by the hundred
+    // that costs more than it saves (plain CG, 1.17 M particles: 1,713
+    // iterations of 0.176 ms instead of 1,626), so the other solves aim at the
+    // goal, at the interval measured for them.
+    static constexpr double kDelta = 0.01, kDeltaMl = 0.0001;
+    static constexpr double kNear = 16.0, kAim = 0.25;
     static constexpr double kStall = 0.5;        // a reliable update that does not halve the best true
     static constexpr int kMaxStalls = 2;         // residual is a stall; this many in a row end the solve
     static constexpr double kUnitRoundoff = 1.1102230246251565e-16;   // 2^-53
@@ -2439,7 +2444,7 @@ void Engine<D>::build_windows(bool fp32)
 // Mixed form: the ICCG with the matrix and the IC(0) factor stored in FP32
 // (the SpMV in difference form, k_cg_spmv<.., true>) and FP64 vectors and
 // arithmetic, with reliable updates.  Whenever the recursive residual has
-// fallen by rel_delta_ since the last update, the true residual r = b - A x
+// fallen by kDelta (kDeltaMl) since the last update, the true residual r = b - A x
 // is recomputed with the FP64 matrix and the iteration resumes from it with
 // its search direction kept.  Stops when ||b - A x|| <= max(cg_tolerance,
 // refine_tolerance ||b||, kFloor u || |b| + |A| |x| ||), u the FP64 unit
@@ -2480,10 +2485,14 @@ void Engine<D>::mixed_solve(int n_eq, long long nnz, bool icc, bool adjoint)
     if (mixed_spmv_ == 2) v.dsum = dsum_.p;   // the assembly's
     const double *zsrc = icc ? z_.p : r_.p;   // the preconditioned residual
     // tolerance of the next inner solve from a true residual `rn`: a reduction
-    // by rel_delta_, or, where that comes near the goal, well below it, since
-    // the true residual ends above the recursive one by its rounding
+    // by delta, or the goal; in the multilevel form, where that comes near the
+    // goal, well below it, since the true residual ends above the recursive one
+    // by its rounding
+    const bool ml = icc && ml_on_;
+    const double delta = rel_delta_ > 0.0 ? rel_delta_ : ml ? kDeltaMl : kDelta;
     auto aim = [&](double goal, double rn) {
-        double t = rel_delta_ * rn;
+        double t = delta * rn;
+        if (!ml) return std::max(goal, t);
         return t > kNear * goal ? t : kAim * goal;
     };
     if (rnorm > target) {

@@ -4,7 +4,8 @@ A step against the oracle's CG in 3-D and 2-D and both precision forms
 (pressure 1e-8, velocity 1e-10, position 1e-14 relative L2, as for a
 preconditioned step), and the mixed form's product from packed words: one
 launch fewer than from the separate arrays (MPS_PACK=0), which a conversion
-makes first, and the same bits.
+makes first, and the same bits.  Its reliable updates come every hundredfold
+fall of the residual, every ten thousandfold in the multilevel form.
 """
 import numpy as np
 import pytest
@@ -75,5 +76,26 @@ def test_mixed_product_reads_packed_words(dim, monkeypatch):
             iters.append(s.metrics()["ppe_iterations"])
     assert iters[0] == iters[1]
     assert launches[1] - launches[0] == 1
+    for f in ("pressure", "vel", "pos"):
+        assert np.array_equal(out[0][f], out[1][f]), f
+
+
+@pytest.mark.parametrize("solver,delta", [("0", "0.01"), ("1", "0.0001")])
+def test_interval_of_the_reliable_updates(solver, delta, monkeypatch):
+    _cuda()
+    from mps_b200.session import start
+    out, met = [], []
+    for env in (None, delta):
+        if env:
+            monkeypatch.setenv("MPS_RELIABLE_DELTA", env)
+        wl = _workload(3)
+        wl.params["solver_type"] = solver
+        with start(wl.config(), 3, T.HostParticles(3, wl.pos, wl.vel, wl.types), precision=1) as s:
+            s.step(1)
+            out.append(s.download())
+            met.append(s.metrics())
+    assert met[0]["converged"] == 1
+    for k in ("ppe_outer", "ppe_iterations"):
+        assert met[0][k] == met[1][k], k
     for f in ("pressure", "vel", "pos"):
         assert np.array_equal(out[0][f], out[1][f]), f
