@@ -272,9 +272,10 @@ private:
     bool structure_ = false;   // cell structure valid for S_[cur_]
     bool grid_ok_ = false;     // the grid's arrays are those of prm_ (false after a failed build_grid)
 
-    // storage of the arrays sized by the capacity, by the grid, and by a solve's
-    // grids (the last for the loop in one cluster)
-    DevGroup state_group_, grid_group_, ml_group_, ml_small_group_;
+    // storage of the arrays sized by the capacity, by the grid (the multilevel
+    // form's apart: other solves do without), and by a solve's grids (the last
+    // for the loop in one cluster)
+    DevGroup state_group_, grid_group_, ml_grid_group_, ml_group_, ml_small_group_;
 
     // ---- sort
     DevArray<int> kcell_, count_, start_, excl_, exoff_, tmp_, perm_, where_, scanws_;
@@ -416,8 +417,9 @@ private:
     DevArray<double> mlcm_, mlB_, mlA_, mlC_, mldinv_, mlb_, mlx_, mly_, mlbd_, mlM_[2], mlMC_, mlcsum_, jdinv_;
     const double *mlM_last_ = nullptr;     // the dense V-cycle of the current solve
     void ml_levels();
+    bool ml_grids();
     void ml_nodes(int nact);
-    void ml_build(int n_eq);
+    bool ml_build(int n_eq);
     MlVecs ml_vecs() const;
     const double *ml_result() const { return ml_ld_ == 0 ? mlx_.p : mly_.p; }
     void ml_update(bool restrict_only, double *x, double *r, const double *p, const double *Ap);
@@ -753,16 +755,12 @@ void Engine<D>::build_grid()
     re_list_ = list_radius(prm_);
     ml_levels();
     grid_group_.reserve([&](auto add) {
-        size_t t = (size_t)total, mt = (size_t)ml_total_;
+        size_t t = (size_t)total;
         add(count_, 2 * (t + 1));   // and the scatter's cursors
         add(start_, t + 2);
         for (auto *v : {&ucount_, &ucol_, &cell_row0_, &ccells_}) add(*v, t);
         for (auto *v : {&rs_, &aflag_, &apos_, &acells_}) add(*v, t + 1);
         add(scanws_, scan_workspace((int)total + 1) + scan_workspace(std::max((int)total, cap_) + 1) + 64);   // a pair's
-        add(mlscan_, scan_workspace(ml_total_ + 1));
-        for (auto *v : {&mlflag_, &mlpos_, &mlmap_, &mlact_}) add(*v, mt + 1);
-        for (auto *v : {&mlcnode_, &mlcell_}) add(*v, t + 1);
-        for (auto *v : {&mlb_, &mlx_, &mly_}) add(*v, mt);
     });
     g_.start = start_.p;
 
@@ -817,6 +815,35 @@ void Engine<D>::ml_levels()
         for (int d = 0; d < D; d++) n[d] = n[d] / 2 + 1;
     }
     ml_total_ = (int)first;
+}
+
+// `reserve` with the device's refusal of memory as false: a solve that cannot
+// have the multilevel form's arrays takes IC(0), as on a grid too large for it.
+template <class Reserve>
+static bool memory_for(Reserve reserve)
+{
+    try {
+        reserve();
+    } catch (const CudaError &e) {
+        if (e.code != MPS_ERR_OOM) throw;
+        return false;
+    }
+    return true;
+}
+
+// The arrays of the nested grids' boxes, on the first solve that uses them.
+template <int D>
+bool Engine<D>::ml_grids()
+{
+    return memory_for([&] {
+        ml_grid_group_.reserve([&](auto add) {
+            size_t t = (size_t)g_.total, mt = (size_t)ml_total_;
+            add(mlscan_, scan_workspace(ml_total_ + 1));
+            for (auto *v : {&mlflag_, &mlpos_, &mlmap_, &mlact_}) add(*v, mt + 1);
+            for (auto *v : {&mlcnode_, &mlcell_}) add(*v, t + 1);
+            for (auto *v : {&mlb_, &mlx_, &mly_}) add(*v, mt);
+        });
+    });
 }
 
 // Constants evaluated with the reference's expressions.
@@ -1475,9 +1502,9 @@ MlVecs Engine<D>::ml_vecs() const
 }
 
 // P, the Galerkin operators and their smoother factors for the current
-// matrix and right-hand side.
+// matrix and right-hand side; false where the device has no memory for them.
 template <int D>
-void Engine<D>::ml_build(int n_eq)
+bool Engine<D>::ml_build(int n_eq)
 {
     using L = MlDim<D>;
     State<D> &s = S();
@@ -1510,7 +1537,7 @@ void Engine<D>::ml_build(int n_eq)
         msize = std::max(msize, nf * nf);
         mcsize = std::max(mcsize, nf * nc);
     }
-    ml_group_.reserve([&](auto add) {
+    auto arrays = [&](auto add) {
         size_t n1 = na1, n = nall, a = nact;
         add(mlncell_, L::NC * n1);
         add(mlcm_, a * L::NC * L::W4);
@@ -1525,7 +1552,8 @@ void Engine<D>::ml_build(int n_eq)
         add(mlpar_, n);
         for (auto &m : mlM_) add(m, msize);
         add(mlMC_, mcsize);
-    });
+    };
+    if (!memory_for([&] { ml_group_.reserve(arrays); })) return false;
     const int *rp = row_ptr_.p, *dp = diagpos_.p, *ci = col_.p;
     const double *A = A_.p;
     adesc_.reserve((size_t)nact + 1);
@@ -1573,18 +1601,21 @@ void Engine<D>::ml_build(int n_eq)
     mlM_last_ = mlM_[cur].p;
     ml_small_ = n_eq <= ml_small_rows_ && (ml_ld_ == 0 || (ml_ld_ == 1 && ml_add_)) &&
                 sizeof(double) * ml_small_vectors() <= ML_CL_SMEM && ml_clusters() > 0;
-    if (ml_small_) {
-        int nd = mlc_.lo[ml_ld_ + 1] - mlc_.lo[ml_ld_];
-        ml_small_group_.reserve([&](auto add) {
-            add(mlcellnode_, (size_t)nact * L::NC);
-            add(mlfine_, (size_t)nd * L::CELLS);
-            add(mlparent_, (size_t)na1 * L::NC);
+    const int nd = mlc_.lo[ml_ld_ + 1] - mlc_.lo[ml_ld_];
+    if (ml_small_)
+        ml_small_ = memory_for([&] {
+            ml_small_group_.reserve([&](auto add) {
+                add(mlcellnode_, (size_t)nact * L::NC);
+                add(mlfine_, (size_t)nd * L::CELLS);
+                add(mlparent_, (size_t)na1 * L::NC);
+            });
         });
+    if (ml_small_)
         launch(k_ml_small_tables<D>, nblk(std::max(nact, std::max(na1, nd)), TPB), TPB, 0, st_, nact, na1, nd, ml_add_,
                mlc_.g[0], mlc_.g[ml_ld_], (const int *)mlcnode_.p, (const int *)mlmap_.p, (const int *)mlunder_.p,
                (const int *)mlabove_.p, (const unsigned char *)mlpar_.p, mlcellnode_.p, mlfine_.p, mlparent_.p);
-    }
     MPS_CUDA(cudaGetLastError());
+    return true;
 }
 
 // The attributes of a launch of the cluster loop, one cluster.
@@ -1961,7 +1992,7 @@ void Engine<D>::ppe(bool clamp)
         ppe_valid_ = true;
         return;
     }
-    ml_on_ = prm_.solver_type == 1 && sweep_mode_ == 3 && ml_total_ > 0;
+    ml_on_ = prm_.solver_type == 1 && sweep_mode_ == 3 && ml_total_ > 0 && ml_grids();
     if (ml_on_) ml_nodes(act_off_[ncol]);
     NbrSource<D> src = near();
     launch(k_row_count<D>, nblk(n_eq, ROW_BLOCK), ROW_BLOCK, 0, st_, src, s, (const int *)part_of_row_.p,
@@ -1994,8 +2025,8 @@ void Engine<D>::ppe(bool clamp)
     MPS_CUDA(cudaEventRecord(ev_[2], st_));
     ic0_valid_ = icc;
     ic0_built_ = false;
-    if (icc && ml_on_) ml_build(n_eq);
-    else if (icc) factor_ic0();
+    if (icc && ml_on_) ml_on_ = ml_build(n_eq);
+    if (icc && !ml_on_) factor_ic0();
     MPS_CUDA(cudaEventRecord(ev_[3], st_));
 
     last_fp32_ = prm_.precision == MPS_PREC_MIXED;
