@@ -33,3 +33,9 @@ def test_cell_offsets_at_tile_edges(cells):
     assert np.array_equal(got_cell, cell)
     assert np.array_equal(start, np.concatenate([[0], np.cumsum(np.bincount(cell, minlength=cells))]))
     assert np.array_equal(order, np.lexsort((-np.arange(n), cell)))
+
+
+@pytest.mark.parametrize("cells", [10239, 10240, 10241])
+def test_cell_offsets_at_long_tile_edges(cells):
+    """Scans above 8,192 elements go by tiles of 2,048."""
+    test_cell_offsets_at_tile_edges(cells)
