@@ -440,6 +440,11 @@ def run_b200(args, rank: int, world: int, local_rank: int):
         for f in forms:
             pm = res[f]["pmet"]
             fp32 = f == "mixed"
+            if pm.get("prof_pcg_launches", 0) > 0 and pm["sweep_inverse_entries"] == 0:
+                # the multilevel form's loop in one cluster, its matrix in shared memory: no HBM roofline
+                kern[f] = {"k_ml_small_ms_per_iteration": pm["prof_pcg_ms"] / max(pm["prof_pcg_iterations"], 1),
+                           "k_ml_small_iterations_per_launch": pm["prof_pcg_iterations"] / pm["prof_pcg_launches"]}
+                continue
             if pm.get("prof_pcg_launches", 0) > 0:
                 # persistent ICCG kernel: one launch per batch of iterations
                 ipl = pm["prof_pcg_iterations"] / pm["prof_pcg_launches"]
@@ -488,7 +493,7 @@ def run_b200(args, rank: int, world: int, local_rank: int):
                              "frac": spmv_b / (spmv_ms / 1e3) / 1e9 / peak,
                              "traffic": None if tsp is None else tsp[0] / tsp[1] * spmv_b,
                              "algorithmic_bytes_per_launch": spmv_b, "ms_per_launch": spmv_ms})
-        top = dict(roof[0])
+        top = dict(roof[0]) if roof else {}
         top.update({"peak_source": f"{peak_kind} hbm_gbs",
                     "timing": "CUDA events on the library stream around every launch of the ICCG loop's kernels "
                               "(k_pcg: one launch per batch of iterations; the launch-per-colour form: every colour "

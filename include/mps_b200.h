@@ -127,8 +127,9 @@ typedef struct {
     double ms_solve;
     /* Per-kernel device time summed over the session while profiling is on
      * (mps_set_profiling): the SpMV of the CG loop, the forward and backward
-     * colour sweeps of the IC(0) preconditioner, and the CG vector kernels;
-     * only iterations that did work are counted. */
+     * colour sweeps of the IC(0) preconditioner, and the CG vector kernels
+     * (with the multilevel preconditioner, its application among them); only
+     * iterations that did work are counted. */
     double prof_spmv_ms;
     long long prof_spmv_launches;
     double prof_fwd_ms;
@@ -149,13 +150,16 @@ typedef struct {
     double ppe_rounding_floor;
     /* Sizes of the last step's IC(0) sweep data: cross-cell entries of the
      * factor read by the forward and the backward sweep, and the entries of
-     * the in-cell block inverses (read once per sweep). */
+     * the in-cell block inverses (read once per sweep); 0 while a session's
+     * solves have needed no factor. */
     long long sweep_cross_lo;
     long long sweep_cross_up;
     long long sweep_inverse_entries;
-    /* Device time of the persistent ICCG kernel (one cooperative launch per
-     * batch of CG iterations) summed over the session while profiling is
-     * on, its launches and the iterations they ran. */
+    /* Device time of the kernels that run the CG loop themselves (the
+     * persistent ICCG kernel, one cooperative launch per batch of iterations;
+     * with the multilevel preconditioner, small systems' loop in one cluster)
+     * summed over the session while profiling is on, their launches and the
+     * iterations they ran. */
     double prof_pcg_ms;
     long long prof_pcg_launches;
     long long prof_pcg_iterations;
@@ -266,7 +270,8 @@ unsigned long long mps_launch_count(void);
  * 0 when surface tension is off.  Host arithmetic, no device needed. */
 int  mps_surface_tension_coeffs(const mps_params_t *params, double *c_ll, double *c_sl);
 
-/* Per-kernel timing of the CG loop with CUDA events (adds no host sync). */
+/* Per-kernel timing of the CG loop with CUDA events: the same kernels and the
+ * same results as without, and no host sync. */
 int  mps_set_profiling(mps_session *s, int on);
 /* Zero the accumulated metrics. */
 int  mps_reset_metrics(mps_session *s);

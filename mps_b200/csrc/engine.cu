@@ -504,6 +504,7 @@ private:
     void sort();
     void unsort();
     void ppe(bool clamp);
+    void prof_loop(int worked, int n_eq, long long nnz);
     template <class TM>
     void pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc, int n_eq, long long nnz,
                    const double *zprev = nullptr);
@@ -2145,6 +2146,21 @@ void Engine<D>::run_sweep(const PcgBufs<TM> &v, bool fwdir)
     }
 }
 
+// Adds a launch that ran `worked` iterations between pev_[0] and pev_[1] to
+// the profiling metrics.
+template <int D>
+void Engine<D>::prof_loop(int worked, int n_eq, long long nnz)
+{
+    float ms = 0;
+    cudaEventElapsedTime(&ms, pev_[0], pev_[1]);
+    met.prof_pcg_ms += ms;
+    met.prof_pcg_launches += 1;
+    met.prof_pcg_iterations += worked;
+    met.prof_iterations += worked;
+    met.prof_nnz_sum += (long long)worked * nnz;
+    met.prof_rows_sum += (long long)worked * n_eq;
+}
+
 // PCG of pressure_solver.c:261-322 (CG of :90-131 when icc is false) on the
 // block-colour system, values and vectors of type T, dot products in FP64.
 // r is initialised from v.b (which may alias r); stops at sqrt(r.r) < tol,
@@ -2158,10 +2174,17 @@ void Engine<D>::pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc,
     using T = double;
     const int RB = red_grid(n_eq, CG_BLOCK);
     int iter_before = 0;
-    if (icc && ml_on_ && ml_small_ && !profiling && ml_small_solve<TM>(v, tol, maxit, zprev)) {
-        MPS_CUDA(cudaMemcpyAsync(sc_host_, sc_.p, sizeof(CGScalars), cudaMemcpyDeviceToHost, st_));
-        MPS_CUDA(cudaStreamSynchronize(st_));
-        return;
+    if (icc && ml_on_ && ml_small_) {
+        const bool prof = profiling;
+        if (zprev) iter_before = sc_host_->iter;
+        if (prof) MPS_CUDA(cudaEventRecord(pev_[0], st_));
+        if (ml_small_solve<TM>(v, tol, maxit, zprev)) {
+            if (prof) MPS_CUDA(cudaEventRecord(pev_[1], st_));
+            MPS_CUDA(cudaMemcpyAsync(sc_host_, sc_.p, sizeof(CGScalars), cudaMemcpyDeviceToHost, st_));
+            MPS_CUDA(cudaStreamSynchronize(st_));
+            if (prof) prof_loop(sc_host_->iter - iter_before, n_eq, nnz);
+            return;
+        }
     }
     if (!zprev) {
         CGScalars init{};
@@ -2248,16 +2271,9 @@ void Engine<D>::pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc,
             if (int_host_[60]) check_err();
             int worked = sc_host_->iter - iter_before;
             if (prof) {
-                float ms = 0;
-                cudaEventElapsedTime(&ms, pev_[0], pev_[1]);
-                met.prof_pcg_ms += ms;
-                met.prof_pcg_launches += 1;
-                met.prof_pcg_iterations += worked;
-                met.prof_iterations += worked;
-                met.prof_nnz_sum += (long long)worked * nnz;
-                met.prof_rows_sum += (long long)worked * n_eq;
+                prof_loop(worked, n_eq, nnz);
+                trace_phases(worked);
             }
-            if (prof) trace_phases(worked);
             iter_before = sc_host_->iter;
             if (sc_host_->done) break;
         }
