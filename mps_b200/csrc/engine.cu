@@ -363,8 +363,14 @@ private:
     double rel_delta_ = 0.0;   // MPS_RELIABLE_DELTA; 0: kDeltaMl or kDelta
     int mixed_spmv_ = 2;
     // CG-loop kernels launched as programmatic dependents (MPS_PDL_MASK): 2 the
-    // colour sweep kernel, 4 SpMV and vector kernels
+    // preconditioner's (colour sweeps, V-cycle), 4 SpMV and vector kernels
     int pdl_mask_ = 6;
+    template <class Kern, class... Args>
+    void launch_loop(int bit, Kern kern, dim3 g, dim3 b, size_t sm, Args... args)
+    {
+        if (pdl_mask_ & bit) launch_pdl(kern, g, b, sm, st_, args...);
+        else launch(kern, g, b, sm, st_, args...);
+    }
     // entries per window of the staged in-cell sweep: MPS_CELL_WIN (256..4096)
     // if set, else 8 KB of inverse entries (1,024 FP64, 2,048 in the mixed
     // form's FP32 sweeps); win_ is the window of the current tables
@@ -1725,10 +1731,9 @@ template <int D>
 void Engine<D>::ml_update(bool restrict_only, double *x, double *r, const double *p, const double *Ap)
 {
     int nact = act_off_[1 << D];
-    launch_pdl(restrict_only ? k_ml_update<D, true> : k_ml_update<D, false>, red_grid(nact, CG_BLOCK / 32), CG_BLOCK,
-               0, st_, nact,
-               (const int2 *)adesc_.p, (const float *)mlfrac_.p, cap_, x, r, p, Ap, mlcsum_.p, partials_.p, ticket_.p,
-               sc_.p);
+    launch_loop(4, restrict_only ? k_ml_update<D, true> : k_ml_update<D, false>, red_grid(nact, CG_BLOCK / 32),
+                CG_BLOCK, 0, nact, (const int2 *)adesc_.p, (const float *)mlfrac_.p, cap_, x, r, p, Ap, mlcsum_.p,
+                partials_.p, ticket_.p, sc_.p);
 }
 
 // The V-cycle: one launch down and one up per grid above the dense one.
@@ -1739,24 +1744,24 @@ void Engine<D>::ml_cycle()
     const CGScalars *sc = sc_.p;
     const int *lo = mlc_.lo;
     int ld = ml_ld_;
-    launch_pdl(k_ml_nodes1<D>, nblk(v.na1, CG_BLOCK), CG_BLOCK, 0, st_, v, sc);
+    launch_loop(2, k_ml_nodes1<D>, nblk(v.na1, CG_BLOCK), CG_BLOCK, 0, v, sc);
     for (int l = 0; l < ld; l++) {
         int nc = lo[l + 2] - lo[l + 1], nf = lo[l + 1] - lo[l];
         if (ml_add_ && l == 0)
-            launch_pdl(k_ml_add_down<D>, nblk(nc, CG_BLOCK), CG_BLOCK, 0, st_, v, mlc_.g[0], lo[1], lo[2], sc);
+            launch_loop(2, k_ml_add_down<D>, nblk(nc, CG_BLOCK), CG_BLOCK, 0, v, mlc_.g[0], lo[1], lo[2], sc);
         else
-            launch_pdl(k_ml_down<D>, nblk(nc, CG_BLOCK / 32) + nblk(nf, CG_BLOCK / 8), CG_BLOCK, 0, st_, v, mlc_.g[l],
-                       l, lo[l], lo[l + 1], lo[l + 2], sc);
+            launch_loop(2, k_ml_down<D>, nblk(nc, CG_BLOCK / 32) + nblk(nf, CG_BLOCK / 8), CG_BLOCK, 0, v,
+                        mlc_.g[l], l, lo[l], lo[l + 1], lo[l + 2], sc);
     }
     int nd = lo[ld + 1] - lo[ld];
-    launch_pdl(k_ml_matvec, nblk(nd, CG_BLOCK / 32), CG_BLOCK, 0, st_, v, lo[ld], nd, sc);
+    launch_loop(2, k_ml_matvec, nblk(nd, CG_BLOCK / 32), CG_BLOCK, 0, v, lo[ld], nd, sc);
     for (int l = ld - 1; l >= 0; l--) {
         const double *cx = l + 1 == ld ? v.x : v.y;
         int nf = lo[l + 1] - lo[l];
         if (ml_add_ && l == 0)
-            launch_pdl(k_ml_add_up<D>, nblk(nf, CG_BLOCK), CG_BLOCK, 0, st_, v, mlc_.g[1], cx, sc);
+            launch_loop(2, k_ml_add_up<D>, nblk(nf, CG_BLOCK), CG_BLOCK, 0, v, mlc_.g[1], cx, sc);
         else
-            launch_pdl(k_ml_up<D>, nblk(nf, CG_BLOCK / 8), CG_BLOCK, 0, st_, v, mlc_.g[l + 1], lo[l], nf, cx, sc);
+            launch_loop(2, k_ml_up<D>, nblk(nf, CG_BLOCK / 8), CG_BLOCK, 0, v, mlc_.g[l + 1], lo[l], nf, cx, sc);
     }
 }
 
@@ -1765,10 +1770,9 @@ template <int D>
 void Engine<D>::ml_prolong(bool rz, const double *r, double *z)
 {
     int nact = act_off_[1 << D];
-    launch_pdl(rz ? k_ml_prolong<D, true> : k_ml_prolong<D, false>, red_grid(nact, CG_BLOCK / 32), CG_BLOCK, 0, st_,
-               nact,
-               (const int2 *)adesc_.p, (const int *)mlcnode_.p, ml_.g[0], (const float *)mlfrac_.p, cap_,
-               (const double *)jdinv_.p, r, z, ml_result(), partials_.p, ticket_.p, sc_.p);
+    launch_loop(2, rz ? k_ml_prolong<D, true> : k_ml_prolong<D, false>, red_grid(nact, CG_BLOCK / 32), CG_BLOCK, 0,
+                nact, (const int2 *)adesc_.p, (const int *)mlcnode_.p, ml_.g[0], (const float *)mlfrac_.p, cap_,
+                (const double *)jdinv_.p, r, z, ml_result(), partials_.p, ticket_.p, sc_.p);
 }
 
 // The IC(0) factor of the current matrix, colour by colour, and the tables
@@ -2067,10 +2071,7 @@ void Engine<D>::run_sweep(const PcgBufs<TM> &v, bool fwdir)
 {
     using T = double;
     int ncol = 1 << D;
-    auto lk = [&](int bit, auto kern, dim3 g, dim3 b, size_t sm, auto... args) {
-        if (pdl_mask_ & bit) launch_pdl(kern, g, b, sm, st_, args...);
-        else launch(kern, g, b, sm, st_, args...);
-    };
+    auto lk = [&](auto... args) { launch_loop(args...); };
     {
         const T *rhs = fwdir ? v.r : v.y;
         T *out = fwdir ? v.y : v.z;
@@ -2198,11 +2199,7 @@ void Engine<D>::pcg_solve(const PcgBufs<TM> &v, double tol, int maxit, bool icc,
         MPS_CUDA(cudaMemsetAsync(&sc_.p->done, 0, sizeof(int), st_));
     }
     T *z = icc ? v.z : v.r;
-    // CG-loop launch: as a programmatic dependent when its group's bit is in pdl_mask_
-    auto lk = [&](int bit, auto kern, dim3 g, dim3 b, size_t sm, auto... args) {
-        if (pdl_mask_ & bit) launch_pdl(kern, g, b, sm, st_, args...);
-        else launch(kern, g, b, sm, st_, args...);
-    };
+    auto lk = [&](auto... args) { launch_loop(args...); };
     auto sweep = [&](bool fwdir) { run_sweep<TM>(v, fwdir); };
     const int lpr = spmv_lpr_ ? spmv_lpr_ : (sizeof(TM) == 8 ? 8 : 16);
     const int SB = red_grid(n_eq, CG_BLOCK / lpr);

@@ -43,3 +43,28 @@ def test_profiling_changes_nothing(loop, precision, monkeypatch):
     whole = loop in ("cluster", "persistent")
     assert (m["prof_pcg_iterations"], m["prof_pcg_launches"] > 0) == (m["total_iterations"] if whole else 0, whole)
     assert (m["prof_pcg_ms"] > 0.0) == whole and (m["prof_vec_ms"] > 0.0) != whole
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("form", ["add", "mult", "dense"])
+def test_serial_launches_give_the_same_bits(form, precision, monkeypatch):
+    """The multilevel loop's launches one after the other (MPS_PDL_MASK=0) and
+    as programmatic dependents: whole (6), and either group alone."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from mps_b200.session import start
+    wl = W.dambreak("c1", l0=0.02, seed=4)
+    monkeypatch.setenv("MPS_ML_SMALL", "0")
+    monkeypatch.setenv("MPS_ML_ADD", "1000000" if form == "add" else "0")
+    monkeypatch.setenv("MPS_ML_DENSE", "1024" if form == "dense" else "64")
+    out = []
+    for mask in ("6", "0", "2", "4"):
+        monkeypatch.setenv("MPS_PDL_MASK", mask)
+        with start(wl.config(), 3, T.HostParticles(3, wl.pos, wl.vel, wl.types), precision=precision) as s:
+            s.step(2)
+            out.append((s.download(), s.metrics()["total_iterations"]))
+    for g, it in out[1:]:
+        assert it == out[0][1]
+        for f in ("pos", "vel", "pressure"):
+            assert np.array_equal(g[f], out[0][0][f]), f
