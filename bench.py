@@ -394,6 +394,20 @@ def pcg_iter_bytes(pmet, fp32: bool, diff: bool) -> float:
     return spmv + fwd + bwd + 12.0 * e
 
 
+def cpu_baseline(args):
+    """The reference on the host cores beside the GPU's line; None with --no-cpu
+    and where it has not been built."""
+    if args.no_cpu:
+        return None
+    try:
+        v, sec, meta = reference_cpu_steps(args.workload, args.cpu_steps, 0, l0=args.l0, restart=args.restart)
+    except FileNotFoundError as e:
+        print(f"cpu_baseline: the reference build {e} is absent", file=sys.stderr)
+        return None
+    return {"value": v, "unit": UNIT, "cores": meta["cores"], "kind": meta["kind"], "sample": meta["sample"],
+            "seconds_per_step": sec}
+
+
 def run_b200(args, rank: int, world: int, local_rank: int):
     import numpy as np
     import torch
@@ -476,8 +490,11 @@ def run_b200(args, rank: int, world: int, local_rank: int):
             sb = sweep_bytes(pm, fp32)
             sw_b = 0.5 * (sb["forward"] + sb["backward"])
             sw_ms = 0.5 * (fwd_ms + bwd_ms)
-            kern[f] = {"k_cg_spmv_ms": spmv_ms, "ic0_forward_sweep_ms(8 colour launches)": fwd_ms,
-                       "ic0_backward_sweep_ms(8 colour launches)": bwd_ms, "cg_axpy_ms": vec_ms}
+            if pm["prof_fwd_sweeps"]:
+                kern[f] = {"k_cg_spmv_ms": spmv_ms, "ic0_forward_sweep_ms(8 colour launches)": fwd_ms,
+                           "ic0_backward_sweep_ms(8 colour launches)": bwd_ms, "cg_axpy_ms": vec_ms}
+            else:
+                kern[f] = {"k_cg_spmv_ms": spmv_ms, "update_and_multilevel_cycle_ms": vec_ms}
             tsw = ncu_traffic("k_sweep_colour", f)
             tsp = ncu_traffic("k_cg_spmv", f)
             if sw_ms > 0:
@@ -499,11 +516,7 @@ def run_b200(args, rank: int, world: int, local_rank: int):
                               "(k_pcg: one launch per batch of iterations; the launch-per-colour form: every colour "
                               "sweep and SpMV), over min(steps, 2) profiled steps right after the timed region",
                     "others": roof[1:]})
-        cpu = None
-        if world == 1 and not args.no_cpu:
-            v, sec, meta = reference_cpu_steps(args.workload, args.cpu_steps, 0, l0=args.l0, restart=args.restart)
-            cpu = {"value": v, "unit": UNIT, "cores": meta["cores"], "kind": meta["kind"], "sample": meta["sample"],
-                   "seconds_per_step": sec}
+        cpu = cpu_baseline(args) if world == 1 else None
         forms_out = {}
         for f in forms:
             r = res[f]
@@ -1003,7 +1016,12 @@ def main():
         if rank != 0:
             return 0
         nsteps = min(args.steps, REF_WINDOW)
-        v, sec, meta = reference_cpu_steps(args.workload, nsteps, 0, l0=args.l0, restart=args.restart)
+        try:
+            v, sec, meta = reference_cpu_steps(args.workload, nsteps, 0, l0=args.l0, restart=args.restart)
+        except FileNotFoundError as e:
+            print(json.dumps({"impl": "reference",
+                              "unavailable": f"the reference build {os.path.relpath(str(e), ROOT)} is absent"}))
+            return 0
         meta["sample"] += (f"; a bounded window of {nsteps} step(s) instead of {args.steps} after {args.warmup} "
                            "warm-up (no warm-up: the reference allocates its PPE buffers in every call)")
         line = {"metric": METRIC, "value": v, "unit": UNIT, "n_gpus": world, "steps": args.steps,
