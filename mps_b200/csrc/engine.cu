@@ -273,9 +273,10 @@ private:
     bool grid_ok_ = false;     // the grid's arrays are those of prm_ (false after a failed build_grid)
 
     // storage of the arrays sized by the capacity, by the grid (the multilevel
-    // form's apart: other solves do without), and by a solve's grids (the last
-    // for the loop in one cluster)
+    // form's apart where the session was not made for it), and by a solve's
+    // grids (the last for the loop in one cluster)
     DevGroup state_group_, grid_group_, ml_grid_group_, ml_group_, ml_small_group_;
+    bool ml_in_grid_ = false;   // grid_group_ holds the multilevel form's arrays too
 
     // ---- sort
     DevArray<int> kcell_, count_, start_, excl_, exoff_, tmp_, perm_, where_, scanws_;
@@ -422,7 +423,10 @@ private:
     DevArray<float> mlfrac_;
     DevArray<double> mlcm_, mlB_, mlA_, mlC_, mldinv_, mlb_, mlx_, mly_, mlbd_, mlM_[2], mlMC_, mlcsum_, jdinv_;
     const double *mlM_last_ = nullptr;     // the dense V-cycle of the current solve
+    bool ml_wanted() const { return prm_.solver_type == 1 && sweep_mode_ == 3 && ml_total_ > 0; }
     void ml_levels();
+    template <class Add>
+    void ml_grid_arrays(Add add);
     bool ml_grids();
     void ml_nodes(int nact);
     bool ml_build(int n_eq);
@@ -733,6 +737,20 @@ void Engine<D>::alloc_state()
     }
 }
 
+// `reserve` with the device's refusal of memory as false: a solve that cannot
+// have the multilevel form's arrays takes IC(0), as on a grid too large for it.
+template <class Reserve>
+static bool memory_for(Reserve reserve)
+{
+    try {
+        reserve();
+    } catch (const CudaError &e) {
+        if (e.code != MPS_ERR_OOM) throw;
+        return false;
+    }
+    return true;
+}
+
 // cell_list_create (neighbor_search.c:92-122) with cell size = list radius:
 // origin, cells per direction and in all of the grid that `p` asks for.
 template <int D>
@@ -761,14 +779,26 @@ void Engine<D>::build_grid()
     g_ = g;
     re_list_ = list_radius(prm_);
     ml_levels();
-    grid_group_.reserve([&](auto add) {
+    auto own = [&](auto add) {
         size_t t = (size_t)total;
         add(count_, 2 * (t + 1));   // and the scatter's cursors
         add(start_, t + 2);
         for (auto *v : {&ucount_, &ucol_, &cell_row0_, &ccells_}) add(*v, t);
         for (auto *v : {&rs_, &aflag_, &apos_, &acells_}) add(*v, t + 1);
         add(scanws_, scan_workspace((int)total + 1) + scan_workspace(std::max((int)total, cap_) + 1) + 64);   // a pair's
-    });
+    };
+    // with the multilevel form's arrays where the session is made for it: a
+    // second allocation would cost its first step 0.3 ms
+    auto both = [&](auto add) {
+        own(add);
+        ml_grid_arrays(add);
+    };
+    bool with_ml = ml_wanted() && memory_for([&] { grid_group_.reserve(both); });
+    if (!with_ml) {
+        if (ml_in_grid_) ml_grid_arrays([](auto &a, size_t) { a.place(nullptr, 0); });
+        grid_group_.reserve(own);
+    }
+    ml_in_grid_ = with_ml;
     g_.start = start_.p;
 
     // cells sorted by (colour, linear index)
@@ -824,33 +854,23 @@ void Engine<D>::ml_levels()
     ml_total_ = (int)first;
 }
 
-// `reserve` with the device's refusal of memory as false: a solve that cannot
-// have the multilevel form's arrays takes IC(0), as on a grid too large for it.
-template <class Reserve>
-static bool memory_for(Reserve reserve)
+// The arrays of the nested grids' boxes: add(array, elements) for each.
+template <int D>
+template <class Add>
+void Engine<D>::ml_grid_arrays(Add add)
 {
-    try {
-        reserve();
-    } catch (const CudaError &e) {
-        if (e.code != MPS_ERR_OOM) throw;
-        return false;
-    }
-    return true;
+    size_t t = (size_t)g_.total, mt = (size_t)ml_total_;
+    add(mlscan_, scan_workspace(ml_total_ + 1));
+    for (auto *v : {&mlflag_, &mlpos_, &mlmap_, &mlact_}) add(*v, mt + 1);
+    for (auto *v : {&mlcnode_, &mlcell_}) add(*v, t + 1);
+    for (auto *v : {&mlb_, &mlx_, &mly_}) add(*v, mt);
 }
 
-// The arrays of the nested grids' boxes, on the first solve that uses them.
+// Has them for a solve; false where the device has no memory for them.
 template <int D>
 bool Engine<D>::ml_grids()
 {
-    return memory_for([&] {
-        ml_grid_group_.reserve([&](auto add) {
-            size_t t = (size_t)g_.total, mt = (size_t)ml_total_;
-            add(mlscan_, scan_workspace(ml_total_ + 1));
-            for (auto *v : {&mlflag_, &mlpos_, &mlmap_, &mlact_}) add(*v, mt + 1);
-            for (auto *v : {&mlcnode_, &mlcell_}) add(*v, t + 1);
-            for (auto *v : {&mlb_, &mlx_, &mly_}) add(*v, mt);
-        });
-    });
+    return memory_for([&] { ml_grid_group_.reserve([&](auto add) { ml_grid_arrays(add); }); });
 }
 
 // Constants evaluated with the reference's expressions.
@@ -1997,7 +2017,7 @@ void Engine<D>::ppe(bool clamp)
         ppe_valid_ = true;
         return;
     }
-    ml_on_ = prm_.solver_type == 1 && sweep_mode_ == 3 && ml_total_ > 0 && ml_grids();
+    ml_on_ = ml_wanted() && ml_grids();
     if (ml_on_) ml_nodes(act_off_[ncol]);
     NbrSource<D> src = near();
     launch(k_row_count<D>, nblk(n_eq, ROW_BLOCK), ROW_BLOCK, 0, st_, src, s, (const int *)part_of_row_.p,

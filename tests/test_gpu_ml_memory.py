@@ -61,10 +61,10 @@ def test_plain_cg_holds_no_nested_grids(dim):
 
 
 @pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("what", ["grids", "operators"])
+@pytest.mark.parametrize("what", ["grids", "grids of a new session", "operators"])
 def test_refused_memory_falls_back_to_ic0(what, precision, monkeypatch):
     torch = _torch()
-    if what == "grids":
+    if what != "operators":
         wl, room = _wide(3, 4.0e7), 1024 * MB      # the grids' arrays take 40 bytes a node and more
     else:
         # wall particles beyond each other's reach, a cell each, around the dam: 4 kB a cell and 2 kB
@@ -84,6 +84,17 @@ def test_refused_memory_falls_back_to_ic0(what, precision, monkeypatch):
         s.step(1)   # multilevel
         got, m = s.download(), s.metrics()
         assert m["converged"] == 1 and m["ppe_iterations"] != met["ppe_iterations"]
+    if what == "grids of a new session":   # its own grid takes 2.2 GB, these 2.4 more
+        held = torch.empty(_free(torch) - 3500 * MB, dtype=torch.uint8, device="cuda")
+        with _start(wl, precision=precision) as s:
+            s.step(1)
+            got, m = s.download(), s.metrics()
+        del held
+        torch.cuda.empty_cache()
+        assert m["converged"] == 1 and m["ppe_iterations"] == met["ppe_iterations"]
+        for f in FIELDS:
+            assert np.array_equal(got[f], want[f]), f
+        return
     wl.params["solver_type"] = "0"
     with _start(wl, precision=precision) as s:
         ck = torch.empty(s.state_bytes(), dtype=torch.uint8, device="cuda")
