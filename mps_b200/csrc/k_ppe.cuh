@@ -161,10 +161,11 @@ __global__ void k_offgrid_rows(State<D> s, int first, int n, int *__restrict__ r
 // ---- assembly --------------------------------------------------------------
 
 constexpr int ROW_BLOCK = 128;
+constexpr int ROW_RUNS = 65534;   // neighbours up to which a row's runs are numbered in 16 bits
 
 // Entries of every row, the start of each neighbour cell's run in it
 // (runs[q][row], q in visit order, so columns ascend along the row) and the
-// diagonal's place.
+// diagonal's place; the last two of rows of up to ROW_RUNS neighbours.
 template <int D>
 __global__ void __launch_bounds__(ROW_BLOCK)
 k_row_count(NbrSource<D> src, State<D> s, const int *__restrict__ part_of_row, const int *__restrict__ row_of,
@@ -315,11 +316,27 @@ k_fill(NbrSource<D> src, State<D> s, Consts k, const int *__restrict__ part_of_r
         if (MIXED && fc) fc[q] = make_uint2(__float_as_uint((float)v), (unsigned)c);
     };
     int c = __ldg(&src.cnt[i]);
-    if (c > src.pitch) {   // more neighbours than the list holds: the first lane walks the cells
+    if (c > src.pitch || c > ROW_RUNS) {
+        // more neighbours than the list holds or 16 bits number: the first lane
+        // walks the cells, once for the runs' starts and once for the entries
         if (l == 0) {
-            int prev = -1, pos = base;
+            constexpr int CELLS = D == 3 ? 27 : 9;
+            int next[CELLS] = {}, below = 0;
             src.cells.for_each(i, [&](int j) {
-                int row = row_of[j], cell = s.cell[j];
+                if (row_of[j] < 0) return;
+                int cell = s.cell[j];
+                next[neighbour_cell<D>(g, cell, ci)]++;
+                below += cell == ci && j < i;
+            });
+            int at = base;
+            for (int q = 0; q < CELLS; q++) {
+                int nb = visit_cell<D>(par, q), m = next[nb] + (nb == CELLS / 2);
+                if (nb == CELLS / 2) dpos = at + below;
+                next[nb] = at;
+                at += m;
+            }
+            src.cells.for_each(i, [&](int j) {
+                int row = row_of[j];
                 if (s.type[j] == DUMMY) return;
                 double pj[D];
                 load_vec<D>(pj, s.pos, j);
@@ -329,10 +346,7 @@ k_fill(NbrSource<D> src, State<D> s, Consts k, const int *__restrict__ part_of_r
                     known = known || w > 0.0;
                     return;
                 }
-                if (cell != prev) {
-                    prev = cell;
-                    pos = run_of(cell);
-                }
+                int &pos = next[neighbour_cell<D>(g, s.cell[j], ci)];
                 if (pos == dpos) pos++;
                 put(pos, row, k.neg_coeff * w);
                 sum_off += k.neg_coeff * w;

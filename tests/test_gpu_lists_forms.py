@@ -59,3 +59,43 @@ def test_no_room_for_lists(dim, precision):
     assert np.array_equal(nb.reshape(-1, 2000)[used], nb2.reshape(-1, 2000)[used])
     for f in FIELDS:
         assert np.array_equal(a[f], b[f]), f
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_matrix_of_rows_beyond_the_lists(dim):
+    """Rows with more neighbours than a list holds are assembled from the cells,
+    with run starts of their own: the matrix is the oracle's bit for bit, in
+    both precision forms."""
+    _cuda()
+    import ctypes as C
+    from mps_b200 import config as CF
+    from mps_b200.session import Session
+    from oracle.pyoracle import Oracle
+    wl = lists._workload(dim, True)
+    cfg = wl.config()
+    orc = Oracle(dim)
+    hp = T.HostParticles(dim, wl.pos, wl.vel, wl.types)
+    orc.initial_params(hp, cfg)
+    hp.ps.n0 *= 0.6   # fluid of twice the lattice's density: inside, not on the surface
+    re = CF.neighbor_radius(cfg)
+    m = cfg.max_neighbors
+    nl = T.HostNeighborList(hp.n, m)
+    cl = orc.cell_list(hp.n, re, cfg)
+    assert orc.search(nl, hp, cl, re) == 0
+    orc.lib.oracle_number_density(C.byref(hp.ps), C.byref(nl.nl), C.byref(cfg))
+    orc.lib.oracle_judge_free_surface(C.byref(hp.ps), cfg.surface_threshold)
+    want = orc.assemble(hp, nl, cfg)
+    q = re / cfg.particle_distance
+    k = np.arange(-4, 5)
+    g = np.stack(np.meshgrid(*[k] * dim), -1).reshape(-1, dim)
+    room = (int(1.4 * np.sum((g ** 2).sum(-1) < q * q)) + 15) & ~7
+    unknown = want[0] >= 0
+    assert (nl.count[: hp.n][unknown] > room).sum() > 100 and (nl.count[: hp.n][unknown] <= room).sum() > 100
+    for precision in (0, 1):
+        with Session(cfg, dim, hp.n, precision=precision) as s:
+            s.upload(hp)
+            s.set_initial_params(hp.ps.n0, hp.ps.lambda_, hp.ps.n0_count)
+            s.run_stage("solve_pressure", nl.neighbors[: hp.n * m], nl.count[: hp.n], m)
+            got = s.ppe()
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b)
