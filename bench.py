@@ -6,11 +6,11 @@
 A step is one full MPS time step (simulation.c:19-118 of the reference) of
 the 3-D dam break named by --workload, device-resident: explicit viscosity
 and collision, the cell-sort neighbour search, number density and surface
-flags, PPE assembly, IC(0) factorisation and the PCG solve to the absolute
+flags, PPE assembly, the preconditioner and the PCG solve to the absolute
 tolerance 1e-9, the pressure gradient and the correction.  `value` is fluid
 particle-steps/s over all ranks (each rank runs an independent replica with
 its own seed: the time step has no partition that avoids a halo exchange
-per operator and changes the IC(0) preconditioner).  The workload's PPE
+per operator and per CG iteration).  The workload's PPE
 matrix alone is 2.7 GB at c2, far above the 126 MB L2, so consecutive steps
 do not run from cache.
 
@@ -512,9 +512,9 @@ def run_b200(args, rank: int, world: int, local_rank: int):
                              "algorithmic_bytes_per_launch": spmv_b, "ms_per_launch": spmv_ms})
         top = dict(roof[0]) if roof else {}
         top.update({"peak_source": f"{peak_kind} hbm_gbs",
-                    "timing": "CUDA events on the library stream around every launch of the ICCG loop's kernels "
+                    "timing": "CUDA events on the library stream around every launch of the CG loop's kernels "
                               "(k_pcg: one launch per batch of iterations; the launch-per-colour form: every colour "
-                              "sweep and SpMV), over min(steps, 2) profiled steps right after the timed region",
+                              "sweep and SpMV; the multilevel form: every SpMV), over min(steps, 2) profiled steps right after the timed region",
                     "others": roof[1:]})
         cpu = cpu_baseline(args) if world == 1 else None
         forms_out = {}

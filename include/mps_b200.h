@@ -36,8 +36,8 @@ extern "C" {
 
 /* Precision forms of the step. */
 #define MPS_PREC_FP64  0   /* the reference's arithmetic, FP64 everywhere */
-#define MPS_PREC_MIXED 1   /* PPE matrix and IC(0) factor stored in FP32 (SpMV in difference
-                              form), FP64 vectors, dot products, refinement residuals and
+#define MPS_PREC_MIXED 1   /* PPE matrix, and IC(0) factor where used, stored in FP32 (SpMV in
+                              difference form), FP64 vectors, dot products, refinement residuals and
                               everything outside the PPE solve; the adjoint PPE solve too */
 
 /* PPE unknown orderings for the IC(0) preconditioner. */

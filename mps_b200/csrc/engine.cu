@@ -10,13 +10,16 @@
 //                                                a fresh sort (2-D all-pairs)
 //   neighbour search           sort()            counting sort by cell
 //   number density + surface   k_density
-//   PPE                        ppe()             assembly, IC(0), PCG
+//   PPE                        ppe()             assembly, preconditioner
+//                                                (multilevel, or IC(0)), PCG
 //   clamp (optional)           k_writeback
 //   pressure gradient          k_pmin, k_gradient
 //   correction, wall, ghosts   k_correct
 //
-// All work is issued on one stream; the host synchronises twice per step
-// to size the PPE (n_eq, nnz) and once per CG batch to test convergence.
+// All work is issued on one stream.  The host reads from it to size the PPE
+// (rows, then entries and grid nodes), after every batch of CG iterations (or
+// once, where the loop is one launch), for the true residual, and for the
+// error word at the end of the step.
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -1550,8 +1553,9 @@ bool Engine<D>::ml_build(int n_eq)
     // large to be dense (solve at 7,457 unknowns: 1.13 ms, against 1.28 by
     // launches), and nowhere above (13,334: 1.84 ms against 2.52, 57,816: 1.99
     // against 2.31).  From 20,000 to 40,000 unknowns it stays although slower
-    // (26,632: 2.4 ms against 1.8): the iteration count there is held to at
-    // least half of natural-order IC(0)'s, 95, and 36 is below that (49).
+    // (26,632: 2.30 ms against 1.79, 32,868: 2.38 against 1.91): a parity test
+    // of 26,632 unknowns holds the iteration count to at least half of
+    // natural-order IC(0)'s, 95, and 36 is below that (49).
     ml_add_ = ml_ld_ > 0 && (ml_add_rows_ >= 0 ? n_eq < ml_add_rows_
                                                : n_eq <= ml_small_rows_ || (n_eq >= 20000 && n_eq < 40000));
     // zero around the nodes in use (the dense grid alone reads no neighbours)
@@ -2505,9 +2509,9 @@ void Engine<D>::build_windows(bool fp32)
     win_valid_ = true;
 }
 
-// Mixed form: the ICCG with the matrix and the IC(0) factor stored in FP32
-// (the SpMV in difference form, k_cg_spmv<.., true>) and FP64 vectors and
-// arithmetic, with reliable updates.  Whenever the recursive residual has
+// Mixed form: CG with the matrix, and the IC(0) factor where that is the
+// preconditioner, stored in FP32 (the SpMV in difference form,
+// k_cg_spmv<.., true>) and FP64 vectors and arithmetic, with reliable updates.  Whenever the recursive residual has
 // fallen by kDelta (kDeltaMl) since the last update, the true residual r = b - A x
 // is recomputed with the FP64 matrix and the iteration resumes from it with
 // its search direction kept.  Stops when ||b - A x|| <= max(cg_tolerance,
@@ -2775,8 +2779,8 @@ void Engine<D>::adjoint_get(double *lam_pos, double *lam_vel, double *grad_gravi
 // Adjoint of one step.  The session holds the step's input state; the
 // adjoint seeds hold the adjoint of its output.  The step is recomputed
 // (recording x*, u*), its implicit part is reversed on the fresh structure
-// (correction, gradient, PPE by a second ICCG solve with the same matrix and
-// IC(0) factor, density), the input state is restored and the explicit part
+// (correction, gradient, PPE by a second solve with the same matrix and
+// preconditioner, density), the input state is restored and the explicit part
 // is reversed on the previous step's structure (collision, explicit update,
 // viscosity).  Afterwards the seeds hold the adjoint of the step's input,
 // the parameter gradients have this step's terms added, and the session

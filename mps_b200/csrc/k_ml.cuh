@@ -30,9 +30,9 @@
 // are used in P, P^T and A_1.
 //
 // Measured against the block-colour IC(0) (B200, the solve of a step): 3-D dam
-// break of 2.85 M particles, mixed form, 619 -> 30 iterations, 747 -> 23.5 ms;
-// 1.17 M particles in FP64, 507 -> 43, 336 -> 14.3 ms; 117 k particles, 160 ->
-// 40, 36.9 -> 2.7 ms; 2,158 particles in 2-D, 94 -> 37, 6.4 -> 1.0 ms.  What
+// break of 2.85 M particles, mixed form, 619 -> 30 iterations, 747 -> 21.6 ms;
+// 1.17 M particles in FP64, 507 -> 44, 333 -> 14.6 ms; 117 k particles, 173 ->
+// 40, 31.1 -> 2.6 ms; 2,158 particles in 2-D, 92 -> 36, 6.3 -> 0.43 ms.  What
 // remains of an iteration is the product with the matrix (HBM) at large sizes
 // and the chain of dependent launches at small ones.  With a V-cycle of
 // separate residual, restriction and interpolation steps the same solves took
@@ -1205,11 +1205,10 @@ __global__ void __launch_bounds__(CG_BLOCK) k_ml_matvec(MlVecs v, int lo, int n,
 
 // ---- small systems: the whole loop in one cluster ------------------------------------
 //
-// Below some ten thousand unknowns an iteration of the launched kernels is
-// six or seven launches of 3-9 us, nearly all of it launch and drain.  Here
-// one cluster of ML_CL CTAs runs the loop to its end, four cluster barriers an
-// iteration (the product, the update, the coarse correction, its
-// interpolation).  A barrier costs about 1,700 cycles and a load from L2 about
+// At up to 8,192 unknowns an iteration of the launched kernels is six or seven
+// launches of 3-9 us, nearly all of it launch and drain.  Here one cluster of
+// ML_CL CTAs runs the loop to its end, four cluster barriers an iteration (the
+// product, the update, the coarse correction, its interpolation).  A barrier costs about 1,700 cycles and a load from L2 about
 // 700, so what counts is the number of dependent ones: the direction and the
 // CTA's rows of the matrix (where they fit) sit in shared memory, loads go out
 // in predicated batches, the dot products' parts are stored into every CTA's
