@@ -1316,6 +1316,7 @@ void Engine<D>::set_initial_params(double n0, double lambda, int n0_count)
 template <int D>
 void Engine<D>::upload_list(const int *nb, const int *cnt, int max_nb)
 {
+    need_grid();
     int n = n_;
     if (max_nb <= 0) throw CudaError("max_neighbors must be positive", MPS_ERR_INVALID);
     int mc = 0;
@@ -1972,6 +1973,7 @@ void Engine<D>::require_ic0()
 {
     if (!ppe_valid_ || !ic0_valid_) throw CudaError("no IC(0) factor: run an ICCG step first", MPS_ERR_INVALID);
     if (ic0_built_ || n_eq_ == 0) return;
+    need_grid();   // the scans' workspace is the grid's
     factor_ic0();
     if (last_fp32_) convert_ic0();
     check_err();
